@@ -170,6 +170,9 @@ struct Lp {
     uint8_t *bid, *nid;
 };
 
+template <int N>
+struct IntC { static constexpr int value = N; };   // a compile-time width as an argument
+
 // Order-preserving unsigned images of non-negative values (min over the
 // keys = min over the values); all-ones marks "no candidate".
 __device__ __forceinline__ unsigned key_of(float v) { return __float_as_uint(v); }
@@ -308,6 +311,248 @@ __device__ int warp_simplex(const Lp<T> &L, T tol_piv, T tol_dj, int max_piv, in
     }
     *piv_out = piv;
     return status;
+}
+
+// The top 32 bits of a finite positive double's value as a float: exponent
+// and 23 mantissa bits, truncated (relative error < 2^-23); *ok false when the
+// exponent leaves [2^-100, 2^100].  Integer operations only: an F64 conversion
+// takes a slot of the FP64 pipe, which holds 2 lanes per clock and SM here.
+__device__ __forceinline__ float trunc_float(unsigned long long bits, bool *ok)
+{
+    const int hi = (int)(bits >> 32);
+    const int e = hi >> 20;
+    *ok = e >= 1023 - 100 && e <= 1023 + 100;
+    return __uint_as_float(((unsigned)(hi - (896 << 20)) << 3) | ((unsigned)bits >> 29));
+}
+
+// warp_simplex for an FP64 tableau in shared memory of at most 32 NS rows and
+// 31 columns: its rules, operations and roundings (so the same pivots and
+// bit-identical values), with the bookkeeping in registers as in
+// simplex_fast32 (each lane the ids of its rows lane, lane + 32, ...; lanes
+// 0..ncols the objective row; lanes 0..ncols-1 the nonbasic ids).
+//
+// Bound by the FP64 pipe (a warp instruction takes 16 cycles of an SM) and, on
+// small levels, by the pivot's latency.  Hence
+//  * the ratio test divides only where it has to: an FP32 quotient of the
+//    truncated operands (relative error below 2^-20) finds the rows within
+//    2^-18 of the smallest; a single such row wins without a division, several
+//    are compared by their exact quotients.  The generic loop divides once per
+//    row slot and once more for the degeneracy test;
+//  * comparisons against the tolerances and zero are integer comparisons;
+//  * the row update loads four columns of every row slot before it stores any
+//    (the compiler must otherwise keep each load behind the previous store).
+// An FP64 pivot of a 51 x 6 tableau takes about 27 FP64 warp instructions
+// instead of 67.  Measured, FP64 path of the n = 10, m = 43 problem (128K
+// sets): LP1 3,030 -> 2,008 us, the optimality kernel 4,457 -> 2,884 us; the
+// mixed path's k_optimality_fp64 on the m = 62 problem to |S| = 4 1,707 ->
+// 1,130 us and k_lp1_fp64 on the ill-conditioned one 2,718 -> 2,143 us (1,400
+// cycles of an SM per 78 x 25 pivot, 1,200 of them the DFMAs of the update).
+// tab, bid and nid are byte offsets into the block's dynamic shared memory
+// (the function is not inlined: its five callers share one copy).
+template <int NS>
+__device__ __noinline__ int simplex_fast64(unsigned tab_o, int ld, int nrows, int ncols, int nfree, unsigned bid_o,
+                                           unsigned nid_o, double tol_piv, double tol_dj, int max_piv,
+                                           int degen_switch, int *piv_out)
+{
+    extern __shared__ __align__(16) unsigned char smem[];
+    constexpr unsigned long long kInf = 0x7ff0000000000000ULL, kSign = 0x8000000000000000ULL;
+    const int lane = lane_id();
+    double *tab = reinterpret_cast<double *>(smem + tab_o);
+    uint8_t *bid = smem + bid_o, *nid = smem + nid_o;
+    int rowoff[NS], bidr[NS];   // bidr: the basic id, -1 past the last row
+#pragma unroll
+    for (int s = 0; s < NS; s++) {
+        const int i = lane + 32 * s;
+        bidr[s] = i < nrows ? (int)bid[i] : -1;
+        rowoff[s] = i * ld;
+    }
+    double *obj = tab + (size_t)nrows * ld;
+    double ob = lane <= ncols ? obj[lane] : 0.0;
+    int nidl = lane < ncols ? (int)nid[lane] : 255;
+    const long long tpiv = __double_as_longlong(tol_piv), tdj = __double_as_longlong(tol_dj);
+    int piv = 0, degen = 0, status;
+    bool bland = false;
+    for (;;) {
+        // pricing: largest |reduced cost|, smallest id on ties (Bland: smallest id)
+        long long sc = __double_as_longlong(ob);
+        if (nidl < nfree) sc &= (long long)~kSign;
+        bool el = lane < ncols && sc > tdj && sc <= (long long)kInf;
+        unsigned m = __ballot_sync(FULLMASK, el);
+        if (!m) { status = LP_OPTIMAL; break; }
+        if (!bland) {
+            // (every lane takes part in the reductions, eligible or not)
+            const unsigned hi = (unsigned)((unsigned long long)sc >> 32), lo = (unsigned)sc;
+            const unsigned hmax = __reduce_max_sync(FULLMASK, el ? hi : 0u);
+            el = el && hi == hmax;
+            m = __ballot_sync(FULLMASK, el);
+            if (m & (m - 1)) {
+                const unsigned lmax = __reduce_max_sync(FULLMASK, el ? lo : 0u);
+                el = el && lo == lmax;
+                m = __ballot_sync(FULLMASK, el);
+            }
+        }
+        if (m & (m - 1)) {
+            const unsigned im = __reduce_min_sync(FULLMASK, el ? (unsigned)nidl : 0xffffffffu);
+            m = __ballot_sync(FULLMASK, el && (unsigned)nidl == im);
+        }
+        const int q = __ffs(m) - 1;
+        const double obq = __shfl_sync(FULLMASK, ob, q);
+        const unsigned long long flip = obq > 0.0 ? 0ull : kSign;   // a = sign(obq) T[i][q]
+        // ratio test: smallest max(beta,0)/a over a > tol_piv, smallest id on ties
+        double aq[NS];
+        float qf[NS];
+        unsigned pass = 0, unsure = 0;   // bit s: row slot s is in the test / its FP32 quotient says nothing
+        float qmin = pos_inf<float>();
+#pragma unroll
+        for (int s = 0; s < NS; s++) {
+            aq[s] = 0.0;
+            qf[s] = pos_inf<float>();
+            if (bidr[s] >= 0) {
+                aq[s] = tab[rowoff[s] + q];
+                const unsigned long long a = (unsigned long long)__double_as_longlong(aq[s]) ^ flip;
+                if (bidr[s] >= nfree && (long long)a > tpiv && a <= kInf) {
+                    pass |= 1u << s;
+                    const unsigned long long b = (unsigned long long)__double_as_longlong(tab[rowoff[s] + ncols]);
+                    if ((long long)b > 0 && b <= kInf) {
+                        bool oka, okb;
+                        const float af = trunc_float(a, &oka), bf = trunc_float(b, &okb);
+                        const float v = __fdividef(bf, af);
+                        // an underflowing quotient has lost its relative accuracy
+                        if (oka && okb && v >= 0x1p-100f) qf[s] = v;
+                        else unsure |= 1u << s;
+                    } else {
+                        qf[s] = 0.0f;
+                    }
+                    qmin = fminf(qmin, qf[s]);
+                }
+            }
+        }
+        const unsigned qk = __reduce_min_sync(FULLMASK, __float_as_uint(qmin));
+        const float lim = __uint_as_float(qk) * (1.0f + 0x1p-18f);   // inf stays inf
+        int r = -1, ncand = 0;
+        unsigned cand = 0;
+#pragma unroll
+        for (int s = 0; s < NS; s++) {
+            const bool c = ((pass >> s) & 1u) && (((unsure >> s) & 1u) || qf[s] <= lim);
+            if (c) cand |= 1u << s;
+            const unsigned cm = __ballot_sync(FULLMASK, c);
+            if (cm) r = 32 * s + __ffs(cm) - 1;
+            ncand += __popc(cm);
+        }
+        if (ncand == 0) { status = LP_UNBOUNDED; break; }
+        if (ncand > 1) {
+            // the exact quotients of the rows within the FP32 error of the smallest
+            unsigned long long rkey = ~0ull;
+            unsigned rid = 0xffffffffu;
+            int bri = -1;
+#pragma unroll
+            for (int s = 0; s < NS; s++) {
+                if ((cand >> s) & 1u) {
+                    double beta = tab[rowoff[s] + ncols];
+                    if (!(beta > 0.0)) beta = 0.0;
+                    const double a = __longlong_as_double((long long)((unsigned long long)__double_as_longlong(aq[s]) ^ flip));
+                    const unsigned long long k = key_of(ratio_div(beta, a));
+                    if (bri < 0 || k < rkey || (k == rkey && (unsigned)bidr[s] < rid)) {
+                        rkey = k; rid = (unsigned)bidr[s]; bri = lane + 32 * s;
+                    }
+                }
+            }
+            r = warp_argmin(rkey, rid, bri);
+            if (r < 0) { status = LP_UNBOUNDED; break; }
+        }
+        if (piv >= max_piv) { status = LP_ITER_LIMIT; break; }
+        double *Rp = tab + (size_t)r * ld;
+        const double br = Rp[ncols], prq = Rp[q];
+        // the ratio is zero (a degenerate pivot) when beta is, or underflows
+        bool zero = !(br > 0.0);
+        if (!zero && br < 1e-280) zero = ratio_div(br, fabs(prq)) == 0.0;
+        const double inv = __drcp_rn(prq);
+        const int owner = r & 31, oslot = r >> 5;
+        int lid = bidr[0];
+#pragma unroll
+        for (int s = 1; s < NS; s++) if (s == oslot) lid = bidr[s];
+        lid = __shfl_sync(FULLMASK, lid, owner);
+        const int eid = __shfl_sync(FULLMASK, nidl, q);
+        double rl = lane <= ncols ? Rp[lane] : 0.0;
+        rl = lane == q ? inv : xmul(rl, inv);
+        __syncwarp();
+        if (lane <= ncols) Rp[lane] = rl;
+        __syncwarp();
+        bool upd[NS];
+        double nf[NS];
+#pragma unroll
+        for (int s = 0; s < NS; s++) {
+            upd[s] = bidr[s] >= 0 && !(lane == owner && s == oslot);
+            nf[s] = -aq[s];
+        }
+        auto columns = [&](int c0, auto width) {
+            constexpr int W = decltype(width)::value;
+            double Rc[W], t[NS][W];
+#pragma unroll
+            for (int j = 0; j < W; j++) Rc[j] = Rp[c0 + j];
+#pragma unroll
+            for (int s = 0; s < NS; s++)
+                if (upd[s]) {
+#pragma unroll
+                    for (int j = 0; j < W; j++) t[s][j] = tab[rowoff[s] + c0 + j];
+                }
+#pragma unroll
+            for (int s = 0; s < NS; s++)
+                if (upd[s]) {
+#pragma unroll
+                    for (int j = 0; j < W; j++) tab[rowoff[s] + c0 + j] = xfma(nf[s], Rc[j], t[s][j]);
+                }
+        };
+        int c0 = 0;
+#pragma unroll 1
+        for (; c0 + 3 <= ncols; c0 += 4) columns(c0, IntC<4>{});
+        const int rem = ncols + 1 - c0;
+        if (rem == 3) columns(c0, IntC<3>{});
+        else if (rem == 2) columns(c0, IntC<2>{});
+        else if (rem == 1) columns(c0, IntC<1>{});
+#pragma unroll
+        for (int s = 0; s < NS; s++) if (upd[s]) tab[rowoff[s] + q] = xmul(nf[s], inv);
+        if (lane <= ncols) ob = lane == q ? xmul(-obq, inv) : xfma(-obq, rl, ob);
+#pragma unroll
+        for (int s = 0; s < NS; s++) if (s == oslot && lane == owner) bidr[s] = eid;
+        if (lane == q) nidl = lid;
+        __syncwarp();
+        piv++;
+        degen = zero ? degen + 1 : 0;
+        bland = degen >= degen_switch;
+    }
+    if (lane <= ncols) obj[lane] = ob;
+    if (lane < ncols) nid[lane] = (uint8_t)nidl;
+#pragma unroll
+    for (int s = 0; s < NS; s++) if (bidr[s] >= 0) bid[lane + 32 * s] = (uint8_t)bidr[s];
+    __syncwarp();
+    *piv_out = piv;
+    return status;
+}
+
+// resident blocks (of 4 warps) the kernels with FP64 simplexes are compiled
+// for: 128 registers, 16 warps per SM (12 and 20 warps measured the same
+// within 5 % on five batches: the FP64 pipe is the bound there)
+constexpr int kF64Blocks = 4;
+
+// warp_simplex for an FP64 tableau whose arrays lie in the block's dynamic
+// shared memory: simplex_fast64 up to 128 rows and 31 columns (every tableau of
+// the workloads here), the generic loop above; the same pivots either way
+__device__ __forceinline__ int warp_simplex_f64(const Lp<double> &L, double tol_piv, double tol_dj, int max_piv,
+                                                int degen_switch, int *piv_out)
+{
+    if (L.nrows > 128 || L.ncols > 31 || !(tol_piv > 0.0) || !(tol_dj > 0.0))
+        return warp_simplex<double>(L, tol_piv, tol_dj, max_piv, degen_switch, piv_out);
+    extern __shared__ __align__(16) unsigned char smem[];
+    const unsigned to = (unsigned)(reinterpret_cast<unsigned char *>(L.tab) - smem);
+    const unsigned bo = (unsigned)(L.bid - smem), no = (unsigned)(L.nid - smem);
+#define MQ_F64(NS) simplex_fast64<NS>(to, L.ld, L.nrows, L.ncols, L.nfree, bo, no, tol_piv, tol_dj, max_piv, \
+                                      degen_switch, piv_out)
+    if (L.nrows <= 32) return MQ_F64(1);
+    if (L.nrows <= 64) return MQ_F64(2);
+    if (L.nrows <= 96) return MQ_F64(3);
+    return MQ_F64(4);
+#undef MQ_F64
 }
 
 // Full-warp FP32 simplex with register bookkeeping, for tableaus of at most
@@ -1100,7 +1345,8 @@ __device__ __noinline__ void cold_stage_lp1_f32(const DevBuffers &B, const InstD
 //             certified (see below), otherwise the candidate is queued for
 //             the FP64 re-solve.
 template <typename T>
-__global__ void __launch_bounds__(128) k_feasibility(DevBuffers B, Tol tol, SlotDims sd, int level, int chunk)
+__device__ __forceinline__ void feasibility_body(const DevBuffers &B, const Tol &tol, const SlotDims &sd, int level,
+                                                 int chunk)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     const int lane = lane_id(), wib = threadIdx.x >> 5;
@@ -1277,7 +1523,7 @@ __global__ void __launch_bounds__(128) k_feasibility(DevBuffers B, Tol tol, Slot
         // and rows of free variables that enter the basis are dropped
         if constexpr (sizeof(T) == 4) st = warp_simplex_f32<kFastChunks>(L, tpiv, tdj, tol.max_pivots, tol.degen_switch, &piv,
                                                                           par.lo, par.hi, nv, true, &rows);
-        else st = warp_simplex<T>(L, tpiv, tdj, tol.max_pivots, tol.degen_switch, &piv);
+        else st = warp_simplex_f64(L, tpiv, tdj, tol.max_pivots, tol.degen_switch, &piv);
         const T z = obj[pcols];
         uint64_t lo = par.lo, hi = par.hi;
         if (c.j < 64) lo |= 1ull << c.j; else hi |= 1ull << (c.j - 64);
@@ -1419,10 +1665,21 @@ __global__ void __launch_bounds__(128) k_feasibility(DevBuffers B, Tol tol, Slot
     }
 }
 
+__global__ void __launch_bounds__(128) k_feasibility_f32(DevBuffers B, Tol tol, SlotDims sd, int level, int chunk)
+{
+    feasibility_body<float>(B, tol, sd, level, chunk);
+}
+
+__global__ void __launch_bounds__(128, kF64Blocks) k_feasibility_f64(DevBuffers B, Tol tol, SlotDims sd, int level,
+                                                                     int chunk)
+{
+    feasibility_body<double>(B, tol, sd, level, chunk);
+}
+
 // ---------------------------------------------------------------------
 // K2b: FP64 LP1 re-solve (mixed precision), cold from the root tableau
 // ---------------------------------------------------------------------
-__global__ void __launch_bounds__(128) k_lp1_fp64(DevBuffers B, Tol tol, SlotDims sd, int level)
+__global__ void __launch_bounds__(128, kF64Blocks) k_lp1_fp64(DevBuffers B, Tol tol, SlotDims sd, int level)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     const int lane = lane_id(), wib = threadIdx.x >> 5;
@@ -1463,7 +1720,7 @@ __global__ void __launch_bounds__(128) k_lp1_fp64(DevBuffers B, Tol tol, SlotDim
         __syncwarp();
         Lp<double> L{tab, ld, M1, nv, nv, bid, nid};
         int piv = 0;
-        const int st = warp_simplex<double>(L, tol.tol_piv, tol.tol_dj, tol.max_pivots, tol.degen_switch, &piv);
+        const int st = warp_simplex_f64(L, tol.tol_piv, tol.tol_dj, tol.max_pivots, tol.degen_switch, &piv);
         const double z = obj[nv];
         const bool feasible = (st == LP_OPTIMAL) && (z <= tol.tol_feas);
         const long long rec = (B.rec && ctl->rec_base + w < B.rec_cap) ? ctl->rec_base + w : -1;
@@ -2186,7 +2443,7 @@ __device__ void lp2_short_mplp(const DevBuffers &B, const Tol &tol, const InstDe
     int st;
     {
         Lp<double> L{T, ld, nrows, ncols, ncols, bid, nid};
-        st = warp_simplex<double>(L, tpiv, tdj, tol.max_pivots, tol.degen_switch, &piv1);
+        st = warp_simplex_f64(L, tpiv, tdj, tol.max_pivots, tol.degen_switch, &piv1);
     }
     res.lp2_piv = piv1;
     if (st != LP_OPTIMAL) { res.lp2_status = st; return; }
@@ -2231,7 +2488,7 @@ __device__ void lp2_short_mplp(const DevBuffers &B, const Tol &tol, const InstDe
     __syncwarp();
     {
         Lp<double> L{T, ld, nrows + 1, ncols, ncols, bid, nid};
-        st = warp_simplex<double>(L, tpiv, tdj, tol.max_pivots, tol.degen_switch, &piv2);
+        st = warp_simplex_f64(L, tpiv, tdj, tol.max_pivots, tol.degen_switch, &piv2);
     }
     res.lp2_piv = piv1 + piv2;
     res.lp2_status = st;
@@ -2305,7 +2562,7 @@ __device__ void chebyshev_ball(const Tol &tol, const InstDesc &I, OptWs<T> &ws, 
     {
         Lp<T> L{Tb, ld2, nc, P1, P1, bid, nid};
         int piv = 0;
-        res.cheb_status = warp_simplex<T>(L, tpiv, tdj, tol.max_pivots, tol.degen_switch, &piv);
+        res.cheb_status = warp_simplex_f64(L, tpiv, tdj, tol.max_pivots, tol.degen_switch, &piv);
         res.cheb_piv = piv;
     }
     if (res.cheb_status == LP_OPTIMAL) {
@@ -2521,7 +2778,7 @@ __device__ OptResult eval_optimality(const DevBuffers &B, const Tol &tol, const 
     {
         Lp<T> L{Tb, ld2, R2, P1, P1, bid, nid};
         int piv = 0;
-        res.lp2_status = warp_simplex<T>(L, tpiv, tdj, tol.max_pivots, tol.degen_switch, &piv);
+        res.lp2_status = warp_simplex_f64(L, tpiv, tdj, tol.max_pivots, tol.degen_switch, &piv);
         res.lp2_piv = piv;
     }
     if (res.lp2_status == LP_OPTIMAL) {
@@ -2569,7 +2826,7 @@ __device__ void write_opt(const DevBuffers &B, const Node &nd, int level, const 
 // instances, LP = true those of mpLP instances (launched only when a batch
 // has one), so that the mpQP kernel carries no mpLP code.
 template <typename T, bool LP>
-__global__ void __launch_bounds__(128) k_optimality(DevBuffers B, Tol tol, SlotDims sd, int level)
+__global__ void __launch_bounds__(128, kF64Blocks) k_optimality(DevBuffers B, Tol tol, SlotDims sd, int level)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     const int lane = lane_id(), wib = threadIdx.x >> 5;
@@ -2616,7 +2873,7 @@ __global__ void __launch_bounds__(128) k_optimality(DevBuffers B, Tol tol, SlotD
 }
 
 template <bool LP>
-__global__ void __launch_bounds__(128) k_optimality_fp64(DevBuffers B, Tol tol, SlotDims sd, int level)
+__global__ void __launch_bounds__(128, kF64Blocks) k_optimality_fp64(DevBuffers B, Tol tol, SlotDims sd, int level)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     const int lane = lane_id(), wib = threadIdx.x >> 5;
@@ -4167,7 +4424,7 @@ __global__ void __launch_bounds__(32, 32) k_opt_screen(DevBuffers B, Tol tol, Sl
 // maximum is at most d_i + tol.  One warp per row, the FP64 warp simplex from
 // the slack basis (u = 0 is feasible: d >= 0).  out[c] = 1 redundant, 0 not
 // (an iteration limit keeps the row).
-__global__ void __launch_bounds__(32) k_redundancy(const double *M, const double *d, int nrows, int nv, int ld,
+__global__ void __launch_bounds__(32, 4 * kF64Blocks) k_redundancy(const double *M, const double *d, int nrows, int nv, int ld,
                                                    const int *check, int n_check, double tol, Tol lt, int max_piv,
                                                    int *out)
 {
@@ -4194,7 +4451,7 @@ __global__ void __launch_bounds__(32) k_redundancy(const double *M, const double
         __syncwarp();
         Lp<double> L{T, ld, nrows, nv, nv, bid, nid};
         int piv = 0;
-        const int st = warp_simplex<double>(L, lt.tol_piv, lt.tol_dj, max_piv, lt.degen_switch, &piv);
+        const int st = warp_simplex_f64(L, lt.tol_piv, lt.tol_dj, max_piv, lt.degen_switch, &piv);
         const double maxval = -T[(size_t)nrows * ld + nv];
         if (lane == 0) out[c] = (st == LP_OPTIMAL && maxval <= d[i] + tol) ? 1 : 0;
         __syncwarp();
@@ -4330,7 +4587,7 @@ __global__ void k_finalize(DevBuffers B, int level)
 // then the normalised region rows [CR_As | CR_bs] (n_cr x (p+1)).
 // sizes = {k, n, p, n_cr}; k = -1 when the KKT factor fails (LICQ), k = -2
 // for an mpLP set with |S| < n (x(theta) is not unique; nothing written).
-__global__ void __launch_bounds__(128) k_region_laws(DevBuffers B, Tol tol, SlotDims sd, const uint64_t *masks,
+__global__ void __launch_bounds__(128, kF64Blocks) k_region_laws(DevBuffers B, Tol tol, SlotDims sd, const uint64_t *masks,
                                                      long long n_sets, double *laws, int *sizes, long long stride,
                                                      double *radius, double *err)
 {
@@ -4477,8 +4734,8 @@ const void *kernel_ptr(const char *name)
     struct E { const char *n; const void *f; };
     static const E tab[] = {
         {"enumerate", (const void *)k_enumerate},
-        {"feas64", (const void *)k_feasibility<double>},
-        {"feas32", (const void *)k_feasibility<float>},
+        {"feas64", (const void *)k_feasibility_f64},
+        {"feas32", (const void *)k_feasibility_f32},
         {"lp1_fp64", (const void *)k_lp1_fp64},
         {"lp1_cert", (const void *)k_lp1_cert},
         {"opt64", (const void *)k_optimality<double, false>},
@@ -4521,8 +4778,8 @@ cudaError_t launch_feasibility(const DevBuffers &B, const Tol &tol, const SlotDi
                                int grid, size_t smem, cudaStream_t s, int warps, int chunk)
 {
     if (warps < 1 || warps > 4 || chunk < 1 || chunk > kFeasChunkMax) return cudaErrorInvalidValue;
-    if (prec == PREC_FP64) k_feasibility<double><<<grid, 32 * warps, smem, s>>>(B, tol, sd, level, chunk);
-    else k_feasibility<float><<<grid, 32 * warps, smem, s>>>(B, tol, sd, level, chunk);
+    if (prec == PREC_FP64) k_feasibility_f64<<<grid, 32 * warps, smem, s>>>(B, tol, sd, level, chunk);
+    else k_feasibility_f32<<<grid, 32 * warps, smem, s>>>(B, tol, sd, level, chunk);
     return cudaGetLastError();
 }
 
