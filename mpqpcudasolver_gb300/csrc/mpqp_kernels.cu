@@ -567,6 +567,16 @@ __device__ __forceinline__ int warp_simplex_f64(const Lp<double> &L, double tol_
 // below nfree are free variables (nfree >= ncols: an LP1 tableau whose fixed
 // slack columns were moved past the right-hand side has fewer columns than
 // free variables).
+//
+// Bound by instruction issue and shared-memory wavefronts about equally (about
+// 95 wavefronts of the 140 cycles a pivot of 56 x 14 took an SM).  A minimum is
+// found by one reduction and a ballot (ids are compared only on a tie), the
+// fixed and free variables are flags on the ids, and the pivot and the
+// degeneracy test come from the ratio test's registers: LP1 of the m = 62 batch
+// (59.9M sets) 189 -> 173 ms, of 64 MPC problems (1.3M sets) 3.9 -> 3.5 ms.
+// Measured and left out: the tableau in registers (lane l rows l, l + 32, the
+// pivot column by a jump on its number): 73M instead of 254M wavefronts, but
+// 128 registers and 222 ms; the update by fma.rn.f32x2: spills, 181 ms.
 constexpr int kFastRows = 96;
 constexpr int kFastChunks = 6;
 
@@ -583,107 +593,121 @@ __device__ int simplex_fast32(float *tab, int ld, int nrows, int ncols, int nfre
                               uint64_t fix_lo, uint64_t fix_hi, int fix_base, bool compact, int *nrows_out)
 {
     constexpr int NR = NRS;
+    // flags above the 8-bit ids: a free variable; a variable fixed at zero while nonbasic
+    constexpr int kFree = 1 << 8, kFixed = 1 << 9;
     const int lane = lane_id();
-    int rowoff[NR], bidr[NR];
-    bool valid[NR];
+    auto flagged = [&](int id) {
+        const int fi = id - fix_base;
+        return id | (id < nfree ? kFree : 0) | (fi >= 0 && fi < 128 && mask_has(fix_lo, fix_hi, fi) ? kFixed : 0);
+    };
+    int rowoff[NR], bidr[NR];   // bidr: flagged basic id, -1 past the last row
 #pragma unroll
     for (int s = 0; s < NR; s++) {
         const int i = lane + 32 * s;
-        valid[s] = i < nrows;
+        bidr[s] = i < nrows ? flagged(bid[i]) : -1;
         rowoff[s] = i * ld;
-        bidr[s] = valid[s] ? bid[i] : 255;
     }
     float *obj = tab + nrows * ld;
     float ob = lane <= ncols ? obj[lane] : 0.0f;
-    int nidl = lane < ncols ? nid[lane] : 255;
+    int nidl = lane < ncols ? flagged(nid[lane]) : kFixed;
     int piv = 0, degen = 0, status;
     bool bland = false;
     for (;;) {
         // pricing: largest |reduced cost|, smallest id on ties (Bland: smallest id)
-        unsigned key = 0xffffffffu, kid = 0xffffffffu;
-        int kidx = -1;
-        if (lane < ncols) {
-            const float sc = nidl < nfree ? fabsf(ob) : ob;
-            const int fi = nidl - fix_base;
-            const bool fixed = fi >= 0 && fi < 128 && mask_has(fix_lo, fix_hi, fi);
-            if (sc > tol_dj && !fixed) { key = bland ? 0u : ~key_of(sc); kid = (unsigned)nidl; kidx = lane; }
+        const float sc = (nidl & kFree) ? fabsf(ob) : ob;
+        unsigned key = (sc > tol_dj && !(nidl & kFixed)) ? __float_as_uint(sc) : 0u;
+        if (bland && key) key = 1u;
+        const unsigned kmax = __reduce_max_sync(FULLMASK, key);
+        if (kmax == 0u) { status = LP_OPTIMAL; break; }
+        unsigned cm = __ballot_sync(FULLMASK, key == kmax);
+        if (cm & (cm - 1)) {
+            const unsigned im = __reduce_min_sync(FULLMASK, key == kmax ? (unsigned)(nidl & 255) : 0xffffffffu);
+            cm = __ballot_sync(FULLMASK, key == kmax && (unsigned)(nidl & 255) == im);
         }
-        const int q = warp_argmin(key, kid, kidx);
-        if (q < 0) { status = LP_OPTIMAL; break; }
+        const int q = __ffs(cm) - 1;
         const float obq = __shfl_sync(FULLMASK, ob, q);
+        const int eid = __shfl_sync(FULLMASK, nidl, q);
         const float sg = obq > 0.0f ? 1.0f : -1.0f;
         // ratio test: smallest max(beta,0)/a over a > tol_piv, smallest id on ties
-        unsigned rkey = 0xffffffffu, rid = 0xffffffffu;
-        int bri = -1;
         float aq[NR];
+        unsigned rk[NR], rkey = 0xffffffffu;
 #pragma unroll
         for (int s = 0; s < NR; s++) {
             aq[s] = 0.0f;
-            if (valid[s]) {
+            rk[s] = 0xffffffffu;
+            if (bidr[s] >= 0) {
                 aq[s] = tab[rowoff[s] + q];
-                if (bidr[s] >= nfree) {
-                    const float a = sg * aq[s];
-                    if (a > tol_piv) {
-                        float beta = tab[rowoff[s] + ncols];
-                        if (!(beta > 0.0f)) beta = 0.0f;
-                        const unsigned k = key_of(ratio_div(beta, a));
-                        if (bri < 0 || k < rkey || (k == rkey && (unsigned)bidr[s] < rid)) {
-                            rkey = k; rid = (unsigned)bidr[s]; bri = lane + 32 * s;
-                        }
-                    }
+                const float a = sg * aq[s];
+                if (a > tol_piv && !(bidr[s] & kFree)) {
+                    rk[s] = key_of(ratio_div(fmaxf(tab[rowoff[s] + ncols], 0.0f), a));
+                    rkey = rk[s] < rkey ? rk[s] : rkey;
                 }
             }
         }
-        const int r = warp_argmin(rkey, rid, bri);
-        if (r < 0) { status = LP_UNBOUNDED; break; }
+        const unsigned rmin = __reduce_min_sync(FULLMASK, rkey);
+        if (rmin == 0xffffffffu) { status = LP_UNBOUNDED; break; }
         if (piv >= max_piv) { status = LP_ITER_LIMIT; break; }
-        float *Rp = tab + r * ld;
-        float br = Rp[ncols];
-        if (!(br > 0.0f)) br = 0.0f;
-        const float prq = Rp[q];
-        const float rr = ratio_div(br, sg * prq);
-        const float inv = xdiv(1.0f, prq);
-        const int owner = r & 31, oslot = r >> 5;
-        const int lid = __shfl_sync(FULLMASK, (int)rid, owner);   // the owner's best row is r
-        const int eid = __shfl_sync(FULLMASK, nidl, q);
-        __syncwarp();
-        if (lane <= ncols) Rp[lane] = (lane == q) ? inv : xmul(Rp[lane], inv);
-        __syncwarp();
-        const float rl = lane <= ncols ? Rp[lane] : 0.0f;
-        bool upd[NR];
+        int owner = 0, oslot = 0, nmin = 0;
 #pragma unroll
-        for (int s = 0; s < NR; s++) upd[s] = valid[s] && lane + 32 * s != r;
+        for (int s = 0; s < NR; s++) {
+            const unsigned b = __ballot_sync(FULLMASK, rk[s] == rmin);
+            if (b) { owner = __ffs(b) - 1; oslot = s; }
+            nmin += __popc(b);
+        }
+        if (nmin > 1) {
+            unsigned rid = 0xffffffffu;
+#pragma unroll
+            for (int s = 0; s < NR; s++)
+                if (rk[s] == rmin && (unsigned)(bidr[s] & 255) < rid) rid = (unsigned)(bidr[s] & 255);
+            rid = __reduce_min_sync(FULLMASK, rid);
+#pragma unroll
+            for (int s = 0; s < NR; s++) {
+                const unsigned b = __ballot_sync(FULLMASK, rk[s] == rmin && (unsigned)(bidr[s] & 255) == rid);
+                if (b) { owner = __ffs(b) - 1; oslot = s; }
+            }
+        }
+        float prq = aq[0];
+        int lid = bidr[0];
+#pragma unroll
+        for (int s = 1; s < NR; s++) if (s == oslot) { prq = aq[s]; lid = bidr[s]; }
+        prq = __shfl_sync(FULLMASK, prq, owner);
+        lid = __shfl_sync(FULLMASK, lid, owner);
+        const int r = owner + 32 * oslot;
+        float *Rp = tab + r * ld;
+        const float inv = __frcp_rn(prq);
+        __syncwarp();
+        float rl = 0.0f;
+        if (lane <= ncols) {
+            rl = lane == q ? inv : xmul(Rp[lane], inv);
+            Rp[lane] = rl;
+        }
+        __syncwarp();
         // chunk by chunk (one float4 of the pivot row live), then column q
 #pragma unroll
         for (int c = 0; c < NCH; c++) {
             const float4 Rc = reinterpret_cast<const float4 *>(Rp)[c];
 #pragma unroll
             for (int s = 0; s < NR; s++) {
-                if (upd[s]) {
+                if (bidr[s] >= 0 && !(s == oslot && lane == owner)) {
                     float4 *Tc = reinterpret_cast<float4 *>(tab + rowoff[s]) + c;
-                    const float nf = -aq[s];
                     float4 t = *Tc;
-                    t.x = __fmaf_rn(nf, Rc.x, t.x);
-                    t.y = __fmaf_rn(nf, Rc.y, t.y);
-                    t.z = __fmaf_rn(nf, Rc.z, t.z);
-                    t.w = __fmaf_rn(nf, Rc.w, t.w);
+                    t.x = __fmaf_rn(-aq[s], Rc.x, t.x);
+                    t.y = __fmaf_rn(-aq[s], Rc.y, t.y);
+                    t.z = __fmaf_rn(-aq[s], Rc.z, t.z);
+                    t.w = __fmaf_rn(-aq[s], Rc.w, t.w);
                     *Tc = t;
                 }
             }
         }
 #pragma unroll
-        for (int s = 0; s < NR; s++) if (upd[s]) tab[rowoff[s] + q] = xmul(-aq[s], inv);
-        if (lane <= ncols) {
-            const float nfo = -obq;
-            ob = (lane == q) ? xmul(nfo, inv) : __fmaf_rn(nfo, rl, ob);
-        }
-        if (lane == owner) {
+        for (int s = 0; s < NR; s++)
+            if (bidr[s] >= 0 && !(s == oslot && lane == owner)) tab[rowoff[s] + q] = xmul(-aq[s], inv);
+        if (lane <= ncols) ob = lane == q ? xmul(-obq, inv) : __fmaf_rn(-obq, rl, ob);
 #pragma unroll
-            for (int s = 0; s < NR; s++) if (s == oslot) bidr[s] = eid;
-        }
+        for (int s = 0; s < NR; s++) if (s == oslot && lane == owner) bidr[s] = eid;
         if (lane == q) nidl = lid;
         __syncwarp();
-        if (compact && eid < nfree) {
+        if (compact && (eid & kFree)) {
             // row r now belongs to a free variable: the last row takes its place
             const int last = nrows - 1;
             if (r != last) {
@@ -693,25 +717,23 @@ __device__ int simplex_fast32(float *tab, int ld, int nrows, int ncols, int nfre
                 for (int s = 0; s < NR; s++) if (s == (last >> 5)) lb = bidr[s];
                 lb = __shfl_sync(FULLMASK, lb, last & 31);
                 if (lane <= ncols) Rp[lane] = v;
-                if (lane == owner) {
 #pragma unroll
-                    for (int s = 0; s < NR; s++) if (s == oslot) bidr[s] = lb;
-                }
+                for (int s = 0; s < NR; s++) if (s == oslot && lane == owner) bidr[s] = lb;
             }
             nrows = last;
 #pragma unroll
-            for (int s = 0; s < NR; s++) valid[s] = lane + 32 * s < nrows;
+            for (int s = 0; s < NR; s++) if (lane + 32 * s >= nrows) bidr[s] = -1;
             __syncwarp();
         }
         piv++;
-        degen = (rr == 0.0f) ? degen + 1 : 0;
+        degen = rmin == 0u ? degen + 1 : 0;
         bland = degen >= degen_switch;
     }
     // write the bookkeeping back
     if (lane <= ncols) obj[lane] = ob;
     if (lane < ncols) nid[lane] = (uint8_t)nidl;
 #pragma unroll
-    for (int s = 0; s < NR; s++) if (valid[s]) bid[lane + 32 * s] = (uint8_t)bidr[s];
+    for (int s = 0; s < NR; s++) if (bidr[s] >= 0) bid[lane + 32 * s] = (uint8_t)bidr[s];
     __syncwarp();
     *piv_out = piv;
     if (nrows_out) *nrows_out = nrows;
