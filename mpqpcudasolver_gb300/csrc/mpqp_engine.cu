@@ -362,6 +362,8 @@ struct mpqp_plan {
     size_t smem_tiles = 0;
     int grid_lanes = 0;         // ... at levels |S| <= kLaneMaxK: one set per thread
     size_t smem_lanes = 0;
+    std::vector<double> lvl_sets;   // per level, an upper bound on the batch's sets (combinatorial, budgets)
+    int grid_direct = 0;        // k_optimality<double> over a whole small level (mixed precision)
     int lane_cap = 3;           // pivots of its first pass (MPQP_SCREEN_CAP)
     int lane_cap2 = 6;          // ... of its second (MPQP_SCREEN_CAP2; 0: uncapped, no third pass)
     // launch settings the autotuner chooses: threads per set in the screen's
@@ -535,6 +537,14 @@ static int grid_for(const void *fn, size_t smem, int *grid, int block = 128)
     return MPQP_OK;
 }
 
+// waves of the FP64 optimality kernel (4 warps a block, one set a warp) up to
+// which a level skips the FP32 screen, and of the one-set-per-thread screen up
+// to which it runs uncapped.  Optimality kernels of a whole run with neither,
+// at (1, 1) waves and at (3, 4): 43 small problems (28K sets) 1,089, 751 and
+// 645 us; n = 10, m = 43, |S| <= 4 (128K) 921, 689 and 600 us; m = 62, |S| <= 4
+// (592K) 2,566, 2,284 and 2,280 us; beyond that no change
+constexpr double kDirectWaves = 3.0, kOnePassWaves = 4.0;
+
 // The fixed launch sequence of one enumeration.  timed: record an event
 // before every launch (and one after the last) on the same stream.
 static int enqueue(mpqp_plan *P, cudaStream_t s, bool timed)
@@ -562,6 +572,13 @@ static int enqueue(mpqp_plan *P, cudaStream_t s, bool timed)
         return MPQP_OK;
     };
 #define L(name, x) do { int _r = pre(name); if (_r) return _r; _r = chk(name, x); if (_r) return _r; } while (0)
+    // levels of mpQPs with a few sets per FP64 warp skip the FP32 screen: its
+    // three to five dependent launches cost such a level more than evaluating
+    // every set in FP64 at once.  Not with mpLP instances: their LP2 takes
+    // about 50 pivots over p + n + 2 columns
+    auto direct = [&](int level) {
+        return mixed && !P->has_lp && P->lvl_sets[level] <= kDirectWaves * 4.0 * P->grid_direct;
+    };
     // FP32 screen: the dual route and/or the primal route, each launched only
     // when some instance takes it; FP64: the optimality kernel
     auto launch_opt = [&](int level) -> int {
@@ -573,14 +590,24 @@ static int enqueue(mpqp_plan *P, cudaStream_t s, bool timed)
                   launch_optimality(B, P->tol, P->sd, level, true, P->grid_opt_lp, P->smem_opt, s));
             return MPQP_OK;
         }
+        if (direct(level)) {
+            L("k_optimality<double>",
+              launch_optimality(B, P->tol, P->sd, level, false, P->grid_direct, P->smem_optfb, s));
+            return MPQP_OK;
+        }
         const bool lanes = level <= kLaneMaxK && !B.lp2b[0] && (P->screen_dual || P->lanes_lp);
         if (lanes) {
+            // a level of a few waves of sets: one uncapped pass.  Its time is
+            // about that of its longest LPs, which three passes only add to
+            const bool one_pass = P->lvl_sets[level] <= kOnePassWaves * 32.0 * P->grid_lanes;
+            const int cap1 = one_pass ? 0 : P->lane_cap;
             L("k_opt_screen<dual,lanes>", launch_opt_screen_lanes(B, P->tol, P->sd, level, P->lp2_screen,
-                                                                  P->grid_lanes, P->smem_lanes, s, 0, P->lane_cap));
-            L("k_opt_screen<dual,lanes,rerun>", launch_opt_screen_lanes(B, P->tol, P->sd, level, P->lp2_screen,
-                                                                        P->grid_lanes, P->smem_lanes, s, 1,
-                                                                        P->lane_cap2));
-            if (P->lane_cap2 > 0)
+                                                                  P->grid_lanes, P->smem_lanes, s, 0, cap1));
+            if (!one_pass)
+                L("k_opt_screen<dual,lanes,rerun>", launch_opt_screen_lanes(B, P->tol, P->sd, level, P->lp2_screen,
+                                                                            P->grid_lanes, P->smem_lanes, s, 1,
+                                                                            P->lane_cap2));
+            if (!one_pass && P->lane_cap2 > 0)
                 L("k_opt_screen<dual,lanes,rerun2>", launch_opt_screen_lanes(B, P->tol, P->sd, level, P->lp2_screen,
                                                                              P->grid_lanes, P->smem_lanes, s, 2, 0));
             if (P->lanes_lp)
@@ -605,7 +632,7 @@ static int enqueue(mpqp_plan *P, cudaStream_t s, bool timed)
     };
     // FP64 re-evaluation of the sets the FP32 screen left undecided
     auto launch_optfb = [&](int level) -> int {
-        if (!mixed) return MPQP_OK;
+        if (!mixed || direct(level)) return MPQP_OK;
         if (P->has_qp)
             L("k_optimality_fp64",
               launch_optimality_fp64(B, P->tol, P->sd, level, false, P->grid_optfb, P->smem_optfb, s));
@@ -770,6 +797,7 @@ static int plan_create_locked(int n_inst, const mpqp_problem *probs, const mpqp_
                 if (k < P->desc[i].k_max) lvl_tab[k] += nk * (double)P->desc[i].tab_elems * (double)es;
             }
         }
+        P->lvl_sets = lvl;
         for (int k = 0; k <= kMaxK; k++) {
             lvl_max = std::max(lvl_max, lvl[k]);
             arena_max = std::max(arena_max, lvl_tab[k] + lvl_tab[k + 1]);
@@ -928,6 +956,7 @@ static int plan_create_locked(int n_inst, const mpqp_problem *probs, const mpqp_
         (rc = P->prec == PREC_MIXED ? grid_for(kernel_ptr("screen_dual_lanes"), P->smem_lanes, &P->grid_lanes, 32)
                                     : 0) ||
         (rc = grid_for(kernel_ptr("opt_fp64"), P->smem_optfb, &P->grid_optfb)) ||
+        (rc = P->prec == PREC_MIXED && !P->has_lp ? grid_for(kernel_ptr("opt64"), P->smem_optfb, &P->grid_direct) : 0) ||
         (rc = P->has_lp && P->prec != PREC_MIXED ? grid_for(kernel_ptr("opt64_lp"), P->smem_opt, &P->grid_opt_lp) : 0) ||
         (rc = P->has_lp ? grid_for(kernel_ptr("opt_fp64_lp"), P->smem_optfb, &P->grid_optfb_lp) : 0)) {
         free_plan_mem(P);

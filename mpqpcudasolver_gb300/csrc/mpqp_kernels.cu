@@ -2843,8 +2843,9 @@ __device__ void write_opt(const DevBuffers &B, const Node &nd, int level, const 
     }
 }
 
-// Final FP64 verdicts of every feasible set of a level (the FP64 path;
-// instantiated for T = double only).  LP = false takes the sets of mpQP
+// Final FP64 verdicts of every feasible set of a level (the FP64 path, and the
+// small levels of the mixed one, which have no FP32 screen; instantiated for
+// T = double only).  LP = false takes the sets of mpQP
 // instances, LP = true those of mpLP instances (launched only when a batch
 // has one), so that the mpQP kernel carries no mpLP code.
 template <typename T, bool LP>
@@ -2860,38 +2861,37 @@ __global__ void __launch_bounds__(128, kF64Blocks) k_optimality(DevBuffers B, To
     static_assert(sizeof(T) == 8, "the FP32 screen is k_opt_screen");
     LocalInstCounters lc;
     lc.reset(-1);
+    auto flush = [&]() {
+        if (lc.inst < 0 || lane != 0) return;
+        InstCtl *ic = &B.ictl[lc.inst];
+        atomicAdd((unsigned long long *)&ic->optimal, (unsigned long long)lc.a);
+        atomicAdd((unsigned long long *)&ic->region, (unsigned long long)lc.b);
+        atomicAdd((unsigned long long *)&ic->lp2_piv, (unsigned long long)lc.c);
+        atomicAdd((unsigned long long *)&ic->cheb_piv, (unsigned long long)lc.d);
+        if (B.precision == PREC_MIXED) atomicAdd((unsigned long long *)&ic->fb_opt, (unsigned long long)lc.e);
+    };
     for (;;) {
         long long x;
         if (lane == 0) x = (long long)atomicAdd(&ctl->ctr[LP ? 6 : 3], 1ull);
         x = __shfl_sync(FULLMASK, x, 0);
         if (x >= nn) break;
         const Node nd = B.node[side][x];
+        // (mixed precision: no first-stage basis for the children to start from)
+        if (B.lp2b[side] && lane == 0) B.lp2b[side][x] = ~0ull;
         if ((nd.flags & (NODE_VALID | NODE_FEASIBLE)) != (NODE_VALID | NODE_FEASIBLE)) continue;
         const InstDesc &I = B.inst[nd.inst];
         if (level < I.k_min || (I.lp != 0) != LP) continue;
-        if (nd.inst != lc.inst) {
-            if (lc.inst >= 0 && lane == 0) {
-                atomicAdd((unsigned long long *)&B.ictl[lc.inst].optimal, (unsigned long long)lc.a);
-                atomicAdd((unsigned long long *)&B.ictl[lc.inst].region, (unsigned long long)lc.b);
-                atomicAdd((unsigned long long *)&B.ictl[lc.inst].lp2_piv, (unsigned long long)lc.c);
-                atomicAdd((unsigned long long *)&B.ictl[lc.inst].cheb_piv, (unsigned long long)lc.d);
-            }
-            lc.reset(nd.inst);
-        }
+        if (nd.inst != lc.inst) { flush(); lc.reset(nd.inst); }
         const OptResult res = eval_optimality<T, LP>(B, tol, I, nd.lo, nd.hi, ws);
         lc.c += res.lp2_piv;
         lc.d += res.cheb_piv;
         lc.a += res.optimal;
         lc.b += res.region;
+        lc.e++;
         if (lane == 0) write_opt(B, nd, level, res, true);
         __syncwarp();
     }
-    if (lc.inst >= 0 && lane == 0) {
-        atomicAdd((unsigned long long *)&B.ictl[lc.inst].optimal, (unsigned long long)lc.a);
-        atomicAdd((unsigned long long *)&B.ictl[lc.inst].region, (unsigned long long)lc.b);
-        atomicAdd((unsigned long long *)&B.ictl[lc.inst].lp2_piv, (unsigned long long)lc.c);
-        atomicAdd((unsigned long long *)&B.ictl[lc.inst].cheb_piv, (unsigned long long)lc.d);
-    }
+    flush();
 }
 
 template <bool LP>
