@@ -92,7 +92,8 @@ struct Prepared {
     std::vector<double> WhL, wcL, Hm, cv;   // mpLP only: A H, A c, H, c
     std::vector<double> blo, bhi;   // parameter box, when At is [diag(+); diag(-)]
     std::vector<double> root;    // LP1 root tableau, FP64 stride ld1d
-    std::vector<double> root_f;  // the same values at the plan's stride ld1 (FP32 copy)
+    std::vector<double> root_f;  // the pre-pivoted root at the plan's stride ld1, then its ids (FP32 copy)
+    std::vector<double> root_p;  // its tableau at stride ld1d, FP64 (mixed precision)
 };
 
 static inline int odd_up(int x) { return (x & 1) ? x : x + 1; }
@@ -112,11 +113,13 @@ static inline int four_mod8_up(int x) { int y = (x + 3) & ~3; return (y & 4) ? y
 // (bid over M1, 255 past the live rows, then nid over nv); d.root_rows the
 // live rows.  Pivots in FP64: T_r /= T_rq (T_rq -> 1 / T_rq), then
 // T_i -= T_iq T_r (T_iq -> -T_iq / T_rq), the Tucker pivot of the kernels.
-static void prepivot_root_f(InstDesc &d, std::vector<double> &root_f)
+// Returns the largest |T_ij| any of the pivots left.
+static double prepivot_root_f(InstDesc &d, std::vector<double> &root_f)
 {
     const int ld = d.ld1, nv = d.nv, M1 = d.M1;
     std::vector<double> T(root_f.begin(), root_f.begin() + (size_t)(M1 + 1) * ld);
     std::vector<int> bid(M1), nid(nv);
+    double growth = 0.0;
     for (int i = 0; i < M1; i++) bid[i] = nv + i;
     for (int j = 0; j < nv; j++) nid[j] = j;
     for (int q = 0; q < nv; q++) {
@@ -151,6 +154,8 @@ static void prepivot_root_f(InstDesc &d, std::vector<double> &root_f)
             Ti[q] = -f * inv;
         }
         std::swap(bid[r], nid[q]);
+        for (int i = 0; i < M1; i++)
+            for (int j = 0; j < nv; j++) growth = std::max(growth, std::fabs(T[(size_t)i * ld + j]));
     }
     std::vector<double> out((size_t)d.tab_elems + M1 + nv, 0.0);
     int rows = 0;
@@ -165,6 +170,7 @@ static void prepivot_root_f(InstDesc &d, std::vector<double> &root_f)
     for (int j = 0; j < nv; j++) out[(size_t)d.tab_elems + M1 + j] = nid[j];
     root_f.swap(out);
     d.root_rows = rows;
+    return growth;
 }
 
 static void fwd_sub(const double *L, int n, const double *rhs, int rs, double *y, int ys)
@@ -184,6 +190,11 @@ static void bwd_sub(const double *L, int n, const double *y, int ysd, double *x,
         x[(size_t)i * xs] = acc / L[i * n + i];
     }
 }
+
+// largest entry growth of the host's pre-pivoting (FP64: errors of about 1e-16
+// times it, against the 1e-9 of tol_feas) with which the FP64 re-solves start
+// from the pre-pivoted root
+constexpr double kPrepivotGrowth = 1e4;
 
 static int prepare_instance(const mpqp_problem &P, Prepared &out, int prec)
 {
@@ -316,7 +327,16 @@ static int prepare_instance(const mpqp_problem &P, Prepared &out, int prec)
     };
     fill_root(out.root, d.ld1d);
     fill_root(out.root_f, d.ld1);
-    prepivot_root_f(d, out.root_f);
+    // the FP64 re-solves of the mixed path start from the same pre-pivoted
+    // tableau, unless its pivots grew the entries so far that starting from the
+    // constraint rows themselves is the safer FP64 arbiter
+    const double growth = prepivot_root_f(d, out.root_f);
+    if (prec == PREC_MIXED && growth <= kPrepivotGrowth) {
+        out.root_p.assign((size_t)(d.root_rows + 1) * d.ld1d, 0.0);
+        for (int i = 0; i <= d.root_rows; i++)
+            for (int j = 0; j <= d.nv; j++)
+                out.root_p[(size_t)i * d.ld1d + j] = out.root_f[(size_t)i * d.ld1 + j];
+    }
     // parameter box: row c reads s theta_c <= bt_c (s > 0), row p + c reads
     // s' theta_c <= bt_{p+c} (s' < 0), nothing else nonzero
     d.box = ncp == 2 * p;
@@ -742,6 +762,7 @@ static int plan_create_locked(int n_inst, const mpqp_problem *probs, const mpqp_
         d.f_Wm = put(fp, pr.Wm); d.f_Wh = put(fp, pr.Wh); d.f_wc = put(fp, pr.wc);
         d.f_At = put(fp, pr.At); d.f_bt = put(fp, pr.bt); d.f_root = put(fp, pr.root_f);
         d.f_blo = put(fp, pr.blo); d.f_bhi = put(fp, pr.bhi);
+        d.o_rootp = pr.root_p.empty() ? -1 : put(dp, pr.root_p);
         // mpLP: FP32 copies of the multiplier law's right-hand sides and of
         // the stationarity residual's data for the FP32 screen
         d.f_WhL = d.f_wcL = d.f_AT = d.f_Hm = d.f_cv = -1;

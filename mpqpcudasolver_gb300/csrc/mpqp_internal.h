@@ -70,6 +70,7 @@ struct InstDesc {
     // Hm = H, cv = c (the multiplier law and the stationarity residual)
     long long o_Wm, o_Wh, o_wc, o_At, o_bt, o_QiAT, o_QiH, o_Qic, o_root;
     long long o_WhL, o_wcL, o_Hm, o_cv;
+    long long o_rootp;          // the pre-pivoted LP1 root in FP64 (root_rows + 1 rows of ld1d), -1: none
     // offsets (elements) into the FP32 pool
     long long f_Wm, f_Wh, f_wc, f_At, f_bt, f_root;
     long long f_blo, f_bhi;     // parameter box lo <= theta <= hi (FP32), valid when box

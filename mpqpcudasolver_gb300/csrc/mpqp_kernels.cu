@@ -1210,10 +1210,11 @@ __device__ long long store_node(const DevBuffers &B, int side, int level, const 
             warp_copy_v<TT>(dst, (const TT *)tab, I.tab_elems);
         } else {
             // re-stride (and convert) row by row; padding columns become 0
-            const int ncol = I.nv + 1;
-            for (int e = lane; e < I.tab_elems; e += 32) {
+            // (rows_store >= 0: the live rows and the objective row after them)
+            const int ncol = I.nv + 1, last = rows_store >= 0 ? rows_store : I.M1;
+            for (int e = lane; e < (last + 1) * I.ld1; e += 32) {
                 const int i = e / I.ld1, j = e - i * I.ld1;
-                dst[e] = (i <= I.M1 && j < ncol) ? (TT)tab[(size_t)i * src_ld + j] : TT(0);
+                dst[e] = j < ncol ? (TT)tab[(size_t)i * src_ld + j] : TT(0);
             }
         }
         if (!bulk) {
@@ -1304,6 +1305,31 @@ __device__ __noinline__ void queue_undecided_lp1(const DevBuffers &B, int w, con
     if (qi < B.q_cap) B.q_lp1[qi] = w; else atomicOr(&ctl->overflow, OV_QUEUE);
 }
 
+// obj += sum over i in (lo, hi) of w_i, in the basis of the tableau (nrows
+// rows, nv columns): a basic slack's row, -1 in a nonbasic slack's column; in
+// ascending i, from the objective row as it is.
+template <typename T>
+__device__ __forceinline__ void add_set_objective(const T *tab, int ld, int rows, int nv, const uint8_t *bid,
+                                                  const uint8_t *nid, T *obj, uint64_t lo, uint64_t hi)
+{
+    const int lane = lane_id();
+    while (lo | hi) {
+        int i;
+        if (lo) { i = __ffsll((long long)lo) - 1; lo &= lo - 1; }
+        else { i = 64 + __ffsll((long long)hi) - 1; hi &= hi - 1; }
+        int rho = -1;
+        for (int r = lane; r < rows; r += 32) if (bid[r] == nv + i) rho = r;
+        rho = __reduce_max_sync(FULLMASK, rho);
+        if (rho >= 0) {
+            const T *row = tab + (size_t)rho * ld;
+            for (int cc = lane; cc <= nv; cc += 32) obj[cc] = xadd(obj[cc], row[cc]);
+        } else {
+            for (int cc = lane; cc < nv; cc += 32) if (nid[cc] == nv + i) obj[cc] = obj[cc] - T(1);
+        }
+        __syncwarp();
+    }
+}
+
 // LP1 of S' = S u {j} started from the root tableau (all slacks basic) when
 // the parent kept no tableau: the root copied into the warp's slot (after
 // the previous child's bulk store has read it), the root basis ids, and the
@@ -1333,24 +1359,8 @@ __device__ __forceinline__ void cold_stage_lp1_body(const DevBuffers &B, const I
         for (int c = lane; c < nv; c += 32) nid[c] = (uint8_t)c;
     }
     __syncwarp();
-    T *obj = tab + (size_t)rows * ld;
     if (j < 64) lo |= 1ull << j; else hi |= 1ull << (j - 64);
-    while (lo | hi) {
-        int i;
-        if (lo) { i = __ffsll((long long)lo) - 1; lo &= lo - 1; }
-        else { i = 64 + __ffsll((long long)hi) - 1; hi &= hi - 1; }
-        // w_i basic: its row joins the objective; nonbasic: -1 in its column
-        int rho = -1;
-        for (int r = lane; r < rows; r += 32) if (bid[r] == nv + i) rho = r;
-        rho = __reduce_max_sync(FULLMASK, rho);
-        if (rho >= 0) {
-            const T *row = tab + (size_t)rho * ld;
-            for (int cc = lane; cc <= nv; cc += 32) obj[cc] = xadd(obj[cc], row[cc]);
-        } else {
-            for (int cc = lane; cc < nv; cc += 32) if (nid[cc] == nv + i) obj[cc] = obj[cc] - T(1);
-        }
-        __syncwarp();
-    }
+    add_set_objective(tab, ld, rows, nv, bid, nid, tab + (size_t)rows * ld, lo, hi);
 }
 
 __device__ __noinline__ void cold_stage_lp1_f32(const DevBuffers &B, const InstDesc &I, int inst, float *tab,
@@ -1701,6 +1711,12 @@ __global__ void __launch_bounds__(128, kF64Blocks) k_feasibility_f64(DevBuffers 
 // ---------------------------------------------------------------------
 // K2b: FP64 LP1 re-solve (mixed precision), cold from the root tableau
 // ---------------------------------------------------------------------
+// Bound by the FP64 pipe.  It starts from the pre-pivoted root (every free
+// variable basic, its row dropped: m + ncp - nv rows) where the host found that
+// root's entry growth small: 54 rows instead of 78 on the ill-conditioned
+// n = 16, m = 62, p = 8 problem, so two row slots instead of three, and no
+// pivots spent on bringing the free variables in.  36.5K re-solves 2,012 ->
+// 1,200 us, and LP1 of their children (fewer rows) 432 -> 318 us.
 __global__ void __launch_bounds__(128, kF64Blocks) k_lp1_fp64(DevBuffers B, Tol tol, SlotDims sd, int level)
 {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -1726,21 +1742,21 @@ __global__ void __launch_bounds__(128, kF64Blocks) k_lp1_fp64(DevBuffers B, Tol 
         const int M1 = I.M1, nv = I.nv, ld = I.ld1d;
         uint64_t lo = par.lo, hi = par.hi;
         if (c.j < 64) lo |= 1ull << c.j; else hi |= 1ull << (c.j - 64);
-        const double *root = B.dpool + I.o_root;
-        warp_copy<double, double>(tab, root, (M1 + 1) * ld);
         uint8_t *bid = ids, *nid = ids + M1;
-        for (int i = lane; i < M1; i += 32) bid[i] = (uint8_t)(nv + i);
-        for (int j = lane; j < nv; j += 32) nid[j] = (uint8_t)j;
-        __syncwarp();
-        double *obj = tab + (size_t)M1 * ld;
-        for (int cc = lane; cc <= nv; cc += 32) {
-            double acc = 0.0;
-            for (int i = 0; i < I.m; i++)
-                if (mask_has(lo, hi, i)) acc = __dadd_rn(acc, root[(size_t)i * ld + cc]);
-            obj[cc] = acc;
+        const bool pre = I.o_rootp >= 0;
+        const int rows = pre ? I.root_rows : M1;
+        warp_copy<double, double>(tab, B.dpool + (pre ? I.o_rootp : I.o_root), (rows + 1) * ld);
+        if (pre) {
+            const float *rid = B.fpool + I.f_root + I.tab_elems;
+            for (int i = lane; i < M1 + nv; i += 32) ids[i] = (uint8_t)(int)rid[i];
+        } else {
+            for (int i = lane; i < M1; i += 32) bid[i] = (uint8_t)(nv + i);
+            for (int j = lane; j < nv; j += 32) nid[j] = (uint8_t)j;
         }
         __syncwarp();
-        Lp<double> L{tab, ld, M1, nv, nv, bid, nid};
+        double *obj = tab + (size_t)rows * ld;
+        add_set_objective(tab, ld, rows, nv, bid, nid, obj, lo, hi);
+        Lp<double> L{tab, ld, rows, nv, nv, bid, nid};
         int piv = 0;
         const int st = warp_simplex_f64(L, tol.tol_piv, tol.tol_dj, tol.max_pivots, tol.degen_switch, &piv);
         const double z = obj[nv];
@@ -1760,7 +1776,7 @@ __global__ void __launch_bounds__(128, kF64Blocks) k_lp1_fp64(DevBuffers B, Tol 
         }
         if (feasible || B.exhaustive)
             store_node<float, double>(B, side, level, I, inst, lo, hi, feasible, tab, ids, rec, hcap, 0, I.ld1d, false,
-                                      w);
+                                      w, rows);
     }
 }
 
