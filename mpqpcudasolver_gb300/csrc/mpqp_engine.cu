@@ -565,31 +565,48 @@ static int grid_for(const void *fn, size_t smem, int *grid, int block = 128)
 // (592K) 2,566, 2,284 and 2,280 us; beyond that no change
 constexpr double kDirectWaves = 3.0, kOnePassWaves = 4.0;
 
-// The fixed launch sequence of one enumeration.  timed: record an event
-// before every launch (and one after the last) on the same stream.
-static int enqueue(mpqp_plan *P, cudaStream_t s, bool timed)
+// The fixed launch sequence of one enumeration.  events: none; one before every
+// launch (and one after the last), for the per-kernel times; or one wherever
+// the sequence changes between its LP1 and its optimality phase (phase_times).
+enum EventMode { EV_NONE, EV_LAUNCHES, EV_PHASES };
+
+static bool is_opt_phase(const char *kernel) { return !strncmp(kernel, "k_opt", 5); }
+
+static int enqueue(mpqp_plan *P, cudaStream_t s, EventMode events)
 {
     const DevBuffers &B = P->B;
     const bool mixed = P->prec == PREC_MIXED;
     const char *feas = mixed ? "k_feasibility<float>" : "k_feasibility<double>";
-    int nl = 0;
-    if (timed) P->kname.clear();
+    int nl = 0, ne = 0;
+    if (events != EV_NONE) P->kname.clear();
     auto chk = [&](const char *name, cudaError_t e) -> int {
         if (e != cudaSuccess) { set_err(std::string("launch of ") + name + ": " + cudaGetErrorString(e)); return MPQP_ECUDA; }
         return MPQP_OK;
     };
-    auto pre = [&](const char *name) -> int {
-        if (timed) {
-            if ((int)P->kev.size() <= nl) {
-                cudaEvent_t e;
-                if (cudaEventCreate(&e) != cudaSuccess) { set_err("cudaEventCreate"); return MPQP_ECUDA; }
-                P->kev.push_back(e);
-            }
-            if (cudaEventRecord(P->kev[nl], s) != cudaSuccess) { set_err("cudaEventRecord"); return MPQP_ECUDA; }
-            P->kname.push_back(name);
+    auto record = [&]() -> int {
+        if ((int)P->kev.size() <= ne) {
+            cudaEvent_t e;
+            if (cudaEventCreate(&e) != cudaSuccess) { set_err("cudaEventCreate"); return MPQP_ECUDA; }
+            P->kev.push_back(e);
         }
-        nl++;
+        if (cudaEventRecord(P->kev[ne], s) != cudaSuccess) { set_err("cudaEventRecord"); return MPQP_ECUDA; }
+        ne++;
         return MPQP_OK;
+    };
+    auto pre = [&](const char *name) -> int {
+        nl++;
+        if (events == EV_NONE) return MPQP_OK;
+        if (events == EV_PHASES && !P->kname.empty() && is_opt_phase(P->kname.back()) == is_opt_phase(name)) return MPQP_OK;
+        P->kname.push_back(name);
+        return record();
+    };
+    // A level's grids: the persistent grid, or fewer blocks where the level
+    // cannot have that many items.  Every warp of a grid reads its queue's
+    // counter with an atomic before it can exit: thousands of warps on one
+    // address for a level of a hundred sets.
+    auto grid = [&](int full, int level, int per_block) -> int {
+        const double need = std::ceil(P->lvl_sets[level] / per_block);
+        return need < 1.0 ? 1 : need < full ? (int)need : full;
     };
 #define L(name, x) do { int _r = pre(name); if (_r) return _r; _r = chk(name, x); if (_r) return _r; } while (0)
     // levels of mpQPs with a few sets per FP64 warp skip the FP32 screen: its
@@ -604,15 +621,17 @@ static int enqueue(mpqp_plan *P, cudaStream_t s, bool timed)
     auto launch_opt = [&](int level) -> int {
         if (!mixed) {
             if (P->has_qp)
-                L("k_optimality<double>", launch_optimality(B, P->tol, P->sd, level, false, P->grid_opt, P->smem_opt, s));
+                L("k_optimality<double>",
+                  launch_optimality(B, P->tol, P->sd, level, false, grid(P->grid_opt, level, 4), P->smem_opt, s));
             if (P->has_lp)
                 L("k_optimality<double,mplp>",
-                  launch_optimality(B, P->tol, P->sd, level, true, P->grid_opt_lp, P->smem_opt, s));
+                  launch_optimality(B, P->tol, P->sd, level, true, grid(P->grid_opt_lp, level, 4), P->smem_opt, s));
             return MPQP_OK;
         }
         if (direct(level)) {
             L("k_optimality<double>",
-              launch_optimality(B, P->tol, P->sd, level, false, P->grid_direct, P->smem_optfb, s));
+              launch_optimality(B, P->tol, P->sd, level, false, grid(P->grid_direct, level, 4), P->smem_optfb,
+                                s));
             return MPQP_OK;
         }
         const bool lanes = level <= kLaneMaxK && !B.lp2b[0] && (P->screen_dual || P->lanes_lp);
@@ -622,32 +641,36 @@ static int enqueue(mpqp_plan *P, cudaStream_t s, bool timed)
             const bool one_pass = P->lvl_sets[level] <= kOnePassWaves * 32.0 * P->grid_lanes;
             const int cap1 = one_pass ? 0 : P->lane_cap;
             L("k_opt_screen<dual,lanes>", launch_opt_screen_lanes(B, P->tol, P->sd, level, P->lp2_screen,
-                                                                  P->grid_lanes, P->smem_lanes, s, 0, cap1));
+                                                                  grid(P->grid_lanes, level, 32), P->smem_lanes, s, 0,
+                                                                  cap1));
             if (!one_pass)
                 L("k_opt_screen<dual,lanes,rerun>", launch_opt_screen_lanes(B, P->tol, P->sd, level, P->lp2_screen,
-                                                                            P->grid_lanes, P->smem_lanes, s, 1,
+                                                                            grid(P->grid_lanes, level, 32), P->smem_lanes, s, 1,
                                                                             P->lane_cap2));
             if (!one_pass && P->lane_cap2 > 0)
                 L("k_opt_screen<dual,lanes,rerun2>", launch_opt_screen_lanes(B, P->tol, P->sd, level, P->lp2_screen,
-                                                                             P->grid_lanes, P->smem_lanes, s, 2, 0));
+                                                                             grid(P->grid_lanes, level, 32), P->smem_lanes, s, 2, 0));
             if (P->lanes_lp)
                 L("k_opt_screen<dual,stationarity>", launch_opt_screen(B, P->tol, P->sd, level, P->lp2_screen, 3,
-                                                                       P->grid_tiles, P->smem_tiles, s, P->tile_w));
+                                                                       grid(P->grid_tiles, level, 32 / P->tile_w),
+                                                                       P->smem_tiles, s, P->tile_w));
         }
         if (!lanes && (P->screen_dual || P->lanes_lp))
-            L("k_opt_screen<dual>", launch_opt_screen(B, P->tol, P->sd, level, P->lp2_screen, 0, P->grid_tiles,
-                                                      P->smem_tiles, s, P->tile_w));
+            L("k_opt_screen<dual>", launch_opt_screen(B, P->tol, P->sd, level, P->lp2_screen, 0,
+                                                      grid(P->grid_tiles, level, 32 / P->tile_w), P->smem_tiles, s,
+                                                      P->tile_w));
         if (P->lanes_lp)
             L("k_opt_screen<dual,rows,mplp>",
-              launch_opt_screen(B, P->tol, P->sd, level, P->lp2_screen, 6, P->grid_opt_lprows, P->smem_opt, s,
-                                P->tile_w));
+              launch_opt_screen(B, P->tol, P->sd, level, P->lp2_screen, 6, grid(P->grid_opt_lprows, level, 1),
+                                P->smem_opt, s, P->tile_w));
         if (P->screen_dual) {
             L("k_opt_screen<dual,rows>",
-              launch_opt_screen(B, P->tol, P->sd, level, P->lp2_screen, 2, P->grid_opt3, P->smem_opt, s, P->tile_w));
+              launch_opt_screen(B, P->tol, P->sd, level, P->lp2_screen, 2, grid(P->grid_opt3, level, 1), P->smem_opt, s,
+                                P->tile_w));
         }
         if (P->screen_primal)
-            L("k_opt_screen<primal>", launch_opt_screen(B, P->tol, P->sd, level, P->lp2_screen, 1, P->grid_opt2, P->smem_opt2, s,
-                                                        P->tile_w));
+            L("k_opt_screen<primal>", launch_opt_screen(B, P->tol, P->sd, level, P->lp2_screen, 1,
+                                                        grid(P->grid_opt2, level, 1), P->smem_opt2, s, P->tile_w));
         return MPQP_OK;
     };
     // FP64 re-evaluation of the sets the FP32 screen left undecided
@@ -655,10 +678,11 @@ static int enqueue(mpqp_plan *P, cudaStream_t s, bool timed)
         if (!mixed || direct(level)) return MPQP_OK;
         if (P->has_qp)
             L("k_optimality_fp64",
-              launch_optimality_fp64(B, P->tol, P->sd, level, false, P->grid_optfb, P->smem_optfb, s));
+              launch_optimality_fp64(B, P->tol, P->sd, level, false, grid(P->grid_optfb, level, 4), P->smem_optfb, s));
         if (P->has_lp)
             L("k_optimality_fp64<mplp>",
-              launch_optimality_fp64(B, P->tol, P->sd, level, true, P->grid_optfb_lp, P->smem_optfb, s));
+              launch_optimality_fp64(B, P->tol, P->sd, level, true, grid(P->grid_optfb_lp, level, 4), P->smem_optfb,
+                                     s));
         return MPQP_OK;
     };
     L("k_reset", launch_reset(B, s));
@@ -667,26 +691,19 @@ static int enqueue(mpqp_plan *P, cudaStream_t s, bool timed)
     { const int _o = launch_optfb(0); if (_o) return _o; }
     L("k_finalize", launch_finalize(B, 0, s));
     for (int k = 1; k <= P->kmax; k++) {
-        L("k_enumerate", launch_enumerate(B, k, P->grid_enum, s));
-        L(feas, launch_feasibility(B, P->tol, P->sd, k, P->prec, P->grid_feas, P->smem_feas, s, P->feas_warps,
-                                   P->feas_chunk));
+        L("k_enumerate", launch_enumerate(B, k, grid(P->grid_enum, k - 1, 4), s));
+        L(feas, launch_feasibility(B, P->tol, P->sd, k, P->prec, grid(P->grid_feas, k, P->feas_warps), P->smem_feas, s,
+                                   P->feas_warps, P->feas_chunk));
         if (mixed) {
-            L("k_lp1_cert", launch_lp1_cert(B, P->tol, P->sd, k, P->grid_cert, P->smem_cert, s));
-            L("k_lp1_fp64", launch_lp1_fp64(B, P->tol, P->sd, k, P->grid_lp1fb, P->smem_lp1fb, s));
+            L("k_lp1_cert", launch_lp1_cert(B, P->tol, P->sd, k, grid(P->grid_cert, k, 4), P->smem_cert, s));
+            L("k_lp1_fp64", launch_lp1_fp64(B, P->tol, P->sd, k, grid(P->grid_lp1fb, k, 4), P->smem_lp1fb, s));
         }
         { const int _o = launch_opt(k); if (_o) return _o; }
         { const int _o = launch_optfb(k); if (_o) return _o; }
         L("k_finalize", launch_finalize(B, k, s));
     }
 #undef L
-    if (timed) {
-        if ((int)P->kev.size() <= nl) {
-            cudaEvent_t e;
-            if (cudaEventCreate(&e) != cudaSuccess) { set_err("cudaEventCreate"); return MPQP_ECUDA; }
-            P->kev.push_back(e);
-        }
-        if (cudaEventRecord(P->kev[nl], s) != cudaSuccess) { set_err("cudaEventRecord"); return MPQP_ECUDA; }
-    }
+    if (events != EV_NONE) { const int _r = record(); if (_r) return _r; }
     P->n_launches = nl;
     return MPQP_OK;
 }
@@ -991,7 +1008,7 @@ static int plan_create_locked(int n_inst, const mpqp_problem *probs, const mpqp_
         cudaStream_t cs;
         CK(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
         CK(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
-        rc = enqueue(P, cs, false);
+        rc = enqueue(P, cs, EV_NONE);
         cudaGraph_t g = nullptr;
         cudaError_t e = cudaStreamEndCapture(cs, &g);
         cudaStreamDestroy(cs);
@@ -1036,7 +1053,7 @@ struct TuneKey {
     }
 };
 struct TuneEntry { TuneKey key; int tile_w, feas_warps, feas_chunk; };
-static int mpqp_plan_run_timed_impl(mpqp_plan *P, void *stream);
+static int mpqp_plan_run_timed_impl(mpqp_plan *P, void *stream, EventMode events);
 static std::vector<TuneEntry> g_tune_cache;   // guarded by g_mu
 
 static TuneKey tune_key(int n_inst, const mpqp_problem *probs, const mpqp_options &o)
@@ -1065,7 +1082,7 @@ static double tune_trial(int n_inst, const mpqp_problem *slice, const mpqp_optio
     if (plan_create_locked(n_inst, slice, &o, &P) != MPQP_OK) { cudaGetLastError(); return -1.0; }
     double best = -1.0;
     for (int rep = 0; rep < runs; rep++) {
-        if (mpqp_plan_run_timed_impl(P, nullptr) != MPQP_OK) { best = -1.0; break; }
+        if (mpqp_plan_run_timed_impl(P, nullptr, EV_LAUNCHES) != MPQP_OK) { best = -1.0; break; }
         if (cudaEventSynchronize(P->ev1) != cudaSuccess) { cudaGetLastError(); best = -1.0; break; }
         double ms = 0.0;
         for (size_t i = 0; i < P->kname.size(); i++) {
@@ -1173,7 +1190,7 @@ static int mpqp_plan_run_impl(mpqp_plan *P, void *stream)
     if (P->exec) {
         CK(cudaGraphLaunch(P->exec, s));
     } else {
-        int rc = enqueue(P, s, true);
+        int rc = enqueue(P, s, EV_NONE);
         if (rc) return rc;
     }
     CK(cudaEventRecord(P->ev1, s));
@@ -1192,12 +1209,12 @@ extern "C" int mpqp_plan_run(mpqp_plan *P, void *stream)
 
 extern "C" int mpqp_plan_launches(const mpqp_plan *P) { return P ? P->n_launches : 0; }
 
-static int mpqp_plan_run_timed_impl(mpqp_plan *P, void *stream)
+static int mpqp_plan_run_timed_impl(mpqp_plan *P, void *stream, EventMode events)
 {
     if (!P) return MPQP_EINVAL;
     cudaStream_t s = (cudaStream_t)stream;
     CK(cudaEventRecord(P->ev0, s));
-    int rc = enqueue(P, s, true);
+    int rc = enqueue(P, s, events);
     if (rc) return rc;
     CK(cudaEventRecord(P->ev1, s));
     P->ran = true;
@@ -1208,7 +1225,7 @@ static int mpqp_plan_run_timed_impl(mpqp_plan *P, void *stream)
 extern "C" int mpqp_plan_run_timed(mpqp_plan *P, void *stream)
 {
     try {
-        return mpqp_plan_run_timed_impl(P, stream);
+        return mpqp_plan_run_timed_impl(P, stream, EV_LAUNCHES);
     } catch (...) {
         return host_failure("mpqp_plan_run_timed");
     }
@@ -1261,7 +1278,7 @@ static int phase_times(mpqp_plan *P, double *feas_ms, double *opti_ms)
     for (size_t i = 0; i < P->kname.size(); i++) {
         float e = 0;
         CK(cudaEventElapsedTime(&e, P->kev[i], P->kev[i + 1]));
-        if (!strncmp(P->kname[i], "k_opt", 5)) *opti_ms += e; else *feas_ms += e;
+        if (is_opt_phase(P->kname[i])) *opti_ms += e; else *feas_ms += e;
     }
     return MPQP_OK;
 }
@@ -1515,7 +1532,11 @@ extern "C" int mpqp_solve_batch(int n_inst, const mpqp_problem *probs, const mpq
 {
     *out = nullptr;
     mpqp_plan *P = nullptr;
-    int rc = mpqp_plan_create(n_inst, probs, opt, &P);
+    // one run: capturing and instantiating a graph costs more than its launch saves
+    mpqp_options o;
+    if (opt) o = *opt; else mpqp_default_options(&o);
+    o.use_graph = 0;
+    int rc = mpqp_plan_create(n_inst, probs, &o, &P);
     if (rc) return rc;
     rc = mpqp_plan_run(P, nullptr);
     if (!rc) rc = mpqp_plan_results(P, out);
@@ -1755,8 +1776,8 @@ static GPUResults *mpqp_impl(const double *AxT, int n_c, int n_x, int n_t, int k
     o.precision = MPQP_MIXED;
     const char *env = getenv("MPQP_PRECISION");
     if (env && (!strcmp(env, "fp64") || !strcmp(env, "0"))) o.precision = MPQP_FP64;
-    // one run: launched without a graph, with an event before every launch,
-    // so that the device time splits into its LP1 and optimality phases
+    // one run: launched without a graph, with an event wherever the phase
+    // changes, so that the device time splits into LP1 and optimality
     o.use_graph = 0;
     // MPQP_ARENA_BYTES: a cap on the LP1 tableau arena (levels beyond it are
     // split: see n_splits)
@@ -1775,7 +1796,7 @@ static GPUResults *mpqp_impl(const double *AxT, int n_c, int n_x, int n_t, int k
     {
         mpqp_plan *P = nullptr;
         rc = mpqp_plan_create(1, &pr, &o, &P);
-        if (!rc) rc = mpqp_plan_run_timed(P, nullptr);
+        if (!rc) rc = mpqp_plan_run_timed_impl(P, nullptr, EV_PHASES);
         if (!rc) rc = mpqp_plan_results(P, &R);
         if (!rc) rc = phase_times(P, &feas_ms, &opti_ms);
         mpqp_plan_destroy(P);
