@@ -83,6 +83,28 @@ void set_error_text(const char *msg) { set_err(msg ? msg : ""); }
         }                                                                                              \
     } while (0)
 
+// f(0) .. f(T-1) on up to T threads (the calling thread included); when a
+// thread cannot be started, the calling thread runs the rest.  An exception
+// of any f(t) is rethrown in the calling thread once all have finished.
+template <typename F>
+static void run_parallel(unsigned T, F f)
+{
+    std::vector<std::exception_ptr> err(T);
+    auto guarded = [&](unsigned t) {
+        try { f(t); } catch (...) { err[t] = std::current_exception(); }
+    };
+    std::vector<std::thread> th;
+    try {
+        for (unsigned t = 1; t < T; t++) th.emplace_back(guarded, t);
+    } catch (...) {
+    }
+    guarded(0u);
+    for (unsigned t = (unsigned)th.size() + 1; t < T; t++) guarded(t);
+    for (std::thread &x : th) x.join();
+    for (const std::exception_ptr &e : err)
+        if (e) std::rethrow_exception(e);
+}
+
 // ---------------------------------------------------------------------
 // FP64 precompute (operation order identical to the CPU oracle)
 // ---------------------------------------------------------------------
@@ -113,7 +135,7 @@ static inline int four_mod8_up(int x) { int y = (x + 3) & ~3; return (y & 4) ? y
 // (bid over M1, 255 past the live rows, then nid over nv); d.root_rows the
 // live rows.  Pivots in FP64: T_r /= T_rq (T_rq -> 1 / T_rq), then
 // T_i -= T_iq T_r (T_iq -> -T_iq / T_rq), the Tucker pivot of the kernels.
-// Returns the largest |T_ij| any of the pivots left.
+// Returns the entry growth: the largest multiplier of a pivot or |T_ij| left.
 static double prepivot_root_f(InstDesc &d, std::vector<double> &root_f)
 {
     const int ld = d.ld1, nv = d.nv, M1 = d.M1;
@@ -143,20 +165,21 @@ static double prepivot_root_f(InstDesc &d, std::vector<double> &root_f)
         if (r < 0) continue;
         double *R = T.data() + (size_t)r * ld;
         const double inv = 1.0 / R[q];
-        for (int j = 0; j <= nv; j++) if (j != q) R[j] *= inv;
+        for (int j = 0; j <= nv; j++) R[j] *= inv;
         R[q] = inv;
         for (int i = 0; i <= M1; i++) {
             if (i == r) continue;
             double *Ti = T.data() + (size_t)i * ld;
             const double f = Ti[q];
             if (f == 0.0) continue;
-            for (int j = 0; j <= nv; j++) if (j != q) Ti[j] -= f * R[j];
+            for (int j = 0; j <= nv; j++) Ti[j] -= f * R[j];
             Ti[q] = -f * inv;
         }
         std::swap(bid[r], nid[q]);
-        for (int i = 0; i < M1; i++)
-            for (int j = 0; j < nv; j++) growth = std::max(growth, std::fabs(T[(size_t)i * ld + j]));
+        growth = std::max(growth, cmax * std::fabs(inv));
     }
+    for (int i = 0; i < M1; i++)
+        for (int j = 0; j < nv; j++) growth = std::max(growth, std::fabs(T[(size_t)i * ld + j]));
     std::vector<double> out((size_t)d.tab_elems + M1 + nv, 0.0);
     int rows = 0;
     for (int i = 0; i < M1; i++) {
@@ -173,21 +196,44 @@ static double prepivot_root_f(InstDesc &d, std::vector<double> &root_f)
     return growth;
 }
 
-static void fwd_sub(const double *L, int n, const double *rhs, int rs, double *y, int ys)
+// Y = L^-1 Y and X = L^-T X for n x w right-hand sides, row by row: each entry
+// accumulates in the oracle's order, all w entries of a row together
+static void fwd_sub(const double *L, int n, double *Y, int w)
 {
     for (int i = 0; i < n; i++) {
-        double acc = rhs[(size_t)i * rs];
-        for (int l = 0; l < i; l++) acc = std::fma(-L[i * n + l], y[(size_t)l * ys], acc);
-        y[(size_t)i * ys] = acc / L[i * n + i];
+        double *Yi = Y + (size_t)i * w;
+        for (int l = 0; l < i; l++) {
+            const double f = -L[i * n + l], *Yl = Y + (size_t)l * w;
+            for (int c = 0; c < w; c++) Yi[c] = std::fma(f, Yl[c], Yi[c]);
+        }
+        const double d = L[i * n + i];
+        for (int c = 0; c < w; c++) Yi[c] = Yi[c] / d;
     }
 }
 
-static void bwd_sub(const double *L, int n, const double *y, int ysd, double *x, int xs)
+static void bwd_sub(const double *L, int n, double *X, int w)
 {
     for (int i = n - 1; i >= 0; i--) {
-        double acc = y[(size_t)i * ysd];
-        for (int l = i + 1; l < n; l++) acc = std::fma(-L[l * n + i], x[(size_t)l * xs], acc);
-        x[(size_t)i * xs] = acc / L[i * n + i];
+        double *Xi = X + (size_t)i * w;
+        for (int l = i + 1; l < n; l++) {
+            const double f = -L[l * n + i], *Xl = X + (size_t)l * w;
+            for (int c = 0; c < w; c++) Xi[c] = std::fma(f, Xl[c], Xi[c]);
+        }
+        const double d = L[i * n + i];
+        for (int c = 0; c < w; c++) Xi[c] = Xi[c] / d;
+    }
+}
+
+// out[r][c] += sum over i of V[i][r] U[i][c] (V n x m, U n x w), each entry in
+// ascending i; `out` holds the start values
+static void add_products(const double *V, int m, const double *U, int w, int n, double *out)
+{
+    for (int r = 0; r < m; r++) {
+        double *o = out + (size_t)r * w;
+        for (int i = 0; i < n; i++) {
+            const double v = V[(size_t)i * m + r], *u = U + (size_t)i * w;
+            for (int c = 0; c < w; c++) o[c] = std::fma(v, u[c], o[c]);
+        }
     }
 }
 
@@ -235,6 +281,9 @@ static int prepare_instance(const mpqp_problem &P, Prepared &out, int prec)
     d.lp = 1;
     for (int i = 0; i < n * n && d.lp; i++) if (P.Q[i] != 0.0) d.lp = 0;
     d.ld2lp = odd_up(p + n + 3);
+    std::vector<double> AT((size_t)n * m);
+    for (int r = 0; r < m; r++)
+        for (int i = 0; i < n; i++) AT[(size_t)i * m + r] = P.A[(size_t)r * n + i];
     if (d.lp) {
         // mpLP (Q = 0): Wm = A A^T, Wh = F, wc = b, QiAT = A^T, QiH = Qic = 0,
         // WhL = A H, wcL = A c (each sum over ascending i from 0, the oracle's order)
@@ -242,74 +291,49 @@ static int prepare_instance(const mpqp_problem &P, Prepared &out, int prec)
             set_err("mpLP instance too large for 8-bit basis ids (m + ncp + 3n + p must be <= 252)");
             return MPQP_EINVAL;
         }
-        out.Wm.assign((size_t)m * m, 0.0);
         out.Wh.assign(P.F, P.F + (size_t)m * p);
         out.wc.assign(P.b, P.b + m);
-        out.WhL.assign((size_t)m * p, 0.0);
-        out.wcL.assign(m, 0.0);
-        out.QiAT.assign((size_t)n * m, 0.0);
+        out.QiAT = AT;
         out.QiH.assign((size_t)n * p, 0.0);
         out.Qic.assign(n, 0.0);
         out.Hm.assign(P.H, P.H + (size_t)n * p);
         out.cv.assign(P.c, P.c + n);
-        for (int r = 0; r < m; r++) {
-            for (int s = 0; s < m; s++) {
-                double acc = 0.0;
-                for (int i = 0; i < n; i++) acc = std::fma(P.A[(size_t)r * n + i], P.A[(size_t)s * n + i], acc);
-                out.Wm[(size_t)r * m + s] = acc;
-            }
-            for (int c = 0; c < p; c++) {
-                double acc = 0.0;
-                for (int i = 0; i < n; i++) acc = std::fma(P.A[(size_t)r * n + i], P.H[(size_t)i * p + c], acc);
-                out.WhL[(size_t)r * p + c] = acc;
-            }
-            double acc = 0.0;
-            for (int i = 0; i < n; i++) acc = std::fma(P.A[(size_t)r * n + i], P.c[i], acc);
-            out.wcL[r] = acc;
-            for (int i = 0; i < n; i++) out.QiAT[(size_t)i * m + r] = P.A[(size_t)r * n + i];
-        }
-    }
-    std::vector<double> L((size_t)n * n, 0.0), V((size_t)n * m, 0.0), U((size_t)n * p, 0.0), u(n, 0.0);
-    for (int j = 0; j < n && !d.lp; j++) {
-        for (int i = j; i < n; i++) {
-            double acc = P.Q[i * n + j];
-            for (int l = 0; l < j; l++) acc = std::fma(-L[i * n + l], L[j * n + l], acc);
-            if (i == j) {
-                if (!(acc > 0.0)) { set_err("Q is neither positive definite nor zero"); return MPQP_ENOTSPD; }
-                L[j * n + j] = std::sqrt(acc);
-            } else {
-                L[i * n + j] = acc / L[j * n + j];
+        out.Wm.assign((size_t)m * m, 0.0);
+        out.WhL.assign((size_t)m * p, 0.0);
+        out.wcL.assign(m, 0.0);
+        add_products(AT.data(), m, AT.data(), m, n, out.Wm.data());
+        add_products(AT.data(), m, P.H, p, n, out.WhL.data());
+        add_products(AT.data(), m, P.c, 1, n, out.wcL.data());
+    } else {
+        std::vector<double> L((size_t)n * n, 0.0);
+        for (int j = 0; j < n; j++) {
+            for (int i = j; i < n; i++) {
+                double acc = P.Q[i * n + j];
+                for (int l = 0; l < j; l++) acc = std::fma(-L[i * n + l], L[j * n + l], acc);
+                if (i == j) {
+                    if (!(acc > 0.0)) { set_err("Q is neither positive definite nor zero"); return MPQP_ENOTSPD; }
+                    L[j * n + j] = std::sqrt(acc);
+                } else {
+                    L[i * n + j] = acc / L[j * n + j];
+                }
             }
         }
-    }
-    if (!d.lp) {
-    for (int r = 0; r < m; r++) fwd_sub(L.data(), n, P.A + (size_t)r * n, 1, V.data() + r, m);
-    for (int c = 0; c < p; c++) fwd_sub(L.data(), n, P.H + c, p, U.data() + c, p);
-    fwd_sub(L.data(), n, P.c, 1, u.data(), 1);
-    out.Wm.assign((size_t)m * m, 0.0);
-    out.Wh.assign((size_t)m * p, 0.0);
-    out.wc.assign(m, 0.0);
-    for (int r = 0; r < m; r++) {
-        for (int s = 0; s < m; s++) {
-            double acc = 0.0;
-            for (int i = 0; i < n; i++) acc = std::fma(V[i * m + r], V[i * m + s], acc);
-            out.Wm[r * m + s] = acc;
-        }
-        for (int c = 0; c < p; c++) {
-            double acc = P.F[r * p + c];
-            for (int i = 0; i < n; i++) acc = std::fma(V[i * m + r], U[i * p + c], acc);
-            out.Wh[r * p + c] = acc;
-        }
-        double acc = P.b[r];
-        for (int i = 0; i < n; i++) acc = std::fma(V[i * m + r], u[i], acc);
-        out.wc[r] = acc;
-    }
-    out.QiAT.assign((size_t)n * m, 0.0);
-    out.QiH.assign((size_t)n * p, 0.0);
-    out.Qic.assign(n, 0.0);
-    for (int r = 0; r < m; r++) bwd_sub(L.data(), n, V.data() + r, m, out.QiAT.data() + r, m);
-    for (int c = 0; c < p; c++) bwd_sub(L.data(), n, U.data() + c, p, out.QiH.data() + c, p);
-    bwd_sub(L.data(), n, u.data(), 1, out.Qic.data(), 1);
+        std::vector<double> V = AT, U(P.H, P.H + (size_t)n * p), u(P.c, P.c + n);
+        fwd_sub(L.data(), n, V.data(), m);
+        fwd_sub(L.data(), n, U.data(), p);
+        fwd_sub(L.data(), n, u.data(), 1);
+        out.Wm.assign((size_t)m * m, 0.0);
+        out.Wh.assign(P.F, P.F + (size_t)m * p);
+        out.wc.assign(P.b, P.b + m);
+        add_products(V.data(), m, V.data(), m, n, out.Wm.data());
+        add_products(V.data(), m, U.data(), p, n, out.Wh.data());
+        add_products(V.data(), m, u.data(), 1, n, out.wc.data());
+        bwd_sub(L.data(), n, V.data(), m);
+        bwd_sub(L.data(), n, U.data(), p);
+        bwd_sub(L.data(), n, u.data(), 1);
+        out.QiAT.swap(V);
+        out.QiH.swap(U);
+        out.Qic.swap(u);
     }
     out.At.assign(P.At, P.At + (size_t)ncp * p);
     out.bt.assign(P.bt, P.bt + ncp);
@@ -326,11 +350,14 @@ static int prepare_instance(const mpqp_problem &P, Prepared &out, int prec)
         }
     };
     fill_root(out.root, d.ld1d);
-    fill_root(out.root_f, d.ld1);
     // the FP64 re-solves of the mixed path start from the same pre-pivoted
     // tableau, unless its pivots grew the entries so far that starting from the
     // constraint rows themselves is the safer FP64 arbiter
-    const double growth = prepivot_root_f(d, out.root_f);
+    double growth = 0.0;
+    if (prec == PREC_MIXED) {
+        fill_root(out.root_f, d.ld1);
+        growth = prepivot_root_f(d, out.root_f);
+    }
     if (prec == PREC_MIXED && growth <= kPrepivotGrowth) {
         out.root_p.assign((size_t)(d.root_rows + 1) * d.ld1d, 0.0);
         for (int i = 0; i <= d.root_rows; i++)
@@ -453,6 +480,15 @@ static void fill_defaults(mpqp_options &o)
 #undef DEF
 }
 
+// sub-blocks of a plan's allocations start on 256 bytes
+static size_t pad256(size_t x) { return (x + 255) & ~(size_t)255; }
+// a plan's result block: Ctl, InstCtl[n_inst], OptRec[opt_cap]
+static size_t out_opt_offset(int n_inst) { return pad256(sizeof(Ctl)) + pad256(sizeof(InstCtl) * (size_t)n_inst); }
+// instance data up to this size goes up in one copy, and this many optimal sets
+// come back with the counters
+constexpr size_t kOneUpload = 1 << 19;
+constexpr long long kOptFirst = 512;
+
 // Plan memory comes from one stream-ordered pool per device that keeps what
 // is freed (release threshold: everything).  Freeing the tens of GB of a
 // large plan with cudaFree unmaps them and takes over 100 ms; from the pool,
@@ -542,18 +578,42 @@ static void free_plan_mem(mpqp_plan *P)
     P->ev0 = P->ev1 = P->ev_mid = nullptr;
 }
 
+// Blocks of a persistent grid (SMs x resident blocks).  The answer depends on
+// the kernel, the block and the shared memory alone, so it is asked once per
+// device (a plan asks for a dozen).  A kernel's shared-memory limit only grows:
+// an earlier plan of larger instances may still run.
 static int grid_for(const void *fn, size_t smem, int *grid, int block = 128)
 {
+    struct Limit { int dev; const void *fn; size_t smem; };
+    struct Known { int dev; const void *fn; size_t smem; int block, grid; };
+    static std::mutex mu;
+    static std::vector<Limit> limits;   // one entry per device and kernel
+    static std::vector<Known> known;    // bounded
     int dev = 0, sms = 0, nb = 0;
     CK(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lk(mu);
+    if (smem > 48 * 1024) {
+        Limit *lim = nullptr;
+        for (Limit &l : limits) if (l.dev == dev && l.fn == fn) lim = &l;
+        if (!lim) { limits.push_back(Limit{dev, fn, smem}); lim = &limits.back(); }
+        lim->smem = std::max(lim->smem, smem);
+        const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lim->smem);
+        if (e != cudaSuccess) {
+            lim->smem = 0;
+            set_err(std::string("kernel shared memory limit: ") + cudaGetErrorString(e));
+            return MPQP_ECUDA;
+        }
+    }
+    for (const Known &k : known)
+        if (k.dev == dev && k.fn == fn && k.smem == smem && k.block == block) { *grid = k.grid; return MPQP_OK; }
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    if (smem > 48 * 1024) CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, block, smem));
     if (nb < 1) {
         set_err("kernel does not fit on an SM (shared memory " + std::to_string(smem) + " bytes)");
         return MPQP_EINVAL;
     }
     *grid = nb * sms;
+    if (known.size() < 1024) known.push_back(Known{dev, fn, smem, block, *grid});
     return MPQP_OK;
 }
 
@@ -751,18 +811,36 @@ static int plan_create_locked(int n_inst, const mpqp_problem *probs, const mpqp_
     t.tol_zero_row = o.tol_zero_row;
     // host precompute
     std::vector<Prepared> prep(n_inst);
-    for (int i = 0; i < n_inst; i++) {
-        int rc = prepare_instance(probs[i], prep[i], P->prec);
-        if (rc) { set_err("instance " + std::to_string(i) + ": " + g_err); delete P; return rc; }
+    {
+        // instances are independent: the work (about m^2 n + (m + ncp) nv^2
+        // multiply-adds each) goes to several threads where it outweighs
+        // starting them (tens of microseconds)
+        double work = 0.0;
+        for (int i = 0; i < n_inst; i++)
+            if (probs[i].m > 0 && probs[i].n > 0 && probs[i].m <= kMaxM) work += (double)probs[i].m * probs[i].m * probs[i].n;
+        const unsigned most = work < 4e5 ? 1u : std::min(8u, std::max(1u, std::thread::hardware_concurrency()));
+        const unsigned T = std::min(most, (unsigned)((n_inst + 3) / 4));
+        std::vector<int> rcs(n_inst, MPQP_OK);
+        std::vector<std::string> why(n_inst);
+        run_parallel(T, [&](unsigned t) {
+            for (int i = (int)t; i < n_inst; i += (int)T) {
+                rcs[i] = prepare_instance(probs[i], prep[i], P->prec);
+                if (rcs[i]) why[i] = g_err;   // this thread's text
+            }
+        });
+        for (int i = 0; i < n_inst; i++)
+            if (rcs[i]) { set_err("instance " + std::to_string(i) + ": " + why[i]); delete P; return rcs[i]; }
     }
     // pools
     std::vector<double> dp;
     std::vector<float> fp;
     auto put = [](auto &pool, const std::vector<double> &v) -> long long {
-        long long off = (long long)pool.size();
-        for (double x : v) pool.push_back((typename std::remove_reference<decltype(pool)>::type::value_type)x);
-        while (pool.size() % 4) pool.push_back(0);
-        return off;
+        using E = typename std::remove_reference<decltype(pool)>::type::value_type;
+        const size_t off = pool.size(), n = v.size();
+        pool.resize(off + ((n + 3) & ~(size_t)3));   // new elements are zero
+        E *dst = pool.data() + off;
+        for (size_t i = 0; i < n; i++) dst[i] = (E)v[i];
+        return (long long)off;
     };
     SlotDims &sd = P->sd;
     sd = SlotDims{};
@@ -900,9 +978,20 @@ static int plan_create_locked(int n_inst, const mpqp_problem *probs, const mpqp_
     int rc = MPQP_OK;
     void *p;
 #define AL(ptr, bytes) do { rc = dev_alloc(P, &p, (bytes)); if (rc) { free_plan_mem(P); delete P; return rc; } ptr = (decltype(ptr))p; } while (0)
-    AL(B.inst, sizeof(InstDesc) * n_inst);
-    AL(B.dpool, sizeof(double) * dp.size());
-    AL(B.fpool, sizeof(float) * fp.size());
+    // the instance data in one block (one upload when it is small), and what
+    // plan_results reads back -- Ctl, InstCtl, the first optimal sets -- in another
+    const size_t inst_bytes = pad256(sizeof(InstDesc) * n_inst), dp_bytes = pad256(sizeof(double) * dp.size());
+    const size_t in_bytes = inst_bytes + dp_bytes + sizeof(float) * fp.size();
+    unsigned char *in_block = nullptr;
+    AL(in_block, in_bytes);
+    B.inst = (const InstDesc *)in_block;
+    B.dpool = (const double *)(in_block + inst_bytes);
+    B.fpool = (const float *)(in_block + inst_bytes + dp_bytes);
+    unsigned char *out_block = nullptr;
+    AL(out_block, out_opt_offset(n_inst) + sizeof(OptRec) * opt_cap);
+    B.ctl = (Ctl *)out_block;
+    B.ictl = (InstCtl *)(out_block + pad256(sizeof(Ctl)));
+    B.opt = (OptRec *)(out_block + out_opt_offset(n_inst));
     AL(B.node[0], sizeof(Node) * node_cap);
     AL(B.node[1], sizeof(Node) * node_cap);
     AL(B.tab[0], es * (size_t)tab_cap);
@@ -926,25 +1015,29 @@ static int plan_create_locked(int n_inst, const mpqp_problem *probs, const mpqp_
         AL(B.q_c2b, sizeof(unsigned long long) * B.q_c2_cap);
     }
     AL(B.cert_q, (size_t)B.cert_stride * B.cert_cap);
-    AL(B.opt, sizeof(OptRec) * opt_cap);
     if (rec_cap) AL(B.rec, sizeof(CandRec) * rec_cap);
     if (o.lp2_warm && P->prec == PREC_MIXED) {
         AL(B.lp2b[0], sizeof(unsigned long long) * node_cap);
         AL(B.lp2b[1], sizeof(unsigned long long) * node_cap);
     }
-    AL(B.ictl, sizeof(InstCtl) * n_inst);
-    AL(B.ctl, sizeof(Ctl));
 #undef AL
     CK(cudaStreamSynchronize(0));   // the pool's allocations are stream-ordered on stream 0
-    CK(cudaMemcpy((void *)B.inst, P->desc.data(), sizeof(InstDesc) * n_inst, cudaMemcpyHostToDevice));
-    CK(cudaMemcpy((void *)B.dpool, dp.data(), sizeof(double) * dp.size(), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy((void *)B.fpool, fp.data(), sizeof(float) * fp.size(), cudaMemcpyHostToDevice));
+    if (in_bytes <= kOneUpload) {
+        std::vector<unsigned char> img(in_bytes);
+        memcpy(img.data(), P->desc.data(), sizeof(InstDesc) * n_inst);
+        memcpy(img.data() + inst_bytes, dp.data(), sizeof(double) * dp.size());
+        memcpy(img.data() + inst_bytes + dp_bytes, fp.data(), sizeof(float) * fp.size());
+        CK(cudaMemcpy(in_block, img.data(), in_bytes, cudaMemcpyHostToDevice));
+    } else {
+        CK(cudaMemcpy((void *)B.inst, P->desc.data(), sizeof(InstDesc) * n_inst, cudaMemcpyHostToDevice));
+        CK(cudaMemcpy((void *)B.dpool, dp.data(), sizeof(double) * dp.size(), cudaMemcpyHostToDevice));
+        CK(cudaMemcpy((void *)B.fpool, fp.data(), sizeof(float) * fp.size(), cudaMemcpyHostToDevice));
+    }
     P->h2d_bytes = (long long)(sizeof(InstDesc) * n_inst + sizeof(double) * dp.size() + sizeof(float) * fp.size());
     // the hash is not cleared: a slot counts only when its tag (the run's
     // epoch from the device's counter, and the level) and its fingerprint
     // equal a query's, so an earlier plan's entries in pooled memory and any
     // other leftover bytes read as empty slots
-    CK(cudaMemset(B.ctl, 0, sizeof(Ctl)));
     if (B.lp2b[0]) {
         CK(cudaMemset(B.lp2b[0], 0xff, sizeof(unsigned long long) * node_cap));
         CK(cudaMemset(B.lp2b[1], 0xff, sizeof(unsigned long long) * node_cap));
@@ -1349,28 +1442,6 @@ static void radix_order_range(const OptKeys &K, size_t b, size_t e, uint32_t *ou
     std::copy(order.begin(), order.end(), out);
 }
 
-// f(0) .. f(T-1) on up to T threads (the calling thread included); when a
-// thread cannot be started, the calling thread runs the rest.  An exception
-// of any f(t) is rethrown in the calling thread once all have finished.
-template <typename F>
-static void run_parallel(unsigned T, F f)
-{
-    std::vector<std::exception_ptr> err(T);
-    auto guarded = [&](unsigned t) {
-        try { f(t); } catch (...) { err[t] = std::current_exception(); }
-    };
-    std::vector<std::thread> th;
-    try {
-        for (unsigned t = 1; t < T; t++) th.emplace_back(guarded, t);
-    } catch (...) {
-    }
-    guarded(0u);
-    for (unsigned t = (unsigned)th.size() + 1; t < T; t++) guarded(t);
-    for (std::thread &x : th) x.join();
-    for (const std::exception_ptr &e : err)
-        if (e) std::rethrow_exception(e);
-}
-
 // indices of the optimal-set records in (inst, level, set) order
 static std::vector<uint32_t> sorted_opt_order(const OptRec *ov, size_t n)
 {
@@ -1383,6 +1454,11 @@ static std::vector<uint32_t> sorted_opt_order(const OptRec *ov, size_t n)
         K.or_hi |= K.hi[i]; K.or_lo |= K.lo[i]; K.or_grp |= K.grp[i];
     }
     std::vector<uint32_t> order(n);
+    if (n <= 256) {   // the histograms of a radix sort cost more than these comparisons
+        for (size_t i = 0; i < n; i++) order[i] = (uint32_t)i;
+        std::stable_sort(order.begin(), order.end(), [&K](uint32_t a, uint32_t b) { return opt_key_less(K, a, b); });
+        return order;
+    }
     // large result sets: T contiguous chunks sorted concurrently, then merged
     // pairwise; a merge takes the earlier chunk first on ties, so the result
     // is the same stable order as one sort
@@ -1418,10 +1494,14 @@ static int plan_results_impl(mpqp_plan *P, mpqp_batch_result *&R, bool *complete
     float ms = 0;
     CK(cudaEventElapsedTime(&ms, P->ev0, P->ev1));
     P->last_ms = ms;
+    const size_t off_opt = out_opt_offset(P->n_inst);
+    const long long first = std::min(P->B.opt_cap, kOptFirst);
+    std::vector<unsigned char> head(off_opt + sizeof(OptRec) * first);
+    CK(cudaMemcpy(head.data(), P->B.ctl, head.size(), cudaMemcpyDeviceToHost));
     Ctl ctl;
-    CK(cudaMemcpy(&ctl, P->B.ctl, sizeof(Ctl), cudaMemcpyDeviceToHost));
+    memcpy(&ctl, head.data(), sizeof(Ctl));
     std::vector<InstCtl> ic(P->n_inst);
-    CK(cudaMemcpy(ic.data(), P->B.ictl, sizeof(InstCtl) * P->n_inst, cudaMemcpyDeviceToHost));
+    memcpy(ic.data(), head.data() + pad256(sizeof(Ctl)), sizeof(InstCtl) * P->n_inst);
     R = (mpqp_batch_result *)calloc(1, sizeof(mpqp_batch_result));
     if (!R) throw std::bad_alloc();
     R->n_inst = P->n_inst;
@@ -1455,7 +1535,9 @@ static int plan_results_impl(mpqp_plan *P, mpqp_batch_result *&R, bool *complete
     R->split_levels = (int)ctl.split_levels;
     long long nopt = std::min(ctl.n_opt, P->B.opt_cap);
     std::vector<OptRec> ov(nopt);
-    if (nopt) CK(cudaMemcpy(ov.data(), P->B.opt, sizeof(OptRec) * nopt, cudaMemcpyDeviceToHost));
+    if (nopt) memcpy(ov.data(), head.data() + off_opt, sizeof(OptRec) * std::min(nopt, first));
+    if (nopt > first)
+        CK(cudaMemcpy(ov.data() + first, P->B.opt + first, sizeof(OptRec) * (nopt - first), cudaMemcpyDeviceToHost));
     // order (inst, level, set), sets of one size in the lexicographic order of
     // their sorted element lists: for equal-size sets that is the ascending
     // order of the bit-reversed, complemented masks.  An LSD radix sort on
