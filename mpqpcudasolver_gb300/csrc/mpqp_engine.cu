@@ -28,6 +28,7 @@ namespace mq {
 size_t lp1_smem_per_warp(int prec_bytes, const SlotDims &sd);
 size_t feas_smem_per_warp(int prec_bytes, const SlotDims &sd);
 size_t opt_smem_per_warp(int prec_bytes, const SlotDims &sd);
+size_t opt_fb_smem_per_warp(const SlotDims &sd);
 size_t screen_smem_per_warp(const SlotDims &sd, int route);
 size_t screen_tiles_smem(const SlotDims &sd, int tile_w);
 size_t screen_lanes_smem();
@@ -419,7 +420,7 @@ struct mpqp_plan {
     int tuned = 0;              // 1: the settings came from the autotuner (or its cache)
     size_t smem_opt2 = 0;       // shared memory per block of the primal route
     int grid_enum = 0, grid_feas = 0, grid_lp1fb = 0, grid_opt = 0, grid_optfb = 0, grid_cert = 0;
-    size_t smem_feas = 0, smem_lp1fb = 0, smem_opt = 0, smem_optfb = 0, smem_cert = 0;
+    size_t smem_feas = 0, smem_lp1fb = 0, smem_opt = 0, smem_optfb = 0, smem_direct = 0, smem_cert = 0;
     int n_launches = 0;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -690,7 +691,7 @@ static int enqueue(mpqp_plan *P, cudaStream_t s, EventMode events)
         }
         if (direct(level)) {
             L("k_optimality<double>",
-              launch_optimality(B, P->tol, P->sd, level, false, grid(P->grid_direct, level, 4), P->smem_optfb,
+              launch_optimality(B, P->tol, P->sd, level, false, grid(P->grid_direct, level, 4), P->smem_direct,
                                 s));
             return MPQP_OK;
         }
@@ -1061,7 +1062,8 @@ static int plan_create_locked(int n_inst, const mpqp_problem *probs, const mpqp_
         else if (d.lp && screen_lanes_route(P->lp2_screen, d, sd)) P->lanes_lp = true;
         else P->screen_primal = true;
     }
-    P->smem_optfb = 4 * opt_smem_per_warp(8, sd);
+    P->smem_optfb = 4 * opt_fb_smem_per_warp(sd);
+    P->smem_direct = 4 * opt_smem_per_warp(8, sd);
     if ((rc = grid_for(kernel_ptr("enumerate"), 0, &P->grid_enum)) ||
         (rc = grid_for(kernel_ptr(P->prec == PREC_MIXED ? "feas32" : "feas64"), P->smem_feas, &P->grid_feas,
                        32 * P->feas_warps)) ||
@@ -1087,7 +1089,7 @@ static int plan_create_locked(int n_inst, const mpqp_problem *probs, const mpqp_
         (rc = P->prec == PREC_MIXED ? grid_for(kernel_ptr("screen_dual_lanes"), P->smem_lanes, &P->grid_lanes, 32)
                                     : 0) ||
         (rc = grid_for(kernel_ptr("opt_fp64"), P->smem_optfb, &P->grid_optfb)) ||
-        (rc = P->prec == PREC_MIXED && !P->has_lp ? grid_for(kernel_ptr("opt64"), P->smem_optfb, &P->grid_direct) : 0) ||
+        (rc = P->prec == PREC_MIXED && !P->has_lp ? grid_for(kernel_ptr("opt64"), P->smem_direct, &P->grid_direct) : 0) ||
         (rc = P->has_lp && P->prec != PREC_MIXED ? grid_for(kernel_ptr("opt64_lp"), P->smem_opt, &P->grid_opt_lp) : 0) ||
         (rc = P->has_lp ? grid_for(kernel_ptr("opt_fp64_lp"), P->smem_optfb, &P->grid_optfb_lp) : 0)) {
         free_plan_mem(P);

@@ -338,15 +338,18 @@ __device__ __forceinline__ float trunc_float(unsigned long long bits, bool *ok)
 //    2^-18 of the smallest; a single such row wins without a division, several
 //    are compared by their exact quotients.  The generic loop divides once per
 //    row slot and once more for the degeneracy test;
-//  * comparisons against the tolerances and zero are integer comparisons;
+//  * comparisons against the tolerances and zero are integer comparisons, and
+//    the pivot column, overwritten at the end, is not updated first;
 //  * the row update loads four columns of every row slot before it stores any
 //    (the compiler must otherwise keep each load behind the previous store).
-// An FP64 pivot of a 51 x 6 tableau takes about 27 FP64 warp instructions
+// An FP64 pivot of a 51 x 6 tableau takes about 23 FP64 warp instructions
 // instead of 67.  Measured, FP64 path of the n = 10, m = 43 problem (128K
-// sets): LP1 3,030 -> 2,008 us, the optimality kernel 4,457 -> 2,884 us; the
+// sets): LP1 3,030 -> 1,870 us, the optimality kernel 4,457 -> 2,674 us; the
 // mixed path's k_optimality_fp64 on the m = 62 problem to |S| = 4 1,707 ->
-// 1,130 us and k_lp1_fp64 on the ill-conditioned one 2,718 -> 2,143 us (1,400
-// cycles of an SM per 78 x 25 pivot, 1,200 of them the DFMAs of the update).
+// 1,010 us.  The FP64 pipe is busy 78 to 87 % of these kernels' time (counters).
+// Measured and left out: the last, partial row slot's entries flattened over
+// the lanes (22 % fewer FP64 instructions of LP1, but spills: 1,957 -> 2,318 us)
+// and skipping rows and columns with a zero factor (no gain).
 // tab, bid and nid are byte offsets into the block's dynamic shared memory
 // (the function is not inlined: its five callers share one copy).
 template <int NS>
@@ -356,6 +359,7 @@ __device__ __noinline__ int simplex_fast64(unsigned tab_o, int ld, int nrows, in
 {
     extern __shared__ __align__(16) unsigned char smem[];
     constexpr unsigned long long kInf = 0x7ff0000000000000ULL, kSign = 0x8000000000000000ULL;
+    constexpr unsigned long long kTiny = 0x0580000000000000ULL;   // about 1e-281
     const int lane = lane_id();
     double *tab = reinterpret_cast<double *>(smem + tab_o);
     uint8_t *bid = smem + bid_o, *nid = smem + nid_o;
@@ -397,7 +401,7 @@ __device__ __noinline__ int simplex_fast64(unsigned tab_o, int ld, int nrows, in
         }
         const int q = __ffs(m) - 1;
         const double obq = __shfl_sync(FULLMASK, ob, q);
-        const unsigned long long flip = obq > 0.0 ? 0ull : kSign;   // a = sign(obq) T[i][q]
+        const unsigned long long flip = (unsigned long long)__double_as_longlong(obq) & kSign;   // a = sign(obq) T[i][q]
         // ratio test: smallest max(beta,0)/a over a > tol_piv, smallest id on ties
         double aq[NS];
         float qf[NS];
@@ -464,8 +468,9 @@ __device__ __noinline__ int simplex_fast64(unsigned tab_o, int ld, int nrows, in
         double *Rp = tab + (size_t)r * ld;
         const double br = Rp[ncols], prq = Rp[q];
         // the ratio is zero (a degenerate pivot) when beta is, or underflows
-        bool zero = !(br > 0.0);
-        if (!zero && br < 1e-280) zero = ratio_div(br, fabs(prq)) == 0.0;
+        const unsigned long long brb = (unsigned long long)__double_as_longlong(br);
+        bool zero = !((long long)brb > 0 && brb <= kInf);
+        if (!zero && brb < kTiny) zero = ratio_div(br, fabs(prq)) == 0.0;
         const double inv = __drcp_rn(prq);
         const int owner = r & 31, oslot = r >> 5;
         int lid = bidr[0];
@@ -485,31 +490,33 @@ __device__ __noinline__ int simplex_fast64(unsigned tab_o, int ld, int nrows, in
             upd[s] = bidr[s] >= 0 && !(lane == owner && s == oslot);
             nf[s] = -aq[s];
         }
-        auto columns = [&](int c0, auto width) {
+        // column ci of the ncols columns other than q is ci + (ci >= q)
+        auto columns = [&](int ci, auto width) {
             constexpr int W = decltype(width)::value;
             double Rc[W], t[NS][W];
+            int c[W];
 #pragma unroll
-            for (int j = 0; j < W; j++) Rc[j] = Rp[c0 + j];
+            for (int j = 0; j < W; j++) { c[j] = ci + j + (ci + j >= q ? 1 : 0); Rc[j] = Rp[c[j]]; }
 #pragma unroll
             for (int s = 0; s < NS; s++)
                 if (upd[s]) {
 #pragma unroll
-                    for (int j = 0; j < W; j++) t[s][j] = tab[rowoff[s] + c0 + j];
+                    for (int j = 0; j < W; j++) t[s][j] = tab[rowoff[s] + c[j]];
                 }
 #pragma unroll
             for (int s = 0; s < NS; s++)
                 if (upd[s]) {
 #pragma unroll
-                    for (int j = 0; j < W; j++) tab[rowoff[s] + c0 + j] = xfma(nf[s], Rc[j], t[s][j]);
+                    for (int j = 0; j < W; j++) tab[rowoff[s] + c[j]] = xfma(nf[s], Rc[j], t[s][j]);
                 }
         };
-        int c0 = 0;
+        int ci = 0;
 #pragma unroll 1
-        for (; c0 + 3 <= ncols; c0 += 4) columns(c0, IntC<4>{});
-        const int rem = ncols + 1 - c0;
-        if (rem == 3) columns(c0, IntC<3>{});
-        else if (rem == 2) columns(c0, IntC<2>{});
-        else if (rem == 1) columns(c0, IntC<1>{});
+        for (; ci + 3 < ncols; ci += 4) columns(ci, IntC<4>{});
+        const int rem = ncols - ci;
+        if (rem == 3) columns(ci, IntC<3>{});
+        else if (rem == 2) columns(ci, IntC<2>{});
+        else if (rem == 1) columns(ci, IntC<1>{});
 #pragma unroll
         for (int s = 0; s < NS; s++) if (upd[s]) tab[rowoff[s] + q] = xmul(nf[s], inv);
         if (lane <= ncols) ob = lane == q ? xmul(-obq, inv) : xfma(-obq, rl, ob);
@@ -885,9 +892,21 @@ __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wa
 // optimality slot: R (kmax^2), Y and Lambda (kmax x P1), G (R2 x P1),
 // tableau (rows+1) x ld2, ids (rows + P1, + n + 1 with mpLP instances), S
 // list; FP64 with mpLP instances also Psi (kmax x P1) and Phi (kmax x n).
-// rows = R2 (FP32) or maxR2d (FP64).
+// rows = R2 (FP32) or maxR2d (FP64).  group: k_optimality's slot, with the KKT
+// factors of kGroup sets behind it.
+constexpr int kGroup = 4, kGroupK = 8;   // sets per group, largest |S| of a group
+
+// one set's factor of a group: R, Lambda, S (as in the slot, |S| <= kGroupK)
+__host__ __device__ inline int group_k(const SlotDims &sd) { return sd.maxK < kGroupK ? sd.maxK : kGroupK; }
+__host__ __device__ inline size_t group_bytes(const SlotDims &sd)
+{
+    const int kg = group_k(sd);
+    return align16((size_t)kg * kg * sizeof(double)) + align16((size_t)kg * sd.maxP1 * sizeof(double)) +
+           align16((size_t)kg * sizeof(int));
+}
+
 template <typename T>
-__host__ __device__ inline size_t opt_slot_bytes(const SlotDims &sd)
+__host__ __device__ inline size_t opt_slot_bytes(const SlotDims &sd, bool group = false)
 {
     const bool d = sizeof(T) == 8;
     const int rows = d ? sd.maxR2d : sd.maxR2, ld = d ? sd.maxLD2d : sd.maxLD2;
@@ -896,6 +915,7 @@ __host__ __device__ inline size_t opt_slot_bytes(const SlotDims &sd)
                align16((size_t)rows + sd.maxP1 + (sd.maxN ? sd.maxN + 1 : 0)) + align16((size_t)sd.maxK * sizeof(int));
     if (d && sd.maxN)
         b += align16((size_t)sd.maxK * sd.maxP1 * sizeof(T)) + align16((size_t)sd.maxK * sd.maxN * sizeof(T));
+    if (group) b += kGroup * group_bytes(sd);
     return b;
 }
 
@@ -2104,6 +2124,15 @@ struct OptWs {
     int *S;
     T *Psi, *Phi;   // mpLP (FP64 slots of batches with mpLP instances), else null
     __device__ OptWs() : Psi(nullptr), Phi(nullptr) {}
+    // R, Lambda and S of set g of a group (kkt_factor_group)
+    __device__ void take_group(unsigned char *group, int g, const SlotDims &sd)
+    {
+        const int kg = group_k(sd);
+        unsigned char *b = group + g * group_bytes(sd);
+        R = (T *)b;
+        Lam = (T *)(b + align16((size_t)kg * kg * sizeof(T)));
+        S = (int *)((unsigned char *)Lam + align16((size_t)kg * sd.maxP1 * sizeof(T)));
+    }
     __device__ OptWs(unsigned char *base, const SlotDims &sd)
     {
         const bool d = sizeof(T) == 8;
@@ -2260,6 +2289,77 @@ __device__ int kkt_factor(const KktData<T> &D, const InstDesc &I, uint64_t lo, u
     __syncwarp();
     if (rho_out) *rho_out = __shfl_sync(FULLMASK, rho, 0);
     return 0;
+}
+
+// kkt_factor<double> for up to four sets of k <= kGroupK elements at once, set g
+// in lanes 8 g .. 8 g + 7 (inst, lo, hi, act alike in a set's lanes; act false:
+// no set).  The same operations in the same order per entry, but a warp
+// instruction serves four sets, and the forward substitution runs as further
+// columns of the factor's rows.  The FP64 pipe takes 16 cycles per warp
+// instruction of an SM however few lanes are active, and with one set per warp
+// half of the optimality kernel's FP64 instructions were this factor's (a
+// square root and three divisions per row, in at most p + 1 lanes): about 190 of
+// 381 at k = 4, p = 4, now 37.  k_optimality<double> of the n = 10, m = 43
+// problem (128K sets) 2,674 -> 1,965 us, of 24 small problems (305K sets) 6,932
+// -> 4,220 us.  Leaves R, Lambda and S where w (alike in a set's
+// lanes) points; returns a ballot of the lanes whose set failed the LICQ test.
+__device__ unsigned kkt_factor_group(const DevBuffers &B, double thr, int k, int inst, uint64_t lo, uint64_t hi, bool act,
+                                     const OptWs<double> &w)
+{
+    const int tl = lane_id() & 7;
+    double *R = w.R, *Lam = w.Lam;
+    int *S = w.S;
+    const InstDesc &I = B.inst[act ? inst : 0];
+    const KktData<double> D = kkt_data<double>(B, I);
+    const int m = I.m, p = I.p, P1 = p + 1;
+    if (act && tl < k) {
+        for (int t = 0; t < tl; t++) { if (lo) lo &= lo - 1; else hi &= hi - 1; }
+        S[tl] = lo ? __ffsll((long long)lo) - 1 : 63 + __ffsll((long long)hi);
+    }
+    __syncwarp();
+    bool fail = false;
+    for (int a = 0; a < k; a++) {
+        const int sa = act ? S[a] : 0;
+        const double d0 = act ? D.Wm[(size_t)sa * m + sa] : 1.0;
+        double acc = d0;
+        for (int l = 0; l < a; l++) { const double r = act ? R[l * k + a] : 0.0; acc = xfma(-r, r, acc); }
+        const bool bad = !(acc > thr * d0);
+        fail |= bad;
+        const double raa = xsqrt(bad ? 1.0 : acc);
+        if (act && tl == 0) R[a * k + a] = raa;
+        // the columns right of the diagonal, then those of [Wh | wc]
+        const int nr = k - 1 - a, nc = act ? nr + P1 : 0;
+        const int most = __reduce_max_sync(FULLMASK, nc);
+        for (int c0 = 0; c0 < most; c0 += 8) {
+            const int c = c0 + tl;
+            if (c < nc) {
+                double *X;
+                int ldx;
+                double x;
+                if (c < nr) {
+                    X = R + a + 1 + c; ldx = k;
+                    x = D.Wm[(size_t)sa * m + S[a + 1 + c]];
+                } else {
+                    const int cc = c - nr;
+                    X = Lam + cc; ldx = P1;
+                    x = cc < p ? D.Wh[(size_t)sa * p + cc] : D.wc[sa];
+                }
+                for (int l = 0; l < a; l++) x = xfma(-R[l * k + a], X[l * ldx], x);
+                X[a * ldx] = xdiv(x, raa);
+            }
+        }
+        __syncwarp();
+    }
+    // back substitution, a column per lane
+    for (int cc = tl; act && cc < P1; cc += 8) {
+        for (int a = k - 1; a >= 0; a--) {
+            double x = Lam[a * P1 + cc];
+            for (int l = a + 1; l < k; l++) x = xfma(-R[a * k + l], Lam[l * P1 + cc], x);
+            Lam[a * P1 + cc] = xdiv(x, R[a * k + a]);
+        }
+    }
+    __syncwarp();
+    return __ballot_sync(FULLMASK, act && fail);
 }
 
 // Region rows in the reference order (utils.py:39-57): lambda rows (S
@@ -2742,10 +2842,11 @@ __device__ __noinline__ int lp2_cert64(const KktData<double> &D, const InstDesc 
 // Optimality and region verdict of one feasible set (the FP64 path; the FP32
 // screen of the mixed path is k_opt_screen).  LP: the instance is an mpLP.
 // basis (mixed precision, mpQP over a box): the FP32 dual screen's final
-// basis, checked by lp2_cert64 before the LP2 (~0: none).
+// basis, checked by lp2_cert64 before the LP2 (~0: none).  ws holds the set's
+// KKT factor (k elements; licq_fail: it failed the LICQ test).
 template <typename T, bool LP = false>
 __device__ OptResult eval_optimality(const DevBuffers &B, const Tol &tol, const InstDesc &I, uint64_t lo, uint64_t hi,
-                                     OptWs<T> &ws, unsigned long long basis = ~0ull)
+                                     OptWs<T> &ws, int k, bool licq_fail, unsigned long long basis = ~0ull)
 {
     const int lane = lane_id();
     const int m = I.m, p = I.p, ncp = I.ncp, P1 = p + 1, R2 = m + ncp;
@@ -2758,8 +2859,7 @@ __device__ OptResult eval_optimality(const DevBuffers &B, const Tol &tol, const 
     res.decided = true;
     const T tpiv = (T)tol.tol_piv;
     const T tdj = (T)tol.tol_dj;
-    int k = 0;
-    if (kkt_factor<T>(D, I, lo, hi, (T)tol.tol_licq, ws, &k)) {
+    if (licq_fail) {
         res.licq = 0; res.lp2_status = LP_LICQ_FAIL;
         return res;
     }
@@ -2869,7 +2969,7 @@ __global__ void __launch_bounds__(128, kF64Blocks) k_optimality(DevBuffers B, To
 {
     extern __shared__ __align__(16) unsigned char smem[];
     const int lane = lane_id(), wib = threadIdx.x >> 5;
-    const size_t slot = opt_slot_bytes<T>(sd);
+    const size_t slot = opt_slot_bytes<T>(sd, true);
     OptWs<T> ws(smem + wib * slot, sd);
     const int side = level & 1;
     Ctl *ctl = B.ctl;
@@ -2886,26 +2986,54 @@ __global__ void __launch_bounds__(128, kF64Blocks) k_optimality(DevBuffers B, To
         atomicAdd((unsigned long long *)&ic->cheb_piv, (unsigned long long)lc.d);
         if (B.precision == PREC_MIXED) atomicAdd((unsigned long long *)&ic->fb_opt, (unsigned long long)lc.e);
     };
+    // sets of a level have k = level elements; their KKT factors are computed
+    // a group at a time (single sets where the level cannot fill the warps)
+    const bool grouped = level <= kGroupK;
+    const int claim = grouped ? claim_size(nn, kGroup) : 1;
+    unsigned char *group = smem + wib * slot + opt_slot_bytes<T>(sd);
+    auto takes = [&](const Node &nd) {
+        return (nd.flags & (NODE_VALID | NODE_FEASIBLE)) == (NODE_VALID | NODE_FEASIBLE) && level >= B.inst[nd.inst].k_min &&
+               (B.inst[nd.inst].lp != 0) == LP;
+    };
     for (;;) {
-        long long x;
-        if (lane == 0) x = (long long)atomicAdd(&ctl->ctr[LP ? 6 : 3], 1ull);
-        x = __shfl_sync(FULLMASK, x, 0);
-        if (x >= nn) break;
-        const Node nd = B.node[side][x];
-        // (mixed precision: no first-stage basis for the children to start from)
-        if (B.lp2b[side] && lane == 0) B.lp2b[side][x] = ~0ull;
-        if ((nd.flags & (NODE_VALID | NODE_FEASIBLE)) != (NODE_VALID | NODE_FEASIBLE)) continue;
-        const InstDesc &I = B.inst[nd.inst];
-        if (level < I.k_min || (I.lp != 0) != LP) continue;
-        if (nd.inst != lc.inst) { flush(); lc.reset(nd.inst); }
-        const OptResult res = eval_optimality<T, LP>(B, tol, I, nd.lo, nd.hi, ws);
-        lc.c += res.lp2_piv;
-        lc.d += res.cheb_piv;
-        lc.a += res.optimal;
-        lc.b += res.region;
-        lc.e++;
-        if (lane == 0) write_opt(B, nd, level, res, true);
-        __syncwarp();
+        long long x0;
+        if (lane == 0) x0 = (long long)atomicAdd(&ctl->ctr[LP ? 6 : 3], (unsigned long long)claim);
+        x0 = __shfl_sync(FULLMASK, x0, 0);
+        if (x0 >= nn) break;
+        const int cnt = nn - x0 < claim ? (int)(nn - x0) : claim;
+        unsigned failed = 0;
+        if (grouped) {
+            const int g = lane >> 3;
+            const Node nd = B.node[side][x0 + (g < cnt ? g : 0)];
+            const bool act = g < cnt && takes(nd);
+            ws.take_group(group, g, sd);
+            failed = kkt_factor_group(B, tol.tol_licq, level, nd.inst, nd.lo, nd.hi, act, ws);
+        }
+        for (int g = 0; g < cnt; g++) {
+            const long long x = x0 + g;
+            const Node nd = B.node[side][x];
+            // (mixed precision: no first-stage basis for the children to start from)
+            if (B.lp2b[side] && lane == 0) B.lp2b[side][x] = ~0ull;
+            if (!takes(nd)) continue;
+            const InstDesc &I = B.inst[nd.inst];
+            if (nd.inst != lc.inst) { flush(); lc.reset(nd.inst); }
+            int k = level;
+            bool licq_fail;
+            if (grouped) {
+                ws.take_group(group, g, sd);
+                licq_fail = (failed >> (8 * g)) & 1u;
+            } else {
+                licq_fail = kkt_factor<T>(kkt_data<T>(B, I), I, nd.lo, nd.hi, (T)tol.tol_licq, ws, &k) != 0;
+            }
+            const OptResult res = eval_optimality<T, LP>(B, tol, I, nd.lo, nd.hi, ws, k, licq_fail);
+            lc.c += res.lp2_piv;
+            lc.d += res.cheb_piv;
+            lc.a += res.optimal;
+            lc.b += res.region;
+            lc.e++;
+            if (lane == 0) write_opt(B, nd, level, res, true);
+            __syncwarp();
+        }
     }
     flush();
 }
@@ -2919,7 +3047,10 @@ __global__ void __launch_bounds__(128, kF64Blocks) k_optimality_fp64(DevBuffers 
     OptWs<double> ws(smem + wib * slot, sd);
     const int side = level & 1;
     Ctl *ctl = B.ctl;
-    // the FP64 queue, then the sets queued with an FP32 dual basis to check first
+    // the FP64 queue, then the sets queued with an FP32 dual basis to check
+    // first.  One set at a time: these are few and their LPs long and uneven
+    // (most optimal sets end here); in groups of four the kernel took 2,104
+    // instead of 1,774 us on the ill-conditioned problem
     const long long nq = ctl->n_q_opt < B.q_cap ? ctl->n_q_opt : B.q_cap;
     const long long nc = ctl->n_q_c2 < B.q_c2_cap ? ctl->n_q_c2 : B.q_c2_cap;
     for (;;) {
@@ -2934,7 +3065,9 @@ __global__ void __launch_bounds__(128, kF64Blocks) k_optimality_fp64(DevBuffers 
         const Node nd = B.node[side][xn];
         const InstDesc &I = B.inst[nd.inst];
         if ((I.lp != 0) != LP) continue;
-        const OptResult res = eval_optimality<double, LP>(B, tol, I, nd.lo, nd.hi, ws, basis);
+        int k = 0;
+        const bool licq_fail = kkt_factor<double>(kkt_data<double>(B, I), I, nd.lo, nd.hi, tol.tol_licq, ws, &k) != 0;
+        const OptResult res = eval_optimality<double, LP>(B, tol, I, nd.lo, nd.hi, ws, k, licq_fail, basis);
         if (lane == 0) {
             InstCtl *ic = &B.ictl[nd.inst];
             atomicAdd((unsigned long long *)&ic->fb_opt, 1ull);
@@ -4755,9 +4888,12 @@ size_t screen_tiles_smem(const SlotDims &sd, int tile_w) { return (32 / tile_w) 
 bool screen_dual_route(int mode, const InstDesc &I, const SlotDims &sd) { return dual_route(mode, I, sd); }
 bool screen_lanes_route(int mode, const InstDesc &I, const SlotDims &sd) { return lanes_route(mode, I, sd); }
 
+// k_optimality_fp64 (k_optimality's slot has the group's factors besides)
+size_t opt_fb_smem_per_warp(const SlotDims &sd) { return opt_slot_bytes<double>(sd); }
+
 size_t opt_smem_per_warp(int prec_bytes, const SlotDims &sd)
 {
-    return prec_bytes == 8 ? opt_slot_bytes<double>(sd) : opt_slot_bytes<float>(sd);
+    return prec_bytes == 8 ? opt_slot_bytes<double>(sd, true) : opt_slot_bytes<float>(sd);
 }
 
 }  // namespace mq
