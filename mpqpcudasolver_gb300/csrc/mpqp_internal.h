@@ -89,7 +89,7 @@ struct Node {                   // a feasible (or, when exhaustive, any) active 
     int inst;
     int flags;                  // NodeFlags
     long long tab_off;          // element offset into the tableau arena (-1: none)
-    long long ids_off;          // byte offset into the ids arena
+    long long ids_off;          // byte offset into the ids arena (follows tab_off: see store_node)
     long long rec;              // record index (or -1)
 };
 

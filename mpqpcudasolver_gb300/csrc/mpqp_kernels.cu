@@ -813,11 +813,13 @@ __host__ __device__ inline size_t lp1_slot_bytes(int maxM1, int maxLD1, int maxN
     return lp1_buf_bytes<T>(maxM1, maxLD1, maxNv) + 16;
 }
 
-// slot of k_feasibility: one buffer and the warp's mbarrier (16 bytes, last)
+// slot of k_feasibility: one buffer, the arena offsets reserved for the chunk's
+// candidates and the warp's mbarrier (16 bytes, last)
+constexpr int kChunkOffsets = 2 * 32;
 template <typename T>
 __host__ __device__ inline size_t feas_slot_bytes(int maxM1, int maxLD1, int maxNv)
 {
-    return lp1_buf_bytes<T>(maxM1, maxLD1, maxNv) + 16;
+    return lp1_buf_bytes<T>(maxM1, maxLD1, maxNv) + kChunkOffsets * sizeof(long long) + 16;
 }
 
 // candidates a warp claims at a time (a plan setting, at most 32, by default
@@ -1160,15 +1162,21 @@ __device__ __forceinline__ void warp_copy_v(T *dst, const T *src, int n)
 // bulk: tab and ids are a shared-memory slot of the plan's layout (src_ld 0,
 // TT = TS); lane 0 copies them with bulk stores (bulk_wait_read before the
 // slot is written again, bulk_wait_all before the kernel ends).
+// reserved: the arena space reserved before (reserved[0] the tableau's and
+// reserved[stride] the ids' offset, -1: none).  stride 32: a chunk of
+// k_feasibility, which counts its stores and inserts its sets into the hash
+// itself; stride 1: a candidate's node record.
 template <typename TT, typename TS>
 __device__ long long store_node(const DevBuffers &B, int side, int level, const InstDesc &I, int inst,
                                 uint64_t lo, uint64_t hi, bool feasible, const TS *tab, const uint8_t *ids,
                                 long long rec, long long hcap, int extra_flags, int src_ld = 0, bool bulk = false,
-                                long long pre_idx = -1, int rows_store = -1, int cols_store = -1)
+                                long long pre_idx = -1, int rows_store = -1, int cols_store = -1,
+                                const long long *reserved = nullptr, int stride = 0)
 {
     const int lane = lane_id();
     Ctl *ctl = B.ctl;
     const bool need_tab = level < I.k_max;
+    const bool chunked = stride == 32;   // the caller counts the store and inserts the set into the hash
     long long idx = 0, toff = -1, ioff = -1;
     if (lane == 0) {
         // one arena per kind, side 0 filled upward from 0, side 1 downward
@@ -1177,7 +1185,10 @@ __device__ long long store_node(const DevBuffers &B, int side, int level, const 
         // candidate's index)
         idx = pre_idx >= 0 ? pre_idx : (long long)atomicAdd((unsigned long long *)&ctl->n_node[side], 1ull);
         if (idx >= B.node_cap) { atomicOr(&ctl->overflow, OV_NODE); idx = -1; }
-        if (need_tab && idx >= 0 && !*((volatile int *)&ctl->tab_full[side])) {
+        if (reserved) {
+            toff = reserved[0];
+            ioff = reserved[stride];
+        } else if (need_tab && idx >= 0 && !*((volatile int *)&ctl->tab_full[side])) {
             const long long told = (long long)atomicAdd((unsigned long long *)&ctl->tab_used[side], (unsigned long long)I.tab_elems);
             const long long iold = (long long)atomicAdd((unsigned long long *)&ctl->ids_used[side], (unsigned long long)I.ids_bytes);
             if (told + I.tab_elems + ctl->tab_used[side ^ 1] > B.tab_cap ||
@@ -1206,7 +1217,7 @@ __device__ long long store_node(const DevBuffers &B, int side, int level, const 
             nd.flags = NODE_VALID | (feasible ? NODE_FEASIBLE : 0) | (extra_flags & ~NODE_CERT);
             nd.tab_off = -1; nd.ids_off = -1; nd.rec = rec;
             B.node[side][idx] = nd;
-            if (feasible && !B.exhaustive) {
+            if (feasible && !B.exhaustive && !chunked) {
                 if (!hash_insert(B.hash[side], hcap, hash_tag(ctl->epoch, level), inst, lo, hi))
                     atomicOr(&ctl->overflow, OV_HASH);
             }
@@ -1214,7 +1225,7 @@ __device__ long long store_node(const DevBuffers &B, int side, int level, const 
         return idx;
     }
     if (need_tab) {
-        if (lane == 0) atomicAdd((unsigned long long *)&B.ictl[inst].stored, 1ull);
+        if (lane == 0 && !chunked) atomicAdd((unsigned long long *)&B.ictl[inst].stored, 1ull);
         TT *dst = (TT *)B.tab[side] + toff;
         if (bulk) {
             fence_proxy_async_smem();
@@ -1251,7 +1262,7 @@ __device__ long long store_node(const DevBuffers &B, int side, int level, const 
         nd.tab_off = toff; nd.ids_off = ioff; nd.rec = rec;
         B.node[side][idx] = nd;
         // the hash serves the subset test of the next level only
-        if (feasible && !B.exhaustive && need_tab) {
+        if (feasible && !B.exhaustive && need_tab && !chunked) {
             if (!hash_insert(B.hash[side], hcap, hash_tag(ctl->epoch, level), inst, lo, hi))
                 atomicOr(&ctl->overflow, OV_HASH);
         }
@@ -1409,6 +1420,7 @@ __device__ __forceinline__ void feasibility_body(const DevBuffers &B, const Tol 
     T *tab = (T *)base;
     uint8_t *ids = base + align16((((size_t)(sd.maxM1 + 1) * mld + 3) & ~(size_t)3) * sizeof(T));
     uint64_t *bar = (uint64_t *)(base + slot - 16);
+    long long *room = (long long *)(base + slot - 16) - kChunkOffsets;
     const int side = level & 1, pside = side ^ 1;
     Ctl *ctl = B.ctl;
     const long long ncand = ctl->n_cand;
@@ -1432,16 +1444,60 @@ __device__ __forceinline__ void feasibility_body(const DevBuffers &B, const Tol 
         const Cand mine = lane < cnt ? B.cand[w0 + lane] : Cand{-1, 0};
         // candidate w's node goes to slot w (also when the FP64 re-solve
         // stores it); a candidate that stores none leaves an invalid record
+        // with its reserved arena space (below)
         const long long nbase = w0;
         if (lane == 0) atomicMax((unsigned long long *)&ctl->n_node[side], (unsigned long long)(w0 + cnt));
-        if (lane < cnt && nbase + lane < B.node_cap) {
-            Node gap;
-            gap.lo = 0; gap.hi = 0; gap.inst = 0; gap.flags = 0; gap.tab_off = -1; gap.ids_off = -1; gap.rec = -1;
-            B.node[side][nbase + lane] = gap;
-        }
         // lane t holds candidate t's parent tableau offset (for the prefetch)
         const long long my_toff = lane < cnt ? B.node[pside][mine.parent].tab_off : -1;
         const int my_inst = lane < cnt ? B.node[pside][mine.parent].inst : 0;
+        // Arena space for the tableaus of the whole chunk (also of the few
+        // candidates that will store none; one that goes to the FP64 re-solve
+        // finds its space in its node record): one pair of atomics instead of a
+        // pair per stored candidate, whose round trip the warp waited for.  With
+        // the hash inserts below: LP1 of 32 mpLPs (1.7M sets, 1.7 pivots each)
+        // 5,248 -> 3,297 us, of the m = 62 batch 177 -> 167 ms
+        bool keeps = false;   // this lane's candidate stores a tableau when feasible
+        {
+            const InstDesc &Il = B.inst[my_inst];
+            const InstCtl &il = B.ictl[my_inst];
+            keeps = lane < cnt && level < Il.k_max && !il.stopped &&
+                    !(Il.budget > 0 && il.cum_cand + il.lvl_cand > Il.budget);
+            const int te = keeps ? Il.tab_elems : 0, ib = keeps ? Il.ids_bytes : 0;
+            int ts = te, is = ib;   // inclusive sums
+#pragma unroll
+            for (int off = 1; off < 32; off <<= 1) {
+                const int tv = __shfl_up_sync(FULLMASK, ts, off), iv = __shfl_up_sync(FULLMASK, is, off);
+                if (lane >= off) { ts += tv; is += iv; }
+            }
+            long long tb = -1, ibase = 0;
+            if (lane == 31 && ts > 0 && !*((volatile int *)&ctl->tab_full[side])) {
+                tb = (long long)atomicAdd((unsigned long long *)&ctl->tab_used[side], (unsigned long long)ts);
+                ibase = (long long)atomicAdd((unsigned long long *)&ctl->ids_used[side], (unsigned long long)is);
+            }
+            tb = __shfl_sync(FULLMASK, tb, 31);
+            ibase = __shfl_sync(FULLMASK, ibase, 31);
+            long long toff = -1, ioff = -1;
+            if (keeps && tb >= 0) {
+                const long long told = tb + ts - te, iold = ibase + is - ib;
+                if (told + te + ctl->tab_used[side ^ 1] > B.tab_cap || iold + ib + ctl->ids_used[side ^ 1] > B.ids_cap) {
+                    // the arena is full: this node and the later ones of the level
+                    // keep no tableau (see store_node)
+                    atomicExch(&ctl->tab_full[side], 1);
+                } else {
+                    toff = side == 0 ? told : B.tab_cap - told - te;
+                    ioff = side == 0 ? iold : B.ids_cap - iold - ib;
+                }
+            }
+            room[lane] = toff;
+            room[32 + lane] = ioff;
+            if (lane < cnt && nbase + lane < B.node_cap) {
+                Node gap;
+                gap.lo = 0; gap.hi = 0; gap.inst = 0; gap.flags = 0; gap.tab_off = toff; gap.ids_off = ioff; gap.rec = -1;
+                B.node[side][nbase + lane] = gap;
+            }
+            __syncwarp();
+        }
+        unsigned stored = 0;   // bit t: candidate t was stored and goes into the hash
         // Candidates of their instance's last level (nothing is stored there)
         // decided without an LP: every nonbasic slack is zero at a certified
         // vertex of the parent's face, so a child whose new slack is nonbasic
@@ -1492,6 +1548,7 @@ __device__ __forceinline__ void feasibility_body(const DevBuffers &B, const Tol 
                 atomicAdd((unsigned long long *)&B.ictl[lc.inst].feasible, (unsigned long long)lc.a);
                 atomicAdd((unsigned long long *)&B.ictl[lc.inst].lp1_piv, (unsigned long long)lc.b);
                 atomicAdd(&B.ictl[lc.inst].feas_digest, (unsigned long long)lc.c);
+                atomicAdd((unsigned long long *)&B.ictl[lc.inst].stored, (unsigned long long)lc.d);
             }
             lc.reset(inst);
         }
@@ -1687,7 +1744,11 @@ __device__ __forceinline__ void feasibility_body(const DevBuffers &B, const Tol 
             }
             store_node<T, T>(B, side, level, I, inst, lo, hi, feasible, tab, ids, rec, hcap,
                              mixed && feasible ? NODE_CERT : 0, 0, true, nbase + t, mixed ? rows : -1,
-                             mixed ? cols : -1);
+                             mixed ? cols : -1, room + t, 32);
+            if (level < I.k_max) {
+                lc.d += room[t] >= 0;
+                if (feasible && !B.exhaustive) stored |= 1u << t;
+            }
         }
         if (at_vertex && feasible && level == I.k_max) {
             // later siblings whose new slack is nonbasic at this vertex
@@ -1708,12 +1769,23 @@ __device__ __forceinline__ void feasibility_body(const DevBuffers &B, const Tol 
             done |= __ballot_sync(FULLMASK, lane > t && lane < cnt && mine.parent == c.parent && ((wsel >> (mj & 31)) & 1u));
         }
     }
+        // the chunk's feasible sets into the hash, a lane each: their random
+        // accesses overlap (one at a time, each held the warp up for a round
+        // trip and an atomic's)
+        __syncwarp();
+        if (((stored >> lane) & 1u) && nbase + lane < B.node_cap) {
+            const Node nd = B.node[side][nbase + lane];
+            if (!hash_insert(B.hash[side], hcap, hash_tag(ctl->epoch, level), nd.inst, nd.lo, nd.hi))
+                atomicOr(&ctl->overflow, OV_HASH);
+        }
+        __syncwarp();
     }
     if (lane == 0) bulk_wait_all();
     if (lc.inst >= 0 && lane == 0) {
         atomicAdd((unsigned long long *)&B.ictl[lc.inst].feasible, (unsigned long long)lc.a);
         atomicAdd((unsigned long long *)&B.ictl[lc.inst].lp1_piv, (unsigned long long)lc.b);
         atomicAdd(&B.ictl[lc.inst].feas_digest, (unsigned long long)lc.c);
+        atomicAdd((unsigned long long *)&B.ictl[lc.inst].stored, (unsigned long long)lc.d);
     }
 }
 
@@ -1796,7 +1868,7 @@ __global__ void __launch_bounds__(128, kF64Blocks) k_lp1_fp64(DevBuffers B, Tol 
         }
         if (feasible || B.exhaustive)
             store_node<float, double>(B, side, level, I, inst, lo, hi, feasible, tab, ids, rec, hcap, 0, I.ld1d, false,
-                                      w, rows);
+                                      w, rows, -1, w < B.node_cap ? &B.node[side][w].tab_off : nullptr, 1);
     }
 }
 
