@@ -540,6 +540,31 @@ static size_t free_device_bytes()
     return fb + pool_idle_bytes(dev);
 }
 
+namespace mq {
+// Memory of a single call from the same pool (cudaMalloc without one); null on
+// failure.  pool_free returns it once the work queued on stream 0 is done.
+void *pool_malloc(size_t bytes)
+{
+    int dev = 0;
+    void *p = nullptr;
+    cudaGetDevice(&dev);
+    cudaMemPool_t pool = plan_pool(dev);
+    if ((pool ? cudaMallocFromPoolAsync(&p, bytes, pool, 0) : cudaMalloc(&p, bytes)) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    return p;
+}
+
+void pool_free(void *p)
+{
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (plan_pool(dev)) cudaFreeAsync(p, 0);
+    else cudaFree(p);
+}
+}  // namespace mq
+
 static int dev_alloc(mpqp_plan *P, void **ptr, size_t bytes)
 {
     if (bytes == 0) bytes = 16;
@@ -1664,25 +1689,34 @@ static int mpqp_region_laws_impl(const mpqp_problem *prob, long long n_sets, con
     SlotDims sd = P->sd;
     sd.maxK = std::max(1, kcap);
     const long long stride = mpqp_region_laws_stride(prob);
-    uint64_t *dm = nullptr; double *dl = nullptr, *dr = nullptr, *de = nullptr; int *ds = nullptr;
     size_t smem = 4 * laws_smem_per_warp(sd);
     int grid = 0;
     rc = grid_for(kernel_ptr("laws"), smem, &grid);
+    // masks, laws and the small per-set results (radius, err, sizes) in one
+    // block from the plan's pool (five cudaMalloc and cudaFree pairs took 400 us
+    // of a call), the small results back in one copy
+    const size_t laws_off = pad256(sizeof(uint64_t) * 2 * (size_t)n_sets);
+    const size_t small_off = laws_off + pad256(sizeof(double) * (size_t)stride * (size_t)n_sets);
+    const size_t per_set = 2 * sizeof(double) + 4 * sizeof(int);
+    unsigned char *blk = nullptr;
+    if (!rc) rc = dev_alloc(P, (void **)&blk, small_off + per_set * (size_t)n_sets);
     if (!rc) {
-        CK(cudaMalloc(&dm, sizeof(uint64_t) * 2 * n_sets));
-        CK(cudaMalloc(&dl, sizeof(double) * stride * n_sets));
-        CK(cudaMalloc(&ds, sizeof(int) * 4 * n_sets));
-        if (radius) CK(cudaMalloc(&dr, sizeof(double) * n_sets));
-        if (err) CK(cudaMalloc(&de, sizeof(double) * n_sets));
-        CK(cudaMemcpy(dm, masks, sizeof(uint64_t) * 2 * n_sets, cudaMemcpyHostToDevice));
-        CK(launch_region_laws_r(P->B, P->tol, sd, dm, n_sets, dl, ds, stride, dr, de, grid, smem, nullptr));
-        CK(cudaMemcpy(laws, dl, sizeof(double) * stride * n_sets, cudaMemcpyDeviceToHost));
-        CK(cudaMemcpy(sizes, ds, sizeof(int) * 4 * n_sets, cudaMemcpyDeviceToHost));
-        if (radius) CK(cudaMemcpy(radius, dr, sizeof(double) * n_sets, cudaMemcpyDeviceToHost));
-        if (err) CK(cudaMemcpy(err, de, sizeof(double) * n_sets, cudaMemcpyDeviceToHost));
-        cudaFree(dm); cudaFree(dl); cudaFree(ds);
-        if (dr) cudaFree(dr);
-        if (de) cudaFree(de);
+        double *dl = (double *)(blk + laws_off), *dr = (double *)(blk + small_off), *de = dr + n_sets;
+        int *ds = (int *)(de + n_sets);
+        auto run = [&]() -> int {
+            CK(cudaMemcpy(blk, masks, sizeof(uint64_t) * 2 * n_sets, cudaMemcpyHostToDevice));
+            CK(launch_region_laws_r(P->B, P->tol, sd, (const uint64_t *)blk, n_sets, dl, ds, stride, radius ? dr : nullptr,
+                                    err ? de : nullptr, grid, smem, nullptr));
+            CK(cudaMemcpy(laws, dl, sizeof(double) * stride * n_sets, cudaMemcpyDeviceToHost));
+            std::vector<unsigned char> small(per_set * (size_t)n_sets);
+            CK(cudaMemcpy(small.data(), blk + small_off, small.size(), cudaMemcpyDeviceToHost));
+            const unsigned char *sm = small.data();
+            if (radius) memcpy(radius, sm, sizeof(double) * n_sets);
+            if (err) memcpy(err, sm + sizeof(double) * n_sets, sizeof(double) * n_sets);
+            memcpy(sizes, sm + 2 * sizeof(double) * n_sets, sizeof(int) * 4 * n_sets);
+            return MPQP_OK;
+        };
+        rc = run();
     }
     mpqp_plan_destroy(P);
     return rc;

@@ -4667,6 +4667,11 @@ __global__ void __launch_bounds__(32, 32) k_opt_screen(DevBuffers B, Tol tol, Sl
 // maximum is at most d_i + tol.  One warp per row, the FP64 warp simplex from
 // the slack basis (u = 0 is feasible: d >= 0).  out[c] = 1 redundant, 0 not
 // (an iteration limit keeps the row).
+__host__ __device__ inline size_t redundancy_slot_bytes(int nrows, int ld)
+{
+    return align16((size_t)(nrows + 1) * ld * sizeof(double)) + align16((size_t)nrows + 64);
+}
+
 __global__ void __launch_bounds__(32, 4 * kF64Blocks) k_redundancy(const double *M, const double *d, int nrows, int nv, int ld,
                                                    const int *check, int n_check, double tol, Tol lt, int max_piv,
                                                    int *out)
@@ -4698,6 +4703,192 @@ __global__ void __launch_bounds__(32, 4 * kF64Blocks) k_redundancy(const double 
         const double maxval = -T[(size_t)nrows * ld + nv];
         if (lane == 0) out[c] = (st == LP_OPTIMAL && maxval <= d[i] + tol) ? 1 : 0;
         __syncwarp();
+    }
+}
+
+// Scratch of simplex_block64 in shared memory.
+struct BlockLp {
+    double row[4][32];                  // each warp's copy of the scaled pivot row
+    unsigned long long key[4];
+    unsigned q[4], id[4];
+    int n[4], r[4], rx[4];
+};
+
+// simplex_fast64's pivots (the same rules, operations and values) by a block of
+// four warps on one FP64 tableau of at most 128 rows and 31 columns: thread i
+// holds row i, every warp prices the objective row for itself and keeps its own
+// copy of the scaled pivot row.  For callers with fewer LPs than SMs: one warp
+// gets a quarter of its SM's FP64 pipe (64 cycles per warp instruction), and
+// the update of an 80 x 17 tableau alone took 51 of those per pivot; now 17 on
+// each quarter.  Returns the status; *z_out the objective's right-hand side.
+// Three barriers per pivot (four when the ratio test has to divide).
+__device__ int simplex_block64(double *tab, int ld, int nrows, int ncols, int nfree, uint8_t *bid, const uint8_t *nid,
+                               BlockLp *s, double tol_piv, double tol_dj, int max_piv, int degen_switch, double *z_out)
+{
+    constexpr unsigned long long kInf = 0x7ff0000000000000ULL, kSign = 0x8000000000000000ULL;
+    constexpr unsigned long long kTiny = 0x0580000000000000ULL;   // about 1e-281
+    const int lane = lane_id(), w = threadIdx.x >> 5, i = threadIdx.x;
+    const bool valid = i < nrows;
+    double *Ti = tab + (size_t)(valid ? i : 0) * ld;
+    int bidr = valid ? (int)bid[i] : -1;
+    double ob = lane <= ncols ? tab[(size_t)nrows * ld + lane] : 0.0;
+    int nidl = lane < ncols ? (int)nid[lane] : 255;
+    const long long tpiv = __double_as_longlong(tol_piv), tdj = __double_as_longlong(tol_dj);
+    int piv = 0, degen = 0, status;
+    bool bland = false;
+    for (;;) {
+        // pricing, alike in every warp
+        long long cost = __double_as_longlong(ob);
+        if (nidl < nfree) cost &= (long long)~kSign;
+        bool el = lane < ncols && cost > tdj && cost <= (long long)kInf;
+        unsigned m = __ballot_sync(FULLMASK, el);
+        if (!m) { status = LP_OPTIMAL; break; }
+        if (!bland) {
+            const unsigned hi = (unsigned)((unsigned long long)cost >> 32), lo = (unsigned)cost;
+            const unsigned hmax = __reduce_max_sync(FULLMASK, el ? hi : 0u);
+            el = el && hi == hmax;
+            m = __ballot_sync(FULLMASK, el);
+            if (m & (m - 1)) {
+                const unsigned lmax = __reduce_max_sync(FULLMASK, el ? lo : 0u);
+                el = el && lo == lmax;
+                m = __ballot_sync(FULLMASK, el);
+            }
+        }
+        if (m & (m - 1)) {
+            const unsigned im = __reduce_min_sync(FULLMASK, el ? (unsigned)nidl : 0xffffffffu);
+            m = __ballot_sync(FULLMASK, el && (unsigned)nidl == im);
+        }
+        const int q = __ffs(m) - 1;
+        const double obq = __shfl_sync(FULLMASK, ob, q);
+        const int eid = __shfl_sync(FULLMASK, nidl, q);
+        const unsigned long long flip = (unsigned long long)__double_as_longlong(obq) & kSign;
+        // ratio test: FP32 quotients of the truncated operands first
+        const double aq = valid ? Ti[q] : 0.0;
+        const unsigned long long a = (unsigned long long)__double_as_longlong(aq) ^ flip;
+        const bool pass = bidr >= nfree && (long long)a > tpiv && a <= kInf;
+        bool unsure = false;
+        float qf = pos_inf<float>();
+        if (pass) {
+            const unsigned long long b = (unsigned long long)__double_as_longlong(Ti[ncols]);
+            if ((long long)b > 0 && b <= kInf) {
+                bool oka, okb;
+                const float af = trunc_float(a, &oka), bf = trunc_float(b, &okb);
+                const float v = __fdividef(bf, af);
+                if (oka && okb && v >= 0x1p-100f) qf = v;
+                else unsure = true;
+            } else {
+                qf = 0.0f;
+            }
+        }
+        const unsigned qw = __reduce_min_sync(FULLMASK, __float_as_uint(qf));
+        if (lane == 0) s->q[w] = qw;
+        __syncthreads();
+        const unsigned qk = min(min(s->q[0], s->q[1]), min(s->q[2], s->q[3]));
+        const float lim = __uint_as_float(qk) * (1.0f + 0x1p-18f);
+        const bool cand = pass && (unsure || qf <= lim);
+        const unsigned cm = __ballot_sync(FULLMASK, cand);
+        if (lane == 0) { s->n[w] = __popc(cm); s->r[w] = 32 * w + __ffs(cm) - 1; }
+        __syncthreads();
+        int ncand = 0, r = -1;
+#pragma unroll
+        for (int v = 0; v < 4; v++) { if (s->n[v]) r = s->r[v]; ncand += s->n[v]; }
+        if (ncand == 0) { status = LP_UNBOUNDED; break; }
+        if (ncand > 1) {
+            // exact quotients of the rows within the FP32 error of the smallest
+            unsigned long long key = ~0ull;
+            if (cand) {
+                double beta = Ti[ncols];
+                if (!(beta > 0.0)) beta = 0.0;
+                key = key_of(ratio_div(beta, __longlong_as_double((long long)a)));
+            }
+            __syncwarp();
+            const int rw = warp_argmin(key, cand ? (unsigned)bidr : 0xffffffffu, i);
+            const unsigned long long kw = __shfl_sync(FULLMASK, key, rw < 0 ? 0 : rw & 31);
+            const unsigned iw = __shfl_sync(FULLMASK, (unsigned)bidr, rw < 0 ? 0 : rw & 31);
+            if (lane == 0) { s->key[w] = rw < 0 ? ~0ull : kw; s->id[w] = rw < 0 ? 0xffffffffu : iw; s->rx[w] = rw; }
+            __syncthreads();
+            unsigned long long kb = ~0ull;
+            unsigned ib = 0xffffffffu;
+            r = -1;
+#pragma unroll
+            for (int v = 0; v < 4; v++)
+                if (s->rx[v] >= 0 && (r < 0 || s->key[v] < kb || (s->key[v] == kb && s->id[v] < ib))) {
+                    kb = s->key[v]; ib = s->id[v]; r = s->rx[v];
+                }
+            if (r < 0) { status = LP_UNBOUNDED; break; }
+        }
+        if (piv >= max_piv) { status = LP_ITER_LIMIT; break; }
+        double *Rp = tab + (size_t)r * ld;
+        const double br = Rp[ncols], prq = Rp[q];
+        const int lid = bid[r];
+        const unsigned long long brb = (unsigned long long)__double_as_longlong(br);
+        bool zero = !((long long)brb > 0 && brb <= kInf);
+        if (!zero && brb < kTiny) zero = ratio_div(br, fabs(prq)) == 0.0;
+        const double inv = __drcp_rn(prq);
+        double rl = lane <= ncols ? Rp[lane] : 0.0;
+        rl = lane == q ? inv : xmul(rl, inv);
+        s->row[w][lane] = rl;
+        __syncthreads();   // every warp has read row r and its id
+        if (w == (r >> 5)) {
+            if (lane <= ncols) Rp[lane] = rl;
+            if (i == r) { bid[r] = (uint8_t)eid; bidr = eid; }
+        }
+        if (valid && i != r) {
+            const double nf = -aq;
+            const double *R = s->row[w];
+            int c = 0;
+            for (; c + 3 <= ncols; c += 4) {
+                double t[4];
+#pragma unroll
+                for (int j = 0; j < 4; j++) t[j] = Ti[c + j];
+#pragma unroll
+                for (int j = 0; j < 4; j++) Ti[c + j] = xfma(nf, R[c + j], t[j]);
+            }
+            for (; c <= ncols; c++) Ti[c] = xfma(nf, R[c], Ti[c]);
+            Ti[q] = xmul(nf, inv);
+        }
+        __syncwarp();
+        if (lane <= ncols) ob = lane == q ? xmul(-obq, inv) : xfma(-obq, rl, ob);
+        if (lane == q) nidl = lid;
+        piv++;
+        degen = zero ? degen + 1 : 0;
+        bland = degen >= degen_switch;
+    }
+    *z_out = __shfl_sync(FULLMASK, ob, ncols);
+    return status;
+}
+
+// k_redundancy with a block of four warps per row's LP (nrows <= 128, nv <= 31).
+// One block per row: the 80 rows of a condensed MPC problem, one LP on each of
+// 80 of the 152 SMs, took 120 us with one warp per LP and take 55 us.
+__global__ void __launch_bounds__(128) k_redundancy_block(const double *M, const double *d, int nrows, int nv, int ld,
+                                                          const int *check, int n_check, double tol, Tol lt, int max_piv,
+                                                          int *out)
+{
+    extern __shared__ __align__(16) unsigned char smem[];
+    double *T = (double *)smem;
+    uint8_t *bid = smem + align16((size_t)(nrows + 1) * ld * sizeof(double));
+    uint8_t *nid = bid + nrows;
+    BlockLp *s = reinterpret_cast<BlockLp *>(smem + redundancy_slot_bytes(nrows, ld));
+    for (int c = blockIdx.x; c < n_check; c += gridDim.x) {
+        const int i = check[c];
+        for (int e = threadIdx.x; e < nrows * nv; e += blockDim.x) {
+            const int r = e / nv, j = e - r * nv;
+            T[(size_t)r * ld + j] = M[e];
+        }
+        for (int r = threadIdx.x; r < nrows; r += blockDim.x) {
+            T[(size_t)r * ld + nv] = d[r] + (r == i ? 1.0 : 0.0);
+            bid[r] = (uint8_t)(nv + r);
+        }
+        for (int j = threadIdx.x; j <= nv; j += blockDim.x) {
+            T[(size_t)nrows * ld + j] = j < nv ? M[(size_t)i * nv + j] : 0.0;
+            if (j < nv) nid[j] = (uint8_t)j;
+        }
+        __syncthreads();
+        double z;
+        const int st = simplex_block64(T, ld, nrows, nv, nv, bid, nid, s, lt.tol_piv, lt.tol_dj, max_piv, lt.degen_switch, &z);
+        if (threadIdx.x == 0) out[c] = (st == LP_OPTIMAL && -z <= d[i] + tol) ? 1 : 0;
+        __syncthreads();
     }
 }
 
@@ -5076,19 +5267,25 @@ cudaError_t launch_opt_screen(const DevBuffers &B, const Tol &tol, const SlotDim
     return cudaGetLastError();
 }
 
-size_t redundancy_smem_bytes(int nrows, int ld)
+// four warps per LP where a thread can hold a row and a warp the objective row
+static bool redundancy_block(int nrows, int nv) { return nrows <= 128 && nv <= 31; }
+
+size_t redundancy_smem_bytes(int nrows, int nv, int ld)
 {
-    return align16((size_t)(nrows + 1) * ld * sizeof(double)) + align16((size_t)nrows + 64);
+    return redundancy_slot_bytes(nrows, ld) + (redundancy_block(nrows, nv) ? sizeof(BlockLp) : 0);
 }
 
 cudaError_t launch_redundancy(const double *M, const double *d, int nrows, int nv, int ld, const int *check, int n_check,
                               double tol, const Tol &lt, int max_piv, int *out, int grid, size_t smem, cudaStream_t s)
 {
+    const bool block = redundancy_block(nrows, nv);
     if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(k_redundancy, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        const void *fn = block ? (const void *)k_redundancy_block : (const void *)k_redundancy;
+        cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
     }
-    k_redundancy<<<grid, 32, smem, s>>>(M, d, nrows, nv, ld, check, n_check, tol, lt, max_piv, out);
+    if (block) k_redundancy_block<<<grid, 128, smem, s>>>(M, d, nrows, nv, ld, check, n_check, tol, lt, max_piv, out);
+    else k_redundancy<<<grid, 32, smem, s>>>(M, d, nrows, nv, ld, check, n_check, tol, lt, max_piv, out);
     return cudaGetLastError();
 }
 

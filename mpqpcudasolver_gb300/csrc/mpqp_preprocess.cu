@@ -3,10 +3,11 @@
 // zero rows, duplicate rows, implicit equalities, redundant rows -- on the
 // rows of [A -F; 0 At] u <= [b; bt], u = (x, theta).  The row comparisons
 // are O(rows^2 (n+p)) host work; the redundancy test is one FP64 LP per row,
-// solved on the device, one warp per row (k_redundancy).
+// solved on the device (k_redundancy_block, or one warp per row: k_redundancy).
 #include <cuda_runtime.h>
 
 #include <cmath>
+#include <cstring>
 #include <string>
 #include <vector>
 
@@ -14,10 +15,12 @@
 #include "mpqp_internal.h"
 
 namespace mq {
-size_t redundancy_smem_bytes(int nrows, int ld);
+size_t redundancy_smem_bytes(int nrows, int nv, int ld);
 cudaError_t launch_redundancy(const double *M, const double *d, int nrows, int nv, int ld, const int *check, int n_check,
                               double tol, const Tol &lt, int max_piv, int *out, int grid, size_t smem, cudaStream_t s);
 void set_error_text(const char *msg);
+void *pool_malloc(size_t bytes);    // from the plans' pool, stream 0
+void pool_free(void *p);
 }  // namespace mq
 
 using namespace mq;
@@ -35,15 +38,9 @@ int fail(int rc, const std::string &msg)
 }
 
 struct DevMem {
-    std::vector<void *> ptrs;
-    ~DevMem() { for (void *p : ptrs) cudaFree(p); }
-    template <typename T> T *alloc(size_t n)
-    {
-        void *p = nullptr;
-        if (cudaMalloc(&p, n * sizeof(T) + 16) != cudaSuccess) return nullptr;
-        ptrs.push_back(p);
-        return (T *)p;
-    }
+    void *p;
+    explicit DevMem(size_t bytes) : p(pool_malloc(bytes)) {}
+    ~DevMem() { if (p) pool_free(p); }
 };
 
 }  // namespace
@@ -123,25 +120,30 @@ static int mpqp_reduce_constraints_impl(const mpqp_problem *prob, int *row_statu
         if (row_status[r] == MPQP_ROW_KEPT) { check.push_back(lp_index[r]); check_pos.push_back(r); }
     const int nrows = (int)lp_rows.size(), n_check = (int)check.size();
     if (n_check == 0) return MPQP_OK;
-    std::vector<double> M((size_t)nrows * nv), dd(nrows);
+    // one block up: the rows, their right-hand sides, the rows to check; the
+    // answers behind it (device memory from the plans' pool: a cudaMalloc and
+    // cudaFree per array took 180 us of a call)
+    const size_t n_dbl = (size_t)nrows * nv + nrows, up = n_dbl * sizeof(double) + n_check * sizeof(int);
+    std::vector<double> img(n_dbl + (n_check + 1) / 2);
+    double *M = img.data(), *dd = M + (size_t)nrows * nv;
     for (int i = 0; i < nrows; i++) {
         for (int j = 0; j < nv; j++) M[(size_t)i * nv + j] = a[(size_t)lp_rows[i] * nv + j];
         dd[i] = d[lp_rows[i]];
     }
-    DevMem mem;
-    double *dM = mem.alloc<double>(M.size()), *dd_dev = mem.alloc<double>(dd.size());
-    int *dcheck = mem.alloc<int>(n_check), *dout = mem.alloc<int>(n_check);
-    if (!dM || !dd_dev || !dcheck || !dout) return fail(MPQP_ENOMEM, "mpqp_reduce_constraints: device allocation failed");
-    if (cudaMemcpy(dM, M.data(), M.size() * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemcpy(dd_dev, dd.data(), dd.size() * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemcpy(dcheck, check.data(), check.size() * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess)
+    memcpy(img.data() + n_dbl, check.data(), n_check * sizeof(int));
+    DevMem mem(img.size() * sizeof(double) + n_check * sizeof(int));
+    if (!mem.p) return fail(MPQP_ENOMEM, "mpqp_reduce_constraints: device allocation failed");
+    const double *dM = (const double *)mem.p, *dd_dev = dM + (size_t)nrows * nv;
+    const int *dcheck = (const int *)(dM + n_dbl);
+    int *dout = (int *)(dM + img.size());
+    if (cudaMemcpy(mem.p, img.data(), up, cudaMemcpyHostToDevice) != cudaSuccess)
         return fail(MPQP_ECUDA, "mpqp_reduce_constraints: upload failed");
     Tol lt{};
     lt.tol_piv = 1e-9;
     lt.tol_dj = 1e-9;
     lt.degen_switch = 8;
     const int ld = (nv + 1) | 1;   // odd FP64 row stride: conflict-free scalar access
-    const size_t smem = redundancy_smem_bytes(nrows, ld);
+    const size_t smem = redundancy_smem_bytes(nrows, nv, ld);
     int dev = 0, sms = 1;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -149,7 +151,6 @@ static int mpqp_reduce_constraints_impl(const mpqp_problem *prob, int *row_statu
     const int max_piv = 4 * (nrows + nv) + 64;
     cudaError_t e = launch_redundancy(dM, dd_dev, nrows, nv, ld, dcheck, n_check, kRedundantTol, lt, max_piv, dout,
                                       grid, smem, 0);
-    if (e == cudaSuccess) e = cudaDeviceSynchronize();
     if (e != cudaSuccess) return fail(MPQP_ECUDA, std::string("mpqp_reduce_constraints: ") + cudaGetErrorString(e));
     std::vector<int> out(n_check);
     if (cudaMemcpy(out.data(), dout, n_check * sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess)
