@@ -794,6 +794,9 @@ static int enqueue(mpqp_plan *P, cudaStream_t s, EventMode events)
     return MPQP_OK;
 }
 
+// share of the usable memory up to which a plan keeps vertex masks
+constexpr double kVertexMaskShare = 0.05;
+
 // The body of mpqp_plan_create (the caller holds g_mu); the launch settings
 // come from the options, 0 selecting the defaults.
 static int plan_create_locked(int n_inst, const mpqp_problem *probs, const mpqp_options *opt_in, mpqp_plan **out)
@@ -959,9 +962,14 @@ static int plan_create_locked(int n_inst, const mpqp_problem *probs, const mpqp_
     node_cap = std::max(node_cap, (long long)n_inst);
     long long hash_cap = 16;
     while (hash_cap < 2 * node_cap + 1) hash_cap <<= 1;
+    // vertex masks beside the hash (16 bytes a slot and side) where they take a
+    // small share of the memory; without them every last-level candidate that
+    // its parent or a sibling does not settle runs its LP
+    const double vmask_bytes = 2.0 * (double)hash_cap * sizeof(VertexMask);
+    const bool vmasks = P->prec == PREC_MIXED && !o.record && !o.exhaustive && vmask_bytes <= kVertexMaskShare * usable;
     long long arena_bytes = o.arena_bytes;
     if (arena_bytes <= 0) {
-        const double used = (double)cand_cap * 12 + (double)node_cap * (2 * sizeof(Node) + 4) +
+        const double used = (vmasks ? vmask_bytes : 0.0) + (double)cand_cap * 12 + (double)node_cap * (2 * sizeof(Node) + 4) +
                             (double)hash_cap * 2 * sizeof(HashSlot) +
                             (P->prec == PREC_MIXED ? (double)cand_cap / 8 * 48 + (double)cand_cap : 0.0) +  // certificate and rerun queues
                             (o.lp2_warm && P->prec == PREC_MIXED ? 16.0 * (double)node_cap : 0.0);   // LP2 bases
@@ -1026,6 +1034,10 @@ static int plan_create_locked(int n_inst, const mpqp_problem *probs, const mpqp_
     B.ids[1] = B.ids[0];
     AL(B.hash[0], sizeof(HashSlot) * hash_cap);
     AL(B.hash[1], sizeof(HashSlot) * hash_cap);
+    if (vmasks) {
+        AL(B.vmask[0], sizeof(VertexMask) * hash_cap);
+        AL(B.vmask[1], sizeof(VertexMask) * hash_cap);
+    }
     AL(B.cand, sizeof(Cand) * cand_cap);
     AL(B.q_lp1, sizeof(int) * cand_cap);
     AL(B.q_opt, sizeof(int) * cand_cap);

@@ -106,7 +106,9 @@ constexpr int kNodeRowsShift = 8;
 // descendant, moved past the right-hand side); 0: all nv columns
 constexpr int kNodeColsShift = 17;
 
+// kCandCert in j: feasible at a certified vertex of one of its subsets (no LP)
 struct Cand { int parent; int j; };
+constexpr int kCandCert = 1 << 8;
 
 struct OptRec {
     uint64_t lo, hi;
@@ -140,6 +142,14 @@ struct CandRec {                // identical field layout to the oracle's record
 // 0.  An entry matches only the run and level that wrote it, so a plan's hash
 // memory (from the pool, possibly an earlier plan's) needs no clearing.
 struct HashSlot { unsigned long long w; };
+
+// Beside a hash slot (mixed precision): the constraints that are nonbasic at
+// the certified vertex of the slot's set, bits 0..kVertexMaxM-1, and the instance in
+// the top 16 bits; zero when the set's tableau was not certified.  Every set of
+// these constraints is feasible at that vertex.  Written where the set's
+// children are its instance's last level.
+struct __align__(16) VertexMask { unsigned long long lo, hi; };
+constexpr int kVertexMaxM = 112, kVertexMaxInst = 1 << 16;
 
 // Per-instance level bookkeeping
 struct InstCtl {
@@ -233,6 +243,7 @@ struct DevBuffers {
     long long ids_cap;
     HashSlot *hash[2];
     long long hash_cap;         // power of two
+    VertexMask *vmask[2];       // parallel to hash (may be null)
     Cand *cand;
     long long cand_cap;
     int *q_lp1;                 // candidate indices for the FP64 LP1 re-solve

@@ -128,19 +128,21 @@ __device__ __forceinline__ unsigned long long hash_tag(int epoch, int level)
     return (unsigned long long)(((unsigned)epoch * 64u + (unsigned)level) % 0xffffffu + 1u);
 }
 
-__device__ int hash_find_from(const HashSlot *tab, long long cap, unsigned long long tag, uint64_t fp, uint64_t s)
+// the slot of the set, from slot s on; -1: not there
+__device__ long long hash_find_from(const HashSlot *tab, long long cap, unsigned long long tag, uint64_t fp, uint64_t s)
 {
     const unsigned long long f40 = fp >> 24;
     for (long long probe = 0; probe < cap; probe++) {
         const unsigned long long w = tab[s].w;
         if ((w >> 40) != tag) return -1;
-        if ((w & kFpMask) == f40) return 1;
+        if ((w & kFpMask) == f40) return (long long)s;
         s = (s + 1) & (uint64_t)(cap - 1);
     }
     return -1;
 }
 
-__device__ bool hash_insert(HashSlot *tab, long long cap, unsigned long long tag, int inst, uint64_t lo, uint64_t hi)
+// the slot the set went to; -1: the table is full
+__device__ long long hash_insert(HashSlot *tab, long long cap, unsigned long long tag, int inst, uint64_t lo, uint64_t hi)
 {
     const uint64_t fp = hash_key(inst, lo, hi);
     const unsigned long long w = (tag << 40) | (fp >> 24);
@@ -149,12 +151,12 @@ __device__ bool hash_insert(HashSlot *tab, long long cap, unsigned long long tag
         unsigned long long *h = &tab[s].w;
         const unsigned long long t = *((volatile unsigned long long *)h);
         if ((t >> 40) != tag) {
-            if (atomicCAS(h, t, w) == t) return true;
+            if (atomicCAS(h, t, w) == t) return (long long)s;
             continue;   // lost the slot to another insert: read it again
         }
         s = (s + 1) & (uint64_t)(cap - 1);
     }
-    return false;
+    return -1;
 }
 
 // ---------------------------------------------------------------------
@@ -813,13 +815,13 @@ __host__ __device__ inline size_t lp1_slot_bytes(int maxM1, int maxLD1, int maxN
     return lp1_buf_bytes<T>(maxM1, maxLD1, maxNv) + 16;
 }
 
-// slot of k_feasibility: one buffer, the arena offsets reserved for the chunk's
-// candidates and the warp's mbarrier (16 bytes, last)
+// slot of k_feasibility: one buffer, the vertex masks and the arena offsets
+// reserved for the chunk's candidates, and the warp's mbarrier (16 bytes, last)
 constexpr int kChunkOffsets = 2 * 32;
 template <typename T>
 __host__ __device__ inline size_t feas_slot_bytes(int maxM1, int maxLD1, int maxNv)
 {
-    return lp1_buf_bytes<T>(maxM1, maxLD1, maxNv) + kChunkOffsets * sizeof(long long) + 16;
+    return lp1_buf_bytes<T>(maxM1, maxLD1, maxNv) + 32 * sizeof(VertexMask) + kChunkOffsets * sizeof(long long) + 16;
 }
 
 // candidates a warp claims at a time (a plan setting, at most 32, by default
@@ -1031,8 +1033,18 @@ __global__ void k_enumerate(DevBuffers B, int level)
             const uint64_t clo0 = __shfl_sync(FULLMASK, plo, t), chi0 = __shfl_sync(FULLMASK, phi, t);
             const int cinst = __shfl_sync(FULLMASK, pinst, t);
             const int j = __shfl_sync(FULLMASK, jmin, t) + (idx - __shfl_sync(FULLMASK, excl, t));
-            bool ok = valid;
+            bool ok = valid, cert = false;
             if (ok && !B.exhaustive) {
+                // at its instance's last level a candidate needs no tableau of
+                // its own: it is feasible when one of its subsets has a certified
+                // vertex at which all of the candidate's slacks are nonbasic.
+                // Each subset's vertex has the missing element with a chance of
+                // about one in five, so three quarters of the candidates are
+                // settled here: m = 62 batch (48M last-level candidates) LP1 167
+                // -> 101 ms for 5 ms more in this kernel, 64 MPC problems 3.47 ->
+                // 2.15 ms, m = 62 to |S| = 4 1.70 -> 1.14 ms
+                const VertexMask *vtab = B.vmask[pside];
+                const bool want = vtab && level == B.inst[cinst].k_max;
                 uint64_t lo = clo0, hi = chi0;
                 if (j < 64) lo |= 1ull << j; else hi |= 1ull << (j - 64);
                 // the subsets child minus a, a in the parent, four at a time: the
@@ -1064,10 +1076,21 @@ __global__ void k_enumerate(DevBuffers B, int level)
                     for (int g = 0; g < G; g++) {
                         if (g < n && ok) {
                             if ((hs[g].w >> 40) != tag_prev) ok = false;
-                            else if ((hs[g].w & kFpMask) != (sfp[g] >> 24))
-                                ok = hash_find_from(tab, hcap, tag_prev, sfp[g],
-                                                    (sidx[g] + 1) & (uint64_t)(hcap - 1)) >= 0;
+                            else if ((hs[g].w & kFpMask) != (sfp[g] >> 24)) {
+                                const long long at = hash_find_from(tab, hcap, tag_prev, sfp[g],
+                                                                    (sidx[g] + 1) & (uint64_t)(hcap - 1));
+                                ok = at >= 0;
+                                sidx[g] = ok ? (uint64_t)at : sidx[g];
+                            }
                         }
+                    }
+                    if (ok && want && !cert) {
+                        VertexMask v[G];
+#pragma unroll
+                        for (int g = 0; g < G; g++) v[g] = g < n ? vtab[sidx[g]] : VertexMask{0, 0};
+#pragma unroll
+                        for (int g = 0; g < G; g++)
+                            cert |= (int)(v[g].hi >> 48) == cinst && (v[g].lo & lo) == lo && (v[g].hi & hi) == hi;
                     }
                 }
             }
@@ -1098,7 +1121,7 @@ __global__ void k_enumerate(DevBuffers B, int level)
                 const long long ci = base + __popc(okm & below);
                 if (ci < B.cand_cap) {
                     B.cand[ci].parent = (int)(p0 + t);
-                    B.cand[ci].j = j;
+                    B.cand[ci].j = cert ? j | kCandCert : j;
                 } else {
                     atomicOr(&ctl->overflow, OV_CAND);
                 }
@@ -1154,6 +1177,18 @@ __device__ __forceinline__ void warp_copy_v(T *dst, const T *src, int n)
     const int4 *s4 = reinterpret_cast<const int4 *>(src);
     int4 *d4 = reinterpret_cast<int4 *>(dst);
     for (int e = lane_id(); e < n4; e += 32) d4[e] = s4[e];
+}
+
+// A feasible set into the level's hash, with its vertex mask where its children
+// are the instance's last level (zero elsewhere: every slot of a run has one of
+// that run, so a set found by a fingerprint collision brings a mask that is
+// sound for what it says).
+__device__ __forceinline__ void insert_node(const DevBuffers &B, int side, int level, const InstDesc &I, int inst,
+                                            uint64_t lo, uint64_t hi, long long hcap, VertexMask vm)
+{
+    const long long s = hash_insert(B.hash[side], hcap, hash_tag(B.ctl->epoch, level), inst, lo, hi);
+    if (s < 0) atomicOr(&B.ctl->overflow, OV_HASH);
+    else if (B.vmask[side]) B.vmask[side][s] = level + 1 == I.k_max ? vm : VertexMask{0, 0};
 }
 
 // Append a feasible (or, exhaustive, any) candidate as a node of `side`;
@@ -1217,10 +1252,7 @@ __device__ long long store_node(const DevBuffers &B, int side, int level, const 
             nd.flags = NODE_VALID | (feasible ? NODE_FEASIBLE : 0) | (extra_flags & ~NODE_CERT);
             nd.tab_off = -1; nd.ids_off = -1; nd.rec = rec;
             B.node[side][idx] = nd;
-            if (feasible && !B.exhaustive && !chunked) {
-                if (!hash_insert(B.hash[side], hcap, hash_tag(ctl->epoch, level), inst, lo, hi))
-                    atomicOr(&ctl->overflow, OV_HASH);
-            }
+            if (feasible && !B.exhaustive && !chunked) insert_node(B, side, level, I, inst, lo, hi, hcap, VertexMask{0, 0});
         }
         return idx;
     }
@@ -1262,10 +1294,8 @@ __device__ long long store_node(const DevBuffers &B, int side, int level, const 
         nd.tab_off = toff; nd.ids_off = ioff; nd.rec = rec;
         B.node[side][idx] = nd;
         // the hash serves the subset test of the next level only
-        if (feasible && !B.exhaustive && need_tab && !chunked) {
-            if (!hash_insert(B.hash[side], hcap, hash_tag(ctl->epoch, level), inst, lo, hi))
-                atomicOr(&ctl->overflow, OV_HASH);
-        }
+        if (feasible && !B.exhaustive && need_tab && !chunked)
+            insert_node(B, side, level, I, inst, lo, hi, hcap, VertexMask{0, 0});
     }
     return idx;
 }
@@ -1308,6 +1338,23 @@ __device__ __noinline__ int retire_fixed_columns(float *tab, int ld, int nrows, 
         ncols = last;
     }
     return ncols;
+}
+
+// nb: the constraints (bits, m <= 128) among the nv nonbasic ids, warp-uniform
+__device__ __forceinline__ void nonbasic_mask(const uint8_t *nid, int nv, int m, unsigned (&nb)[4])
+{
+    nb[0] = nb[1] = nb[2] = nb[3] = 0;
+    for (int cc = lane_id(); cc < nv; cc += 32) {
+        const int id = (int)nid[cc] - nv;
+        if (id >= 0 && id < m) {
+            const unsigned bit = 1u << (id & 31);
+            const int wd = id >> 5;
+#pragma unroll
+            for (int k = 0; k < 4; k++) nb[k] |= wd == k ? bit : 0u;
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 4; k++) nb[k] = __reduce_or_sync(FULLMASK, nb[k]);
 }
 
 // An FP32 LP1 candidate without a final verdict, by one lane: with nid (the
@@ -1421,6 +1468,7 @@ __device__ __forceinline__ void feasibility_body(const DevBuffers &B, const Tol 
     uint8_t *ids = base + align16((((size_t)(sd.maxM1 + 1) * mld + 3) & ~(size_t)3) * sizeof(T));
     uint64_t *bar = (uint64_t *)(base + slot - 16);
     long long *room = (long long *)(base + slot - 16) - kChunkOffsets;
+    VertexMask *vms = (VertexMask *)room - 32;
     const int side = level & 1, pside = side ^ 1;
     Ctl *ctl = B.ctl;
     const long long ncand = ctl->n_cand;
@@ -1441,7 +1489,9 @@ __device__ __forceinline__ void feasibility_body(const DevBuffers &B, const Tol 
         w0 = __shfl_sync(FULLMASK, w0, 0);
         if (w0 >= wend || abort) break;
         const int cnt = wend - w0 < chunk ? (int)(wend - w0) : chunk;
-        const Cand mine = lane < cnt ? B.cand[w0 + lane] : Cand{-1, 0};
+        Cand mine = lane < cnt ? B.cand[w0 + lane] : Cand{-1, 0};
+        const bool cert = (mine.j & kCandCert) != 0;
+        mine.j &= kCandCert - 1;
         // candidate w's node goes to slot w (also when the FP64 re-solve
         // stores it); a candidate that stores none leaves an invalid record
         // with its reserved arena space (below)
@@ -1456,12 +1506,13 @@ __device__ __forceinline__ void feasibility_body(const DevBuffers &B, const Tol 
         // pair per stored candidate, whose round trip the warp waited for.  With
         // the hash inserts below: LP1 of 32 mpLPs (1.7M sets, 1.7 pivots each)
         // 5,248 -> 3,297 us, of the m = 62 batch 177 -> 167 ms
-        bool keeps = false;   // this lane's candidate stores a tableau when feasible
+        bool live = false;    // this lane's candidate is checked (its instance has not stopped)
+        bool keeps = false;   // ... and stores a tableau when feasible
         {
             const InstDesc &Il = B.inst[my_inst];
             const InstCtl &il = B.ictl[my_inst];
-            keeps = lane < cnt && level < Il.k_max && !il.stopped &&
-                    !(Il.budget > 0 && il.cum_cand + il.lvl_cand > Il.budget);
+            live = lane < cnt && !il.stopped && !(Il.budget > 0 && il.cum_cand + il.lvl_cand > Il.budget);
+            keeps = live && level < Il.k_max;
             const int te = keeps ? Il.tab_elems : 0, ib = keeps ? Il.ids_bytes : 0;
             int ts = te, is = ib;   // inclusive sums
 #pragma unroll
@@ -1508,8 +1559,8 @@ __device__ __forceinline__ void feasibility_body(const DevBuffers &B, const Tol 
         const bool at_vertex = mixed && !B.rec && !B.exhaustive;
         unsigned done = 0;
         if (at_vertex) {
-            bool q = false;
-            if (lane < cnt) {
+            bool q = cert;
+            if (lane < cnt && !cert) {
                 const Node &pn = B.node[pside][mine.parent];
                 const InstDesc &Il = B.inst[pn.inst];
                 if ((pn.flags & NODE_CERT) && pn.ids_off >= 0 && level == Il.k_max) {
@@ -1520,17 +1571,46 @@ __device__ __forceinline__ void feasibility_body(const DevBuffers &B, const Tol 
             }
             done = __ballot_sync(FULLMASK, q);
         }
-    for (int t = 0; t < cnt; t++) {
+        // the candidates already settled, a lane each: nodes of the last level
+        // (no tableau, nothing into the hash)
+        unsigned todo = cnt == 32 ? FULLMASK : (1u << cnt) - 1u;
+        if (done) {
+            const unsigned settled = __ballot_sync(FULLMASK, ((done >> lane) & 1u) && live);
+            todo &= ~done;
+            if ((settled >> lane) & 1u) {
+                const Node &pn = B.node[pside][mine.parent];
+                Node nd;
+                nd.lo = pn.lo; nd.hi = pn.hi; nd.inst = my_inst;
+                if (mine.j < 64) nd.lo |= 1ull << mine.j; else nd.hi |= 1ull << (mine.j - 64);
+                nd.flags = NODE_VALID | NODE_FEASIBLE;
+                nd.tab_off = -1; nd.ids_off = -1; nd.rec = -1;
+                if (nbase + lane < B.node_cap) B.node[side][nbase + lane] = nd;
+                else atomicOr(&ctl->overflow, OV_NODE);
+                // counted once per instance among these lanes
+                const unsigned grp = __match_any_sync(settled, my_inst);
+                const unsigned long long dg = mask_digest(nd.lo, nd.hi);
+                unsigned long long sum = 0;
+                for (unsigned g = grp; g; g &= g - 1) sum += __shfl_sync(grp, dg, __ffs(g) - 1);
+                if (lane == __ffs(grp) - 1) {
+                    atomicAdd((unsigned long long *)&B.ictl[my_inst].feasible, (unsigned long long)__popc(grp));
+                    atomicAdd(&B.ictl[my_inst].feas_digest, sum);
+                }
+            }
+            __syncwarp();
+        }
+    for (; todo; todo &= todo - 1) {
+        const int t = __ffs(todo) - 1;
         const long long w = w0 + t;
         Cand c;
         c.parent = __shfl_sync(FULLMASK, mine.parent, t);
         c.j = __shfl_sync(FULLMASK, mine.j, t);
         {
             // the next candidate's parent into L2 while this one is solved
-            const int np = __shfl_sync(FULLMASK, mine.parent, (t + 1) & 31);
-            const long long ntoff = __shfl_sync(FULLMASK, my_toff, (t + 1) & 31);
-            const int ninst = __shfl_sync(FULLMASK, my_inst, (t + 1) & 31);
-            if (lane == 0 && t + 1 < cnt && np != c.parent && ntoff >= 0)
+            const int nt = __ffs(todo & (todo - 1)) - 1;   // -1: none
+            const int np = __shfl_sync(FULLMASK, mine.parent, nt & 31);
+            const long long ntoff = __shfl_sync(FULLMASK, my_toff, nt & 31);
+            const int ninst = __shfl_sync(FULLMASK, my_inst, nt & 31);
+            if (lane == 0 && nt >= 0 && np != c.parent && ntoff >= 0)
                 bulk_prefetch_l2((const T *)B.tab[pside] + ntoff, (unsigned)(B.inst[ninst].tab_elems * sizeof(T)));
         }
         const Node par = B.node[pside][c.parent];
@@ -1748,24 +1828,24 @@ __device__ __forceinline__ void feasibility_body(const DevBuffers &B, const Tol 
             if (level < I.k_max) {
                 lc.d += room[t] >= 0;
                 if (feasible && !B.exhaustive) stored |= 1u << t;
+                if (B.vmask[side] && level + 1 == I.k_max) {
+                    // the constraints nonbasic at this certified vertex
+                    unsigned nb[4];
+                    nonbasic_mask(nid, nv, I.m, nb);
+                    const bool fits = feasible && I.m <= kVertexMaxM && inst < kVertexMaxInst;
+                    if (lane == 0) {
+                        vms[t].lo = fits ? nb[0] | (unsigned long long)nb[1] << 32 : 0ull;
+                        vms[t].hi = fits ? nb[2] | (unsigned long long)nb[3] << 32 | (unsigned long long)inst << 48 : 0ull;
+                    }
+                }
             }
         }
         if (at_vertex && feasible && level == I.k_max) {
             // later siblings whose new slack is nonbasic at this vertex
-            unsigned nb0 = 0, nb1 = 0, nb2 = 0, nb3 = 0;
-            for (int cc = lane; cc < nv; cc += 32) {
-                const int id = (int)nid[cc] - nv;
-                if (id >= 0 && id < I.m) {
-                    const unsigned bit = 1u << (id & 31);
-                    const int wd = id >> 5;
-                    nb0 |= wd == 0 ? bit : 0u; nb1 |= wd == 1 ? bit : 0u;
-                    nb2 |= wd == 2 ? bit : 0u; nb3 |= wd == 3 ? bit : 0u;
-                }
-            }
-            nb0 = __reduce_or_sync(FULLMASK, nb0); nb1 = __reduce_or_sync(FULLMASK, nb1);
-            nb2 = __reduce_or_sync(FULLMASK, nb2); nb3 = __reduce_or_sync(FULLMASK, nb3);
+            unsigned nb[4];
+            nonbasic_mask(nid, nv, I.m, nb);
             const int mj = mine.j;
-            const unsigned wsel = mj < 32 ? nb0 : mj < 64 ? nb1 : mj < 96 ? nb2 : nb3;
+            const unsigned wsel = mj < 32 ? nb[0] : mj < 64 ? nb[1] : mj < 96 ? nb[2] : nb[3];
             done |= __ballot_sync(FULLMASK, lane > t && lane < cnt && mine.parent == c.parent && ((wsel >> (mj & 31)) & 1u));
         }
     }
@@ -1775,8 +1855,7 @@ __device__ __forceinline__ void feasibility_body(const DevBuffers &B, const Tol 
         __syncwarp();
         if (((stored >> lane) & 1u) && nbase + lane < B.node_cap) {
             const Node nd = B.node[side][nbase + lane];
-            if (!hash_insert(B.hash[side], hcap, hash_tag(ctl->epoch, level), nd.inst, nd.lo, nd.hi))
-                atomicOr(&ctl->overflow, OV_HASH);
+            insert_node(B, side, level, B.inst[nd.inst], nd.inst, nd.lo, nd.hi, hcap, vms[lane]);
         }
         __syncwarp();
     }
@@ -4922,7 +5001,7 @@ __global__ void k_level0(DevBuffers B)
         nd.rec = (B.rec && inst < B.rec_cap) ? inst : -1;
         B.node[0][inst] = nd;
         if (!B.exhaustive) {
-            hash_insert(B.hash[0], hash_cap_for(B, B.n_inst), hash_tag(ctl->epoch, 0), inst, 0, 0);
+            insert_node(B, 0, 0, I, inst, 0, 0, hash_cap_for(B, B.n_inst), VertexMask{0, 0});
         }
         if (nd.rec >= 0) {
             CandRec &R = B.rec[nd.rec];
