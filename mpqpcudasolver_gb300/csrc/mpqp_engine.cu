@@ -39,6 +39,7 @@ bool screen_lanes_route(int mode, const InstDesc &I, const SlotDims &sd);
 size_t laws_smem_per_warp(const SlotDims &sd);
 const void *kernel_ptr(const char *name);
 cudaError_t launch_enumerate(const DevBuffers &B, int level, int grid, cudaStream_t s);
+cudaError_t launch_cover(const DevBuffers &B, int level, int grid, cudaStream_t s);
 cudaError_t launch_feasibility(const DevBuffers &B, const Tol &tol, const SlotDims &sd, int level, int prec,
                                int grid, size_t smem, cudaStream_t s, int warps, int chunk);
 cudaError_t launch_lp1_fp64(const DevBuffers &B, const Tol &tol, const SlotDims &sd, int level, int grid,
@@ -410,6 +411,8 @@ struct mpqp_plan {
     size_t smem_tiles = 0;
     int grid_lanes = 0;         // ... at levels |S| <= kLaneMaxK: one set per thread
     size_t smem_lanes = 0;
+    std::vector<char> last_after;   // per level: the next one is some instance's last
+    int grid_cover = 0;
     std::vector<double> lvl_sets;   // per level, an upper bound on the batch's sets (combinatorial, budgets)
     int grid_direct = 0;        // k_optimality<double> over a whole small level (mixed precision)
     int lane_cap = 3;           // pivots of its first pass (MPQP_SCREEN_CAP)
@@ -651,6 +654,13 @@ static int grid_for(const void *fn, size_t smem, int *grid, int block = 128)
 // (592K) 2,566, 2,284 and 2,280 us; beyond that no change
 constexpr double kDirectWaves = 3.0, kOnePassWaves = 4.0;
 
+// sets of the next level from which a level's vertices are spread over its cover
+// slots (k_cover): the launch's 10 to 25 us are a loss below.  Enumeration
+// without / with it, sets of the last level: m = 40 to |S| = 3 (9,880) 427 / 439
+// us, m = 62 to 3 (37,820) 703 / 708, m = 40 to 4 (91,390) 921 / 927, m = 84 to 3
+// (95,284) 1,191 / 1,169, m = 48 to 4 (194,580) 1,314 / 1,264
+constexpr double kCoverMin = 100000.0;
+
 // The fixed launch sequence of one enumeration.  events: none; one before every
 // launch (and one after the last), for the per-kernel times; or one wherever
 // the sequence changes between its LP1 and its optimality phase (phase_times).
@@ -787,6 +797,8 @@ static int enqueue(mpqp_plan *P, cudaStream_t s, EventMode events)
         { const int _o = launch_opt(k); if (_o) return _o; }
         { const int _o = launch_optfb(k); if (_o) return _o; }
         L("k_finalize", launch_finalize(B, k, s));
+        if (B.cover[0] && P->last_after[k] && P->lvl_sets[k + 1] >= kCoverMin)
+            L("k_cover", launch_cover(B, k, grid(P->grid_cover, k, 64), s));
     }
 #undef L
     if (events != EV_NONE) { const int _r = record(); if (_r) return _r; }
@@ -794,8 +806,8 @@ static int enqueue(mpqp_plan *P, cudaStream_t s, EventMode events)
     return MPQP_OK;
 }
 
-// share of the usable memory up to which a plan keeps vertex masks
-constexpr double kVertexMaskShare = 0.05;
+// share of the usable memory a plan's cover slots may take
+constexpr double kCoverShare = 0.05;
 
 // The body of mpqp_plan_create (the caller holds g_mu); the launch settings
 // come from the options, 0 selecting the defaults.
@@ -943,6 +955,8 @@ static int plan_create_locked(int n_inst, const mpqp_problem *probs, const mpqp_
             }
         }
         P->lvl_sets = lvl;
+        P->last_after.assign(lvl.size(), 0);
+        for (const InstDesc &d : P->desc) if (d.k_max > 1) P->last_after[d.k_max - 1] = 1;
         for (int k = 0; k <= kMaxK; k++) {
             lvl_max = std::max(lvl_max, lvl[k]);
             arena_max = std::max(arena_max, lvl_tab[k] + lvl_tab[k + 1]);
@@ -962,14 +976,17 @@ static int plan_create_locked(int n_inst, const mpqp_problem *probs, const mpqp_
     node_cap = std::max(node_cap, (long long)n_inst);
     long long hash_cap = 16;
     while (hash_cap < 2 * node_cap + 1) hash_cap <<= 1;
-    // vertex masks beside the hash (16 bytes a slot and side) where they take a
-    // small share of the memory; without them every last-level candidate that
-    // its parent or a sibling does not settle runs its LP
-    const double vmask_bytes = 2.0 * (double)hash_cap * sizeof(VertexMask);
-    const bool vmasks = P->prec == PREC_MIXED && !o.record && !o.exhaustive && vmask_bytes <= kVertexMaskShare * usable;
+    // cover slots beside the hash (mixed precision), as many as a small share of
+    // the memory holds: a last-level candidate without them runs its LP unless
+    // its parent or a sibling settles it
+    long long cover_cap = 0;
+    if (P->prec == PREC_MIXED && !o.record && !o.exhaustive) {
+        cover_cap = hash_cap;
+        while (cover_cap >= 1024 && 2.0 * (double)cover_cap * sizeof(CoverSlot) > kCoverShare * usable) cover_cap >>= 1;
+    }
     long long arena_bytes = o.arena_bytes;
     if (arena_bytes <= 0) {
-        const double used = (vmasks ? vmask_bytes : 0.0) + (double)cand_cap * 12 + (double)node_cap * (2 * sizeof(Node) + 4) +
+        const double used = 2.0 * (double)cover_cap * sizeof(CoverSlot) + (double)cand_cap * 12 + (double)node_cap * (2 * sizeof(Node) + 4) +
                             (double)hash_cap * 2 * sizeof(HashSlot) +
                             (P->prec == PREC_MIXED ? (double)cand_cap / 8 * 48 + (double)cand_cap : 0.0) +  // certificate and rerun queues
                             (o.lp2_warm && P->prec == PREC_MIXED ? 16.0 * (double)node_cap : 0.0);   // LP2 bases
@@ -1034,9 +1051,10 @@ static int plan_create_locked(int n_inst, const mpqp_problem *probs, const mpqp_
     B.ids[1] = B.ids[0];
     AL(B.hash[0], sizeof(HashSlot) * hash_cap);
     AL(B.hash[1], sizeof(HashSlot) * hash_cap);
-    if (vmasks) {
-        AL(B.vmask[0], sizeof(VertexMask) * hash_cap);
-        AL(B.vmask[1], sizeof(VertexMask) * hash_cap);
+    B.cover_cap = cover_cap;
+    if (cover_cap) {
+        AL(B.cover[0], sizeof(CoverSlot) * cover_cap);
+        AL(B.cover[1], sizeof(CoverSlot) * cover_cap);
     }
     AL(B.cand, sizeof(Cand) * cand_cap);
     AL(B.q_lp1, sizeof(int) * cand_cap);
@@ -1104,6 +1122,7 @@ static int plan_create_locked(int n_inst, const mpqp_problem *probs, const mpqp_
     if ((rc = grid_for(kernel_ptr("enumerate"), 0, &P->grid_enum)) ||
         (rc = grid_for(kernel_ptr(P->prec == PREC_MIXED ? "feas32" : "feas64"), P->smem_feas, &P->grid_feas,
                        32 * P->feas_warps)) ||
+        (rc = grid_for(kernel_ptr("cover"), 0, &P->grid_cover)) ||
         (rc = grid_for(kernel_ptr("lp1_fp64"), P->smem_lp1fb, &P->grid_lp1fb)) ||
         (rc = grid_for(kernel_ptr("lp1_cert"), P->smem_cert, &P->grid_cert)) ||
         (rc = P->prec == PREC_MIXED

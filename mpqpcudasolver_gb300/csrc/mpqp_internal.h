@@ -106,7 +106,7 @@ constexpr int kNodeRowsShift = 8;
 // descendant, moved past the right-hand side); 0: all nv columns
 constexpr int kNodeColsShift = 17;
 
-// kCandCert in j: feasible at a certified vertex of one of its subsets (no LP)
+// kCandCert in j: known feasible from one of its subsets' cover slots (no LP)
 struct Cand { int parent; int j; };
 constexpr int kCandCert = 1 << 8;
 
@@ -143,13 +143,14 @@ struct CandRec {                // identical field layout to the oracle's record
 // memory (from the pool, possibly an earlier plan's) needs no clearing.
 struct HashSlot { unsigned long long w; };
 
-// Beside a hash slot (mixed precision): the constraints that are nonbasic at
-// the certified vertex of the slot's set, bits 0..kVertexMaxM-1, and the instance in
-// the top 16 bits; zero when the set's tableau was not certified.  Every set of
-// these constraints is feasible at that vertex.  Written where the set's
-// children are its instance's last level.
-struct __align__(16) VertexMask { unsigned long long lo, hi; };
-constexpr int kVertexMaxM = 112, kVertexMaxInst = 1 << 16;
+// Beside a hash slot (mixed precision), where the children of the slot's set S
+// are its instance's last level: the constraints x for which S u {x} is known
+// feasible (m), and S itself with the instance in the top 16 bits of shi.  m
+// starts as the constraints nonbasic at the certified vertex of S's tableau, all
+// feasible there together; k_cover adds those of the vertices of other sets that
+// lie on S's face too.
+struct __align__(16) CoverSlot { unsigned long long mlo, mhi, slo, shi; };
+constexpr int kCoverMaxM = 112, kCoverMaxInst = 1 << 16;
 
 // Per-instance level bookkeeping
 struct InstCtl {
@@ -243,7 +244,8 @@ struct DevBuffers {
     long long ids_cap;
     HashSlot *hash[2];
     long long hash_cap;         // power of two
-    VertexMask *vmask[2];       // parallel to hash (may be null)
+    CoverSlot *cover[2];        // parallel to the first cover_cap slots of hash (may be null)
+    long long cover_cap;
     Cand *cand;
     long long cand_cap;
     int *q_lp1;                 // candidate indices for the FP64 LP1 re-solve

@@ -122,6 +122,7 @@ __device__ __forceinline__ long long hash_cap_for(const DevBuffers &B, long long
 // (a superset of an infeasible set) is infeasible, so no verdict depends on it.
 __device__ unsigned g_hash_epoch;
 constexpr unsigned long long kFpMask = (1ull << 40) - 1;
+constexpr unsigned long long kCoverLow = (1ull << 48) - 1;   // the set's part of CoverSlot::shi
 
 __device__ __forceinline__ unsigned long long hash_tag(int epoch, int level)
 {
@@ -821,7 +822,7 @@ constexpr int kChunkOffsets = 2 * 32;
 template <typename T>
 __host__ __device__ inline size_t feas_slot_bytes(int maxM1, int maxLD1, int maxNv)
 {
-    return lp1_buf_bytes<T>(maxM1, maxLD1, maxNv) + 32 * sizeof(VertexMask) + kChunkOffsets * sizeof(long long) + 16;
+    return lp1_buf_bytes<T>(maxM1, maxLD1, maxNv) + 64 * sizeof(unsigned long long) + kChunkOffsets * sizeof(long long) + 16;
 }
 
 // candidates a warp claims at a time (a plan setting, at most 32, by default
@@ -1043,8 +1044,8 @@ __global__ void k_enumerate(DevBuffers B, int level)
                 // settled here: m = 62 batch (48M last-level candidates) LP1 167
                 // -> 101 ms for 5 ms more in this kernel, 64 MPC problems 3.47 ->
                 // 2.15 ms, m = 62 to |S| = 4 1.70 -> 1.14 ms
-                const VertexMask *vtab = B.vmask[pside];
-                const bool want = vtab && level == B.inst[cinst].k_max;
+                const CoverSlot *ctab = B.cover[pside];
+                const bool want = ctab && level == B.inst[cinst].k_max;
                 uint64_t lo = clo0, hi = chi0;
                 if (j < 64) lo |= 1ull << j; else hi |= 1ull << (j - 64);
                 // the subsets child minus a, a in the parent, four at a time: the
@@ -1085,12 +1086,18 @@ __global__ void k_enumerate(DevBuffers B, int level)
                         }
                     }
                     if (ok && want && !cert) {
-                        VertexMask v[G];
-#pragma unroll
-                        for (int g = 0; g < G; g++) v[g] = g < n ? vtab[sidx[g]] : VertexMask{0, 0};
+                        CoverSlot v[G];
 #pragma unroll
                         for (int g = 0; g < G; g++)
-                            cert |= (int)(v[g].hi >> 48) == cinst && (v[g].lo & lo) == lo && (v[g].hi & hi) == hi;
+                            v[g] = g < n && (long long)sidx[g] < B.cover_cap ? ctab[sidx[g]] : CoverSlot{0, 0, ~0ull, ~0ull};
+#pragma unroll
+                        for (int g = 0; g < G; g++) {
+                            // the slot is this subset's own, and has the missing element
+                            const unsigned long long slo = v[g].slo, shi = v[g].shi & kCoverLow;
+                            cert |= (int)(v[g].shi >> 48) == cinst && (slo & ~lo) == 0 && (shi & ~hi) == 0 &&
+                                    __popcll(slo) + __popcll(shi) == level - 1 && (v[g].mlo & (lo ^ slo)) == (lo ^ slo) &&
+                                    (v[g].mhi & (hi ^ shi)) == (hi ^ shi);
+                        }
                     }
                 }
             }
@@ -1149,6 +1156,92 @@ __global__ void k_enumerate(DevBuffers B, int level)
     }
 }
 
+// Whether the sets of a level have cover slots: their children are the
+// instance's last level.
+__device__ __forceinline__ bool covers(const InstDesc &I, int inst, int level)
+{
+    return level + 1 == I.k_max && I.m <= kCoverMaxM && inst < kCoverMaxInst;
+}
+
+// elements a of S that k_cover replaces (the largest).  With 0, 1, 2, 3 and all
+// of them the m = 62 batch's LP1 takes 102.7, 93.0, 87.6, 84.6 and 81.9 ms, and
+// k_cover 0, 2.0, 5.4, 9.0 and 16.4 ms (before its loads were grouped, 4.7 with).
+constexpr int kCoverSpread = 2;
+
+// Spreads the certified vertices of a level whose children are last-level
+// candidates: the constraints N nonbasic at a set S's vertex are feasible
+// together, so for every other set S' of |S| elements of N, all of N belongs in
+// the cover slot of S'.  Done for the S' = S - a + b, b in N - S, a lane per S
+// and a, four b at a time; bound by the random accesses (the latency of their
+// chains on a small level).
+__global__ void __launch_bounds__(128) k_cover(DevBuffers B, int level)
+{
+    const int side = level & 1;
+    const Ctl *ctl = B.ctl;
+    const HashSlot *tab = B.hash[side];
+    const long long nn = ctl->n_node[side] < B.node_cap ? ctl->n_node[side] : B.node_cap;
+    const unsigned long long tag = hash_tag(ctl->epoch, level);
+    const long long hcap = ctl->hcap[side] >= 16 && ctl->hcap[side] <= B.hash_cap ? ctl->hcap[side] : B.hash_cap;
+    for (long long x = (long long)blockIdx.x * blockDim.x + threadIdx.x; x < nn * kCoverSpread;
+         x += (long long)gridDim.x * blockDim.x) {
+        const Node nd = B.node[side][x / kCoverSpread];
+        if ((nd.flags & (NODE_VALID | NODE_FEASIBLE | NODE_CERT)) != (NODE_VALID | NODE_FEASIBLE | NODE_CERT) || nd.ids_off < 0)
+            continue;
+        const InstDesc &I = B.inst[nd.inst];
+        if (!covers(I, nd.inst, level) || B.ictl[nd.inst].stopped) continue;
+        // S without its (x % kCoverSpread)-th largest element
+        uint64_t clo = nd.lo, chi = nd.hi;
+        for (int e = (int)(x % kCoverSpread); e > 0; e--) {
+            if (chi) chi &= ~(1ull << (63 - __clzll((long long)chi)));
+            else if (clo) clo &= ~(1ull << (63 - __clzll((long long)clo)));
+        }
+        if (!(clo | chi)) continue;
+        const uint64_t ah = chi ? 1ull << (63 - __clzll((long long)chi)) : 0;
+        const uint64_t al = chi ? 0 : 1ull << (63 - __clzll((long long)clo));
+        const uint8_t *nid = B.ids[side] + nd.ids_off + I.M1;
+        unsigned long long nlo = 0, nhi = 0;
+        for (int c = 0; c < I.nv; c++) {
+            const int id = (int)nid[c] - I.nv;
+            if (id >= 0 && id < I.m) { if (id < 64) nlo |= 1ull << id; else nhi |= 1ull << (id - 64); }
+        }
+        uint64_t blo = nlo & ~nd.lo, bhi = nhi & ~nd.hi;
+        while (blo | bhi) {
+            constexpr int G = 4;
+            uint64_t lo[G], hi[G], fp[G];
+            long long at[G];
+            unsigned long long w[G];
+#pragma unroll
+            for (int g = 0; g < G; g++) {
+                const uint64_t bl = blo & (0 - blo), bh = blo ? 0 : bhi & (0 - bhi);
+                blo &= ~bl; bhi &= ~bh;
+                lo[g] = (nd.lo & ~al) | bl; hi[g] = (nd.hi & ~ah) | bh;
+                fp[g] = hash_key(nd.inst, lo[g], hi[g]);
+                at[g] = bl | bh ? (long long)(fp[g] & (uint64_t)(hcap - 1)) : -1;
+            }
+#pragma unroll
+            for (int g = 0; g < G; g++) w[g] = at[g] >= 0 ? tab[at[g]].w : 0;
+#pragma unroll
+            for (int g = 0; g < G; g++) {
+                if (at[g] >= 0 && w[g] != ((tag << 40) | (fp[g] >> 24)))
+                    at[g] = (w[g] >> 40) == tag
+                                ? hash_find_from(tab, hcap, tag, fp[g], (uint64_t)(at[g] + 1) & (uint64_t)(hcap - 1))
+                                : -1;
+                if (at[g] >= B.cover_cap) at[g] = -1;
+            }
+            CoverSlot v[G];
+#pragma unroll
+            for (int g = 0; g < G; g++) v[g] = at[g] >= 0 ? B.cover[side][at[g]] : CoverSlot{0, 0, ~0ull, ~0ull};
+#pragma unroll
+            for (int g = 0; g < G; g++) {
+                if (at[g] < 0 || v[g].slo != lo[g] || v[g].shi != (hi[g] | (unsigned long long)nd.inst << 48)) continue;
+                CoverSlot *c = B.cover[side] + at[g];
+                if (nlo & ~v[g].mlo) atomicOr(&c->mlo, nlo);
+                if (nhi & ~v[g].mhi) atomicOr(&c->mhi, nhi);
+            }
+        }
+    }
+}
+
 // ---------------------------------------------------------------------
 // helpers for K2
 // ---------------------------------------------------------------------
@@ -1179,16 +1272,20 @@ __device__ __forceinline__ void warp_copy_v(T *dst, const T *src, int n)
     for (int e = lane_id(); e < n4; e += 32) d4[e] = s4[e];
 }
 
-// A feasible set into the level's hash, with its vertex mask where its children
-// are the instance's last level (zero elsewhere: every slot of a run has one of
-// that run, so a set found by a fingerprint collision brings a mask that is
-// sound for what it says).
+// A feasible set into the level's hash, with its cover slot (mlo, mhi: the
+// constraints nonbasic at its certified vertex, 0 without one).
 __device__ __forceinline__ void insert_node(const DevBuffers &B, int side, int level, const InstDesc &I, int inst,
-                                            uint64_t lo, uint64_t hi, long long hcap, VertexMask vm)
+                                            uint64_t lo, uint64_t hi, long long hcap, unsigned long long mlo,
+                                            unsigned long long mhi)
 {
     const long long s = hash_insert(B.hash[side], hcap, hash_tag(B.ctl->epoch, level), inst, lo, hi);
-    if (s < 0) atomicOr(&B.ctl->overflow, OV_HASH);
-    else if (B.vmask[side]) B.vmask[side][s] = level + 1 == I.k_max ? vm : VertexMask{0, 0};
+    if (s < 0) {
+        atomicOr(&B.ctl->overflow, OV_HASH);
+    } else if (B.cover[side] && s < B.cover_cap) {
+        // (a set that has none overwrites what an earlier run left there)
+        B.cover[side][s] = covers(I, inst, level) ? CoverSlot{mlo, mhi, lo, hi | (unsigned long long)inst << 48}
+                                                  : CoverSlot{0, 0, ~0ull, ~0ull};
+    }
 }
 
 // Append a feasible (or, exhaustive, any) candidate as a node of `side`;
@@ -1252,7 +1349,7 @@ __device__ long long store_node(const DevBuffers &B, int side, int level, const 
             nd.flags = NODE_VALID | (feasible ? NODE_FEASIBLE : 0) | (extra_flags & ~NODE_CERT);
             nd.tab_off = -1; nd.ids_off = -1; nd.rec = rec;
             B.node[side][idx] = nd;
-            if (feasible && !B.exhaustive && !chunked) insert_node(B, side, level, I, inst, lo, hi, hcap, VertexMask{0, 0});
+            if (feasible && !B.exhaustive && !chunked) insert_node(B, side, level, I, inst, lo, hi, hcap, 0, 0);
         }
         return idx;
     }
@@ -1295,7 +1392,7 @@ __device__ long long store_node(const DevBuffers &B, int side, int level, const 
         B.node[side][idx] = nd;
         // the hash serves the subset test of the next level only
         if (feasible && !B.exhaustive && need_tab && !chunked)
-            insert_node(B, side, level, I, inst, lo, hi, hcap, VertexMask{0, 0});
+            insert_node(B, side, level, I, inst, lo, hi, hcap, 0, 0);
     }
     return idx;
 }
@@ -1468,7 +1565,7 @@ __device__ __forceinline__ void feasibility_body(const DevBuffers &B, const Tol 
     uint8_t *ids = base + align16((((size_t)(sd.maxM1 + 1) * mld + 3) & ~(size_t)3) * sizeof(T));
     uint64_t *bar = (uint64_t *)(base + slot - 16);
     long long *room = (long long *)(base + slot - 16) - kChunkOffsets;
-    VertexMask *vms = (VertexMask *)room - 32;
+    unsigned long long *vms = (unsigned long long *)room - 64;   // per candidate: its vertex's constraints
     const int side = level & 1, pside = side ^ 1;
     Ctl *ctl = B.ctl;
     const long long ncand = ctl->n_cand;
@@ -1828,14 +1925,13 @@ __device__ __forceinline__ void feasibility_body(const DevBuffers &B, const Tol 
             if (level < I.k_max) {
                 lc.d += room[t] >= 0;
                 if (feasible && !B.exhaustive) stored |= 1u << t;
-                if (B.vmask[side] && level + 1 == I.k_max) {
+                if (B.cover[side] && covers(I, inst, level)) {
                     // the constraints nonbasic at this certified vertex
-                    unsigned nb[4];
-                    nonbasic_mask(nid, nv, I.m, nb);
-                    const bool fits = feasible && I.m <= kVertexMaxM && inst < kVertexMaxInst;
+                    unsigned nb[4] = {0, 0, 0, 0};
+                    if (feasible) nonbasic_mask(nid, nv, I.m, nb);
                     if (lane == 0) {
-                        vms[t].lo = fits ? nb[0] | (unsigned long long)nb[1] << 32 : 0ull;
-                        vms[t].hi = fits ? nb[2] | (unsigned long long)nb[3] << 32 | (unsigned long long)inst << 48 : 0ull;
+                        vms[2 * t] = nb[0] | (unsigned long long)nb[1] << 32;
+                        vms[2 * t + 1] = nb[2] | (unsigned long long)nb[3] << 32;
                     }
                 }
             }
@@ -1855,7 +1951,7 @@ __device__ __forceinline__ void feasibility_body(const DevBuffers &B, const Tol 
         __syncwarp();
         if (((stored >> lane) & 1u) && nbase + lane < B.node_cap) {
             const Node nd = B.node[side][nbase + lane];
-            insert_node(B, side, level, B.inst[nd.inst], nd.inst, nd.lo, nd.hi, hcap, vms[lane]);
+            insert_node(B, side, level, B.inst[nd.inst], nd.inst, nd.lo, nd.hi, hcap, vms[2 * lane], vms[2 * lane + 1]);
         }
         __syncwarp();
     }
@@ -5001,7 +5097,7 @@ __global__ void k_level0(DevBuffers B)
         nd.rec = (B.rec && inst < B.rec_cap) ? inst : -1;
         B.node[0][inst] = nd;
         if (!B.exhaustive) {
-            insert_node(B, 0, 0, I, inst, 0, 0, hash_cap_for(B, B.n_inst), VertexMask{0, 0});
+            insert_node(B, 0, 0, I, inst, 0, 0, hash_cap_for(B, B.n_inst), 0, 0);
         }
         if (nd.rec >= 0) {
             CandRec &R = B.rec[nd.rec];
@@ -5250,6 +5346,7 @@ const void *kernel_ptr(const char *name)
     struct E { const char *n; const void *f; };
     static const E tab[] = {
         {"enumerate", (const void *)k_enumerate},
+        {"cover", (const void *)k_cover},
         {"feas64", (const void *)k_feasibility_f64},
         {"feas32", (const void *)k_feasibility_f32},
         {"lp1_fp64", (const void *)k_lp1_fp64},
@@ -5285,6 +5382,12 @@ const void *kernel_ptr(const char *name)
 cudaError_t launch_enumerate(const DevBuffers &B, int level, int grid, cudaStream_t s)
 {
     k_enumerate<<<grid, 128, 0, s>>>(B, level);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_cover(const DevBuffers &B, int level, int grid, cudaStream_t s)
+{
+    k_cover<<<grid, 128, 0, s>>>(B, level);
     return cudaGetLastError();
 }
 
