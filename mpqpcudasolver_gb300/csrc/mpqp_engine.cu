@@ -39,6 +39,8 @@ bool screen_lanes_route(int mode, const InstDesc &I, const SlotDims &sd);
 size_t laws_smem_per_warp(const SlotDims &sd);
 const void *kernel_ptr(const char *name);
 cudaError_t launch_enumerate(const DevBuffers &B, int level, int grid, cudaStream_t s);
+cudaError_t launch_order(const DevBuffers &B, cudaStream_t s);
+cudaError_t launch_scatter(const DevBuffers &B, int level, int grid, cudaStream_t s);
 cudaError_t launch_cover(const DevBuffers &B, int level, int grid, cudaStream_t s);
 cudaError_t launch_feasibility(const DevBuffers &B, const Tol &tol, const SlotDims &sd, int level, int prec,
                                int grid, size_t smem, cudaStream_t s, int warps, int chunk);
@@ -413,6 +415,8 @@ struct mpqp_plan {
     size_t smem_lanes = 0;
     std::vector<char> last_after;   // per level: the next one is some instance's last
     int grid_cover = 0;
+    std::vector<char> ordered;  // per level: candidates brought into their instances' order
+    int grid_scatter = 0;
     std::vector<double> lvl_sets;   // per level, an upper bound on the batch's sets (combinatorial, budgets)
     int grid_direct = 0;        // k_optimality<double> over a whole small level (mixed precision)
     int lane_cap = 3;           // pivots of its first pass (MPQP_SCREEN_CAP)
@@ -661,6 +665,16 @@ constexpr double kDirectWaves = 3.0, kOnePassWaves = 4.0;
 // (95,284) 1,191 / 1,169, m = 48 to 4 (194,580) 1,314 / 1,264
 constexpr double kCoverMin = 100000.0;
 
+// sets of a level from which its candidates are brought into their instances'
+// order (k_order, k_scatter: about 15 us), in a batch of different shapes, and the
+// largest share of one instance.  Enumeration without / with it, mixed and FP64:
+// 16 instances to |S| = 2 (26,900 sets) 0.990 / 1.012 and 2.13 / 2.14 ms; 32 to 2
+// (48,400) 1.41 / 1.41 and 3.24 / 3.07; 8 to 3 (220,000) 2.60 / 2.45 and 12.5 /
+// 10.8; 32 to 3 (870,000) 9.49 / 7.86 and 44.0 / 39.4; 128 small ones to full depth
+// 36.9 / 35.5 and 122.8 / 97.0 ms.  Past the share one instance is most of the
+// level anyway: |S| = 6 of the m = 62 batch (0.79)
+constexpr double kOrderMin = 40000.0, kOrderShare = 0.75;
+
 // The fixed launch sequence of one enumeration.  events: none; one before every
 // launch (and one after the last), for the per-kernel times; or one wherever
 // the sequence changes between its LP1 and its optimality phase (phase_times).
@@ -787,7 +801,15 @@ static int enqueue(mpqp_plan *P, cudaStream_t s, EventMode events)
     { const int _o = launch_optfb(0); if (_o) return _o; }
     L("k_finalize", launch_finalize(B, 0, s));
     for (int k = 1; k <= P->kmax; k++) {
-        L("k_enumerate", launch_enumerate(B, k, grid(P->grid_enum, k - 1, 4), s));
+        if (P->ordered[k]) {
+            DevBuffers raw = B;
+            raw.cand = B.cand_raw;
+            L("k_enumerate", launch_enumerate(raw, k, grid(P->grid_enum, k - 1, 4), s));
+            L("k_order", launch_order(B, s));
+            L("k_scatter", launch_scatter(B, k, grid(P->grid_scatter, k, 1024), s));
+        } else {
+            L("k_enumerate", launch_enumerate(B, k, grid(P->grid_enum, k - 1, 4), s));
+        }
         L(feas, launch_feasibility(B, P->tol, P->sd, k, P->prec, grid(P->grid_feas, k, P->feas_warps), P->smem_feas, s,
                                    P->feas_warps, P->feas_chunk));
         if (mixed) {
@@ -941,20 +963,27 @@ static int plan_create_locked(int n_inst, const mpqp_problem *probs, const mpqp_
     // combinatorial ceilings: at most C(m, k) candidates / nodes at level k
     double lvl_max = 0, arena_max = 0;
     {
-        std::vector<double> lvl(kMaxK + 2, 0.0), lvl_tab(kMaxK + 2, 0.0);
+        std::vector<double> lvl(kMaxK + 2, 0.0), lvl_tab(kMaxK + 2, 0.0), lvl_top(kMaxK + 2, 0.0);
+        bool mixed_shapes = false;
         for (int i = 0; i < n_inst; i++) {
             // an instance with a budget writes at most that many candidates
             // (and nodes) at any level: a level is enumerated only while it fits
             const double cap_i = P->desc[i].budget > 0 ? (double)P->desc[i].budget : 1e300;
             double cmk = 1.0;
+            mixed_shapes |= P->desc[i].M1 != P->desc[0].M1 || P->desc[i].nv != P->desc[0].nv;
             for (int k = 0; k <= P->desc[i].k_max; k++) {
                 if (k > 0) cmk = cmk * (double)(P->desc[i].m - k + 1) / (double)k;
                 const double nk = std::min(cmk, cap_i);
                 lvl[k] += nk;
+                lvl_top[k] = std::max(lvl_top[k], nk);
                 if (k < P->desc[i].k_max) lvl_tab[k] += nk * (double)P->desc[i].tab_elems * (double)es;
             }
         }
         P->lvl_sets = lvl;
+        P->ordered.assign(lvl.size(), 0);
+        if (mixed_shapes && !o.record && !o.exhaustive)
+            for (size_t k = 1; k < lvl.size(); k++)
+                P->ordered[k] = lvl[k] >= kOrderMin && lvl_top[k] <= kOrderShare * lvl[k];
         P->last_after.assign(lvl.size(), 0);
         for (const InstDesc &d : P->desc) if (d.k_max > 1) P->last_after[d.k_max - 1] = 1;
         for (int k = 0; k <= kMaxK; k++) {
@@ -984,9 +1013,10 @@ static int plan_create_locked(int n_inst, const mpqp_problem *probs, const mpqp_
         cover_cap = hash_cap;
         while (cover_cap >= 1024 && 2.0 * (double)cover_cap * sizeof(CoverSlot) > kCoverShare * usable) cover_cap >>= 1;
     }
+    const bool ordered = std::count(P->ordered.begin(), P->ordered.end(), 1) > 0;
     long long arena_bytes = o.arena_bytes;
     if (arena_bytes <= 0) {
-        const double used = 2.0 * (double)cover_cap * sizeof(CoverSlot) + (double)cand_cap * 12 + (double)node_cap * (2 * sizeof(Node) + 4) +
+        const double used = 2.0 * (double)cover_cap * sizeof(CoverSlot) + (double)cand_cap * (ordered ? 20 : 12) + (double)node_cap * (2 * sizeof(Node) + 4) +
                             (double)hash_cap * 2 * sizeof(HashSlot) +
                             (P->prec == PREC_MIXED ? (double)cand_cap / 8 * 48 + (double)cand_cap : 0.0) +  // certificate and rerun queues
                             (o.lp2_warm && P->prec == PREC_MIXED ? 16.0 * (double)node_cap : 0.0);   // LP2 bases
@@ -1057,6 +1087,7 @@ static int plan_create_locked(int n_inst, const mpqp_problem *probs, const mpqp_
         AL(B.cover[1], sizeof(CoverSlot) * cover_cap);
     }
     AL(B.cand, sizeof(Cand) * cand_cap);
+    if (ordered) AL(B.cand_raw, sizeof(Cand) * cand_cap);
     AL(B.q_lp1, sizeof(int) * cand_cap);
     AL(B.q_opt, sizeof(int) * cand_cap);
     B.q_s0_cap = P->prec == PREC_MIXED ? std::max(cand_cap / 4, (long long)4096) : 0;
@@ -1123,6 +1154,7 @@ static int plan_create_locked(int n_inst, const mpqp_problem *probs, const mpqp_
         (rc = grid_for(kernel_ptr(P->prec == PREC_MIXED ? "feas32" : "feas64"), P->smem_feas, &P->grid_feas,
                        32 * P->feas_warps)) ||
         (rc = grid_for(kernel_ptr("cover"), 0, &P->grid_cover)) ||
+        (rc = grid_for(kernel_ptr("scatter"), 0, &P->grid_scatter)) ||
         (rc = grid_for(kernel_ptr("lp1_fp64"), P->smem_lp1fb, &P->grid_lp1fb)) ||
         (rc = grid_for(kernel_ptr("lp1_cert"), P->smem_cert, &P->grid_cert)) ||
         (rc = P->prec == PREC_MIXED

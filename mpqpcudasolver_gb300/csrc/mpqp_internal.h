@@ -179,6 +179,7 @@ struct InstCtl {
     long long s0_lps, s0_piv, warm_try, warm_used;
     // order-independent digests (sum mod 2^64 of a 64-bit hash of each mask)
     unsigned long long feas_digest, opt_digest, reg_digest;
+    long long cursor;           // k_order, k_scatter: the next slot of its ordered candidates
     int stopped;                // budget exhausted or max level reached
     int truncated;              // stopped by the budget
     int last_level;
@@ -193,6 +194,7 @@ constexpr int kLaneMaxK = 6;
 
 struct Ctl {
     long long n_cand;           // candidates at the current level
+    long long n_raw;            // ... in cand_raw
     long long n_node[2];        // nodes per ping-pong side
     long long tab_used[2];      // elements used per tableau arena
     long long ids_used[2];      // bytes used per ids arena
@@ -247,6 +249,7 @@ struct DevBuffers {
     CoverSlot *cover[2];        // parallel to the first cover_cap slots of hash (may be null)
     long long cover_cap;
     Cand *cand;
+    Cand *cand_raw;             // k_enumerate's order, where k_scatter follows (may be null)
     long long cand_cap;
     int *q_lp1;                 // candidate indices for the FP64 LP1 re-solve
     int *q_opt;                 // node indices for the FP64 optimality re-solve
