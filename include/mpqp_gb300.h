@@ -39,7 +39,7 @@ extern "C" {
  *                    are in active_sets, row-major n_final_lps x n_x,
  *                    ascending indices, unused entries -1 (utils.py:105-116)
  *   time_feas        seconds in the enumeration and LP1 kernels (events
- *                    around each launch)
+ *                    where the sequence changes between the two)
  *   time_opti        seconds in the optimality kernels
  *   time_GPU         seconds of device time for the whole call
  * mpqp() runs in mixed precision (FP32 pivots, every verdict certified or
@@ -138,7 +138,8 @@ typedef struct {
     int precision;           /* MPQP_FP64 or MPQP_MIXED                     */
     int exhaustive;          /* 1: every combination is a candidate          */
     int record;              /* 1: keep one record per checked candidate    */
-    int use_graph;           /* 1: capture the level loop in a CUDA graph   */
+    int use_graph;           /* 1: a plan captures its run in a CUDA graph  */
+                             /* (mpqp_solve_batch runs once, without one)   */
     long long cand_cap;      /* candidates per level (0: derived)           */
     long long node_cap;      /* nodes per level (0: = cand_cap)             */
     long long arena_bytes;   /* tableau arena (0: derived)                  */
@@ -226,7 +227,8 @@ typedef struct {
      * and those that started from it */
     long long lp2_first_stage_lps, lp2_first_stage_pivots, lp2_warm_offered, lp2_warm_started;
     /* mixed precision: sets found not optimal in FP64 from the final basis
-     * of the FP32 dual screen, without the FP64 LP2 (counted in fallback_opt) */
+     * of the FP32 dual screen, without the FP64 LP2 (counted in fallback_opt,
+     * like the sets of levels small enough to be evaluated in FP64 at once) */
     long long lp2_certified;
     /* mixed precision: last-level FP32 LP1 optima whose smallest basic slack
      * lay inside the FP32 margin, found feasible by the FP64 vertex check of

@@ -1041,9 +1041,10 @@ __global__ void k_enumerate(DevBuffers B, int level)
                 // vertex at which all of the candidate's slacks are nonbasic.
                 // Each subset's vertex has the missing element with a chance of
                 // about one in five, so three quarters of the candidates are
-                // settled here: m = 62 batch (48M last-level candidates) LP1 167
-                // -> 101 ms for 5 ms more in this kernel, 64 MPC problems 3.47 ->
-                // 2.15 ms, m = 62 to |S| = 4 1.70 -> 1.14 ms
+                // settled here, more with k_cover: m = 62 batch (48M last-level
+                // candidates) LP1 167 -> 101 -> 87 ms for 5 ms more in this kernel,
+                // 64 MPC problems 3.47 -> 2.15 -> 1.94 ms, m = 62 to |S| = 4 1.70 ->
+                // 1.14 -> 0.93 ms
                 const CoverSlot *ctab = B.cover[pside];
                 const bool want = ctab && level == B.inst[cinst].k_max;
                 uint64_t lo = clo0, hi = chi0;
@@ -1267,7 +1268,8 @@ __device__ __forceinline__ bool covers(const InstDesc &I, int inst, int level)
 
 // elements a of S that k_cover replaces (the largest).  With 0, 1, 2, 3 and all
 // of them the m = 62 batch's LP1 takes 102.7, 93.0, 87.6, 84.6 and 81.9 ms, and
-// k_cover 0, 2.0, 5.4, 9.0 and 16.4 ms (before its loads were grouped, 4.7 with).
+// k_cover 0, 2.0, 5.4, 9.0 and 16.4 ms (before its loads were grouped, 4.7 with,
+// and before the candidates came by instance: LP1 58.7 and k_cover 3.6 ms with 2).
 constexpr int kCoverSpread = 2;
 
 // Spreads the certified vertices of a level whose children are last-level
