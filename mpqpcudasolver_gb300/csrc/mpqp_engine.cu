@@ -1081,13 +1081,7 @@ static int plan_create_locked(int n_inst, const mpqp_problem *probs, const mpqp_
     B.ids[1] = B.ids[0];
     AL(B.hash[0], sizeof(HashSlot) * hash_cap);
     AL(B.hash[1], sizeof(HashSlot) * hash_cap);
-    B.cover_cap = cover_cap;
-    if (cover_cap) {
-        AL(B.cover[0], sizeof(CoverSlot) * cover_cap);
-        AL(B.cover[1], sizeof(CoverSlot) * cover_cap);
-    }
     AL(B.cand, sizeof(Cand) * cand_cap);
-    if (ordered) AL(B.cand_raw, sizeof(Cand) * cand_cap);
     AL(B.q_lp1, sizeof(int) * cand_cap);
     AL(B.q_opt, sizeof(int) * cand_cap);
     B.q_s0_cap = P->prec == PREC_MIXED ? std::max(cand_cap / 4, (long long)4096) : 0;
@@ -1108,6 +1102,22 @@ static int plan_create_locked(int n_inst, const mpqp_problem *probs, const mpqp_
         AL(B.lp2b[1], sizeof(unsigned long long) * node_cap);
     }
 #undef AL
+    // what only saves time comes last: a plan with an arena size of the caller's
+    // that leaves no room for it does without
+    if (cover_cap) {
+        void *c0 = nullptr, *c1 = nullptr;
+        const size_t bytes = sizeof(CoverSlot) * cover_cap;
+        if (dev_alloc(P, &c0, bytes) == MPQP_OK && dev_alloc(P, &c1, bytes) == MPQP_OK) {
+            B.cover[0] = (CoverSlot *)c0;
+            B.cover[1] = (CoverSlot *)c1;
+            B.cover_cap = cover_cap;
+        }
+    }
+    if (ordered) {
+        void *raw = nullptr;
+        if (dev_alloc(P, &raw, sizeof(Cand) * cand_cap) == MPQP_OK) B.cand_raw = (Cand *)raw;
+        else P->ordered.assign(P->ordered.size(), 0);
+    }
     CK(cudaStreamSynchronize(0));   // the pool's allocations are stream-ordered on stream 0
     if (in_bytes <= kOneUpload) {
         std::vector<unsigned char> img(in_bytes);
