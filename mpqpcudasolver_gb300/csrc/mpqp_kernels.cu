@@ -4359,15 +4359,17 @@ __global__ void __launch_bounds__(32) k_opt_screen_lanes(DevBuffers B, Tol tol, 
     // the lanes' counts to their instances, the lanes of one instance in one
     // addition (an addition per lane queued 200,000 of them on the counters of
     // the last instance as the kernel ended: n = 10, m = 43 to |S| = 4 207 -> 113
-    // us, m = 62 to |S| = 4 796 -> 545 us, all passes)
+    // us, m = 62 to |S| = 4 796 -> 545 us, all passes).  By the whole warp, at
+    // points that all of its lanes reach.
     auto flush = [&]() {
-        const unsigned grp = __match_any_sync(__activemask(), lc.inst);
+        const unsigned grp = __match_any_sync(FULLMASK, lc.inst);
         const unsigned piv = __reduce_add_sync(grp, (unsigned)lc.c), lps = __reduce_add_sync(grp, (unsigned)lc.d);
         if (lc.inst >= 0 && lane == __ffs(grp) - 1) {
             atomicAdd((unsigned long long *)&B.ictl[lc.inst].lp2_piv, (unsigned long long)piv);
             atomicAdd((unsigned long long *)&B.ictl[lc.inst].s0_lps, (unsigned long long)lps);
             atomicAdd((unsigned long long *)&B.ictl[lc.inst].s0_piv, (unsigned long long)piv);
         }
+        lc.reset(lc.inst);
     };
     const int max_it = cap > 0 ? cap : tol.max_pivots;
     for (;;) {
@@ -4375,14 +4377,16 @@ __global__ void __launch_bounds__(32) k_opt_screen_lanes(DevBuffers B, Tol tol, 
         if (lane == 0) x0 = (long long)atomicAdd(&ctl->ctr[pass == 0 ? 3 : (pass == 1 ? 9 : 11)], 32ull);
         x0 = __shfl_sync(FULLMASK, x0, 0);
         if (x0 >= nn) break;
-        if (x0 + lane >= nn) continue;
-        const long long x = pass == 0 ? x0 + lane : (long long)(pass == 1 ? B.q_s0 : B.q_s1)[x0 + lane];
+        // (a lane past the end looks at the last item and takes nothing)
+        const long long xi = x0 + lane < nn ? x0 + lane : nn - 1;
+        const long long x = pass == 0 ? xi : (long long)(pass == 1 ? B.q_s0 : B.q_s1)[xi];
         const Node nd = B.node[side][x];
-        if ((nd.flags & (NODE_VALID | NODE_FEASIBLE)) != (NODE_VALID | NODE_FEASIBLE)) continue;
         const InstDesc &I = B.inst[nd.inst];
-        if (level < I.k_min) continue;
-        if (!lanes_route(mode, I, sd)) continue;
-        if (nd.inst != lc.inst) { flush(); lc.reset(nd.inst); }
+        const bool take = x0 + lane < nn && (nd.flags & (NODE_VALID | NODE_FEASIBLE)) == (NODE_VALID | NODE_FEASIBLE) &&
+                          level >= I.k_min && lanes_route(mode, I, sd);
+        if (__any_sync(FULLMASK, take && lc.inst >= 0 && nd.inst != lc.inst)) flush();
+        if (!take) continue;
+        if (nd.inst != lc.inst) lc.reset(nd.inst);
         const KktData<float> D = multiplier_data(B, I);
         const int m = I.m, p = I.p, ncp = I.ncp, P1 = p + 1;
         const float *WhX = D.Wh, *wcX = D.wc;
