@@ -27,8 +27,7 @@
 namespace mq {
 size_t lp1_smem_per_warp(int prec_bytes, const SlotDims &sd);
 size_t feas_smem_per_warp(int prec_bytes, const SlotDims &sd);
-size_t opt_smem_per_warp(int prec_bytes, const SlotDims &sd);
-size_t opt_fb_smem_per_warp(const SlotDims &sd);
+size_t opt_smem_per_warp(const SlotDims &sd, bool group);
 size_t screen_smem_per_warp(const SlotDims &sd, int route);
 size_t screen_tiles_smem(const SlotDims &sd, int tile_w);
 size_t screen_lanes_smem();
@@ -49,7 +48,7 @@ cudaError_t launch_lp1_fp64(const DevBuffers &B, const Tol &tol, const SlotDims 
 cudaError_t launch_lp1_cert(const DevBuffers &B, const Tol &tol, const SlotDims &sd, int level, int grid,
                             size_t smem, cudaStream_t s);
 size_t cert_smem_per_warp(const SlotDims &sd);
-cudaError_t launch_optimality(const DevBuffers &B, const Tol &tol, const SlotDims &sd, int level, bool lp,
+cudaError_t launch_optimality(const DevBuffers &B, const Tol &tol, const SlotDims &sd, int level, bool lp, bool group,
                               int grid, size_t smem, cudaStream_t s);
 cudaError_t launch_opt_screen(const DevBuffers &B, const Tol &tol, const SlotDims &sd, int level, int mode, int route,
                               int grid, size_t smem, cudaStream_t s, int tile_w);
@@ -419,6 +418,7 @@ struct mpqp_plan {
     int grid_scatter = 0;
     std::vector<double> lvl_sets;   // per level, an upper bound on the batch's sets (combinatorial, budgets)
     int grid_direct = 0;        // k_optimality<double> over a whole small level (mixed precision)
+    bool opt_group = false;     // ... and in FP64: its slots have room for the KKT factors of a group of sets
     int lane_cap = 3;           // pivots of its first pass (MPQP_SCREEN_CAP)
     int lane_cap2 = 6;          // ... of its second (MPQP_SCREEN_CAP2; 0: uncapped, no third pass)
     // launch settings the autotuner chooses: threads per set in the screen's
@@ -675,6 +675,36 @@ constexpr double kCoverMin = 100000.0;
 // level anyway: |S| = 6 of the m = 62 batch (0.79)
 constexpr double kOrderMin = 40000.0, kOrderShare = 0.75;
 
+// The most dynamic shared memory a block of the kernels without static shared
+// memory can have (227 KB).
+static size_t block_smem_limit()
+{
+    int dev = 0, bytes = 0;
+    cudaGetDevice(&dev);
+    if (cudaDeviceGetAttribute(&bytes, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) { cudaGetLastError(); return 0; }
+    return (size_t)bytes;
+}
+
+// Whether k_optimality's slots get room for the KKT factors of a group of sets:
+// where the block then fits on an SM, and not where an SM would hold one block
+// instead of two.  Optimality kernel with / without the group, blocks per SM,
+// FP64: n = 8, m = 40, p = 4 (84K sets) 1,461 / 1,846 us, 4 / 4; n = 12, m = 62,
+// p = 6 (40K) 1,856 / 1,811, 3 / 4; n = 14, m = 70, p = 8 (57K) 4,915 / 5,002, 2 /
+// 3; n = 16, m = 112, p = 8 (234K) 30.4 / 19.1 ms, 1 / 2; n = 16, m = 128, p = 8
+// (350K) 72.9 / 46.5 ms, 1 / 2; n = 16, m = 128, p = 10 (350K) 108.5 / 109.9, 1 / 1
+static int group_room(const SlotDims &sd, bool *group)
+{
+    const size_t with = 4 * opt_smem_per_warp(sd, true), without = 4 * opt_smem_per_warp(sd, false);
+    *group = false;
+    if (with > block_smem_limit()) return MPQP_OK;
+    int g1 = 0, g0 = 0, dev = 0, sms = 0, rc;
+    if ((rc = grid_for(kernel_ptr("opt64"), with, &g1)) || (rc = grid_for(kernel_ptr("opt64"), without, &g0))) return rc;
+    CK(cudaGetDevice(&dev));
+    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    *group = g1 == g0 || g1 >= 2 * sms;
+    return MPQP_OK;
+}
+
 // The fixed launch sequence of one enumeration.  events: none; one before every
 // launch (and one after the last), for the per-kernel times; or one wherever
 // the sequence changes between its LP1 and its optimality phase (phase_times).
@@ -732,16 +762,18 @@ static int enqueue(mpqp_plan *P, cudaStream_t s, EventMode events)
         if (!mixed) {
             if (P->has_qp)
                 L("k_optimality<double>",
-                  launch_optimality(B, P->tol, P->sd, level, false, grid(P->grid_opt, level, 4), P->smem_opt, s));
+                  launch_optimality(B, P->tol, P->sd, level, false, P->opt_group, grid(P->grid_opt, level, 4),
+                                    P->smem_opt, s));
             if (P->has_lp)
                 L("k_optimality<double,mplp>",
-                  launch_optimality(B, P->tol, P->sd, level, true, grid(P->grid_opt_lp, level, 4), P->smem_opt, s));
+                  launch_optimality(B, P->tol, P->sd, level, true, P->opt_group, grid(P->grid_opt_lp, level, 4),
+                                    P->smem_opt, s));
             return MPQP_OK;
         }
         if (direct(level)) {
             L("k_optimality<double>",
-              launch_optimality(B, P->tol, P->sd, level, false, grid(P->grid_direct, level, 4), P->smem_direct,
-                                s));
+              launch_optimality(B, P->tol, P->sd, level, false, P->opt_group, grid(P->grid_direct, level, 4),
+                                P->smem_direct, s));
             return MPQP_OK;
         }
         const bool lanes = level <= kLaneMaxK && !B.lp2b[0] && (P->screen_dual || P->lanes_lp);
@@ -1144,7 +1176,10 @@ static int plan_create_locked(int n_inst, const mpqp_problem *probs, const mpqp_
     P->smem_lp1fb = 4 * lp1_smem_per_warp(8, sd);
     P->smem_cert = 4 * cert_smem_per_warp(sd);
     // mixed precision: the grouped FP32 screen, one warp per block
-    P->smem_opt = P->prec == PREC_MIXED ? screen_smem_per_warp(sd, 0) : 4 * opt_smem_per_warp(8, sd);
+    rc = group_room(sd, &P->opt_group);
+    if (rc) { free_plan_mem(P); delete P; return rc; }
+    const size_t smem_opt64 = 4 * opt_smem_per_warp(sd, P->opt_group);
+    P->smem_opt = P->prec == PREC_MIXED ? screen_smem_per_warp(sd, 0) : smem_opt64;
     P->smem_opt2 = screen_smem_per_warp(sd, 1);
     P->smem_tiles = screen_tiles_smem(sd, P->tile_w);
     P->smem_lanes = screen_lanes_smem();
@@ -1158,8 +1193,8 @@ static int plan_create_locked(int n_inst, const mpqp_problem *probs, const mpqp_
         else if (d.lp && screen_lanes_route(P->lp2_screen, d, sd)) P->lanes_lp = true;
         else P->screen_primal = true;
     }
-    P->smem_optfb = 4 * opt_fb_smem_per_warp(sd);
-    P->smem_direct = 4 * opt_smem_per_warp(8, sd);
+    P->smem_optfb = 4 * opt_smem_per_warp(sd, false);
+    P->smem_direct = smem_opt64;
     if ((rc = grid_for(kernel_ptr("enumerate"), 0, &P->grid_enum)) ||
         (rc = grid_for(kernel_ptr(P->prec == PREC_MIXED ? "feas32" : "feas64"), P->smem_feas, &P->grid_feas,
                        32 * P->feas_warps)) ||

@@ -3316,11 +3316,11 @@ __device__ void write_opt(const DevBuffers &B, const Node &nd, int level, const 
 // instances, LP = true those of mpLP instances (launched only when a batch
 // has one), so that the mpQP kernel carries no mpLP code.
 template <typename T, bool LP>
-__global__ void __launch_bounds__(128, kF64Blocks) k_optimality(DevBuffers B, Tol tol, SlotDims sd, int level)
+__global__ void __launch_bounds__(128, kF64Blocks) k_optimality(DevBuffers B, Tol tol, SlotDims sd, int level, bool group_room)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     const int lane = lane_id(), wib = threadIdx.x >> 5;
-    const size_t slot = opt_slot_bytes<T>(sd, true);
+    const size_t slot = opt_slot_bytes<T>(sd, group_room);
     OptWs<T> ws(smem + wib * slot, sd);
     const int side = level & 1;
     Ctl *ctl = B.ctl;
@@ -3338,8 +3338,9 @@ __global__ void __launch_bounds__(128, kF64Blocks) k_optimality(DevBuffers B, To
         if (B.precision == PREC_MIXED) atomicAdd((unsigned long long *)&ic->fb_opt, (unsigned long long)lc.e);
     };
     // sets of a level have k = level elements; their KKT factors are computed
-    // a group at a time (single sets where the level cannot fill the warps)
-    const bool grouped = level <= kGroupK;
+    // a group at a time (single sets where the level cannot fill the warps),
+    // where the slot has room for them
+    const bool grouped = group_room && level <= kGroupK;
     const int claim = grouped ? claim_size(nn, kGroup) : 1;
     unsigned char *group = smem + wib * slot + opt_slot_bytes<T>(sd);
     auto takes = [&](const Node &nd) {
@@ -5440,13 +5441,8 @@ size_t screen_tiles_smem(const SlotDims &sd, int tile_w) { return (32 / tile_w) 
 bool screen_dual_route(int mode, const InstDesc &I, const SlotDims &sd) { return dual_route(mode, I, sd); }
 bool screen_lanes_route(int mode, const InstDesc &I, const SlotDims &sd) { return lanes_route(mode, I, sd); }
 
-// k_optimality_fp64 (k_optimality's slot has the group's factors besides)
-size_t opt_fb_smem_per_warp(const SlotDims &sd) { return opt_slot_bytes<double>(sd); }
-
-size_t opt_smem_per_warp(int prec_bytes, const SlotDims &sd)
-{
-    return prec_bytes == 8 ? opt_slot_bytes<double>(sd, true) : opt_slot_bytes<float>(sd);
-}
+// k_optimality (group: with the factors of a group of sets) and k_optimality_fp64 (without)
+size_t opt_smem_per_warp(const SlotDims &sd, bool group) { return opt_slot_bytes<double>(sd, group); }
 
 }  // namespace mq
 
@@ -5544,12 +5540,12 @@ cudaError_t launch_lp1_cert(const DevBuffers &B, const Tol &tol, const SlotDims 
     return cudaGetLastError();
 }
 
-cudaError_t launch_optimality(const DevBuffers &B, const Tol &tol, const SlotDims &sd, int level, bool lp,
+cudaError_t launch_optimality(const DevBuffers &B, const Tol &tol, const SlotDims &sd, int level, bool lp, bool group,
                               int grid, size_t smem, cudaStream_t s)
 {
     // the FP32 screen of the mixed path is launch_opt_screen
-    if (lp) k_optimality<double, true><<<grid, 128, smem, s>>>(B, tol, sd, level);
-    else k_optimality<double, false><<<grid, 128, smem, s>>>(B, tol, sd, level);
+    if (lp) k_optimality<double, true><<<grid, 128, smem, s>>>(B, tol, sd, level, group);
+    else k_optimality<double, false><<<grid, 128, smem, s>>>(B, tol, sd, level, group);
     return cudaGetLastError();
 }
 

@@ -1,0 +1,52 @@
+"""Instances near the limits of a block's shared memory.
+
+The FP64 optimality kernel factors the KKT systems of four sets at a time when
+its slots have room for them, and one at a time otherwise (or when the room would
+leave an SM one block instead of two): problems on both sides of these limits (with |S| up to n, under a budget that ends the run at |S| =
+2) and of its limit |S| = 8, in both precisions, against the oracle."""
+import numpy as np
+import pytest
+
+from mpqpcudasolver_gb300 import problems as P
+from mpqpcudasolver_gb300 import solver
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+FIELDS = ("mask_lo", "mask_hi", "feasible", "licq", "optimal", "region")
+FP64_FIELDS = FIELDS + ("lp1_status", "lp1_pivots", "z", "lp2_status", "lp2_pivots", "cheb_status", "cheb_pivots")
+
+
+def _key(a):
+    a = a[a["level"] >= 0]
+    return a[np.lexsort([a["mask_lo"], a["mask_hi"]])]
+
+
+def _compare(prob, ref, **kw):
+    want = _key(ref.cand)
+    for precision in (solver.FP64, solver.MIXED):
+        r = solver.solve([prob], precision=precision, record=1, **kw)
+        got = _key(r.rec)
+        assert len(got) == len(want)
+        for f in FP64_FIELDS if precision == solver.FP64 else ("mask_lo", "mask_hi", "feasible", "optimal", "region"):
+            assert np.array_equal(got[f], want[f]), (precision, f)
+        opt = want["optimal"] == 1
+        for f in ("t", "r"):
+            assert np.array_equal(got[f][opt], want[f][opt], equal_nan=True), (precision, f)
+
+
+@pytest.mark.parametrize("make,n,m,p", [(P.random_mpqp, 16, 128, 15), (P.random_mpqp, 16, 128, 16),
+                                        (P.random_mpqp, 12, 80, 21), (P.random_mpqp, 12, 80, 22),
+                                        (P.random_mpqp, 16, 108, 8), (P.random_mpqp, 16, 114, 8),
+                                        (P.random_mplp, 20, 128, 4), (P.random_mplp, 20, 128, 5)])
+def test_both_sides_of_the_group_limit(gpu_lib, make, n, m, p):
+    prob = P.scale_problem(make(n, m, p, seed=m + p))
+    _compare(prob, O.enumerate_sets(prob, k_max=2, nthreads=8), k_max=n, budget=9000, opt_cap=1 << 14)
+
+
+@pytest.mark.parametrize("make,n,m,p", [(P.random_mpqp, 9, 16, 5), (P.random_mplp, 9, 19, 2)])
+def test_group_and_single_factors_by_level(gpu_lib, make, n, m, p):
+    prob = P.scale_problem(make(n, m, p, seed=5))
+    ref = O.enumerate_sets(prob, k_max=n, nthreads=8)
+    assert all(((ref.cand["level"] == k) & (ref.cand["optimal"] == 1)).any() for k in (8, 9))
+    _compare(prob, ref, k_max=n)
