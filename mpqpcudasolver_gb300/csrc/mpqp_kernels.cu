@@ -816,13 +816,16 @@ __host__ __device__ inline size_t lp1_slot_bytes(int maxM1, int maxLD1, int maxN
     return lp1_buf_bytes<T>(maxM1, maxLD1, maxNv) + 16;
 }
 
-// slot of k_feasibility: one buffer, the vertex masks and the arena offsets
-// reserved for the chunk's candidates, and the warp's mbarrier (16 bytes, last)
-constexpr int kChunkOffsets = 2 * 32;
+// slot of k_feasibility: one buffer, in FP32 two words per candidate of the
+// chunk (the arena offsets reserved for it, then its vertex's constraints), and
+// the warp's mbarrier (16 bytes, last).  In FP64, where a buffer can fill a
+// quarter of the SM, the offsets are read from the candidates' node records
+// (LP1 of n = 10, m = 43 to |S| = 4 with the offsets in shared memory / in the
+// records 1,957 / 1,969 us, of 24 small problems 1,547 / 1,586 us).
 template <typename T>
 __host__ __device__ inline size_t feas_slot_bytes(int maxM1, int maxLD1, int maxNv)
 {
-    return lp1_buf_bytes<T>(maxM1, maxLD1, maxNv) + 64 * sizeof(unsigned long long) + kChunkOffsets * sizeof(long long) + 16;
+    return lp1_buf_bytes<T>(maxM1, maxLD1, maxNv) + (sizeof(T) == 4 ? 64 * sizeof(long long) : 0) + 16;
 }
 
 // candidates a warp claims at a time (a plan setting, at most 32, by default
@@ -1399,20 +1402,20 @@ __device__ __forceinline__ void insert_node(const DevBuffers &B, int side, int l
 // TT = TS); lane 0 copies them with bulk stores (bulk_wait_read before the
 // slot is written again, bulk_wait_all before the kernel ends).
 // reserved: the arena space reserved before (reserved[0] the tableau's and
-// reserved[stride] the ids' offset, -1: none).  stride 32: a chunk of
-// k_feasibility, which counts its stores and inserts its sets into the hash
-// itself; stride 1: a candidate's node record.
+// reserved[stride] the ids' offset, -1: none; stride 1: the candidate's node
+// record, whose ids_off follows tab_off).  chunked: k_feasibility, which counts
+// its stores and inserts its sets into the hash itself.
 template <typename TT, typename TS>
 __device__ long long store_node(const DevBuffers &B, int side, int level, const InstDesc &I, int inst,
                                 uint64_t lo, uint64_t hi, bool feasible, const TS *tab, const uint8_t *ids,
                                 long long rec, long long hcap, int extra_flags, int src_ld = 0, bool bulk = false,
                                 long long pre_idx = -1, int rows_store = -1, int cols_store = -1,
-                                const long long *reserved = nullptr, int stride = 0)
+                                const long long *reserved = nullptr, int stride = 0, bool chunked = false)
 {
+    static_assert(offsetof(Node, ids_off) == offsetof(Node, tab_off) + sizeof(long long), "reserved, stride 1");
     const int lane = lane_id();
     Ctl *ctl = B.ctl;
     const bool need_tab = level < I.k_max;
-    const bool chunked = stride == 32;   // the caller counts the store and inserts the set into the hash
     long long idx = 0, toff = -1, ioff = -1;
     if (lane == 0) {
         // one arena per kind, side 0 filled upward from 0, side 1 downward
@@ -1668,8 +1671,7 @@ __device__ __forceinline__ void feasibility_body(const DevBuffers &B, const Tol 
     T *tab = (T *)base;
     uint8_t *ids = base + align16((((size_t)(sd.maxM1 + 1) * mld + 3) & ~(size_t)3) * sizeof(T));
     uint64_t *bar = (uint64_t *)(base + slot - 16);
-    long long *room = (long long *)(base + slot - 16) - kChunkOffsets;
-    unsigned long long *vms = (unsigned long long *)room - 64;   // per candidate: its vertex's constraints
+    long long *room = (long long *)(base + slot - 16) - 64;   // FP32 only
     const int side = level & 1, pside = side ^ 1;
     Ctl *ctl = B.ctl;
     const long long ncand = ctl->n_cand;
@@ -1740,8 +1742,10 @@ __device__ __forceinline__ void feasibility_body(const DevBuffers &B, const Tol 
                     ioff = side == 0 ? iold : B.ids_cap - iold - ib;
                 }
             }
-            room[lane] = toff;
-            room[32 + lane] = ioff;
+            if constexpr (mixed) {
+                room[lane] = toff;
+                room[32 + lane] = ioff;
+            }
             if (lane < cnt && nbase + lane < B.node_cap) {
                 Node gap;
                 gap.lo = 0; gap.hi = 0; gap.inst = 0; gap.flags = 0; gap.tab_off = toff; gap.ids_off = ioff; gap.rec = -1;
@@ -2023,19 +2027,21 @@ __device__ __forceinline__ void feasibility_body(const DevBuffers &B, const Tol 
                     cols = feasible && !B.exhaustive
                                ? retire_fixed_columns(tab, ld, rows, pcols, nid, nv, lo, hi) : pcols;
             }
+            const long long *res = mixed ? room + t
+                                         : nbase + t < B.node_cap ? &B.node[side][nbase + t].tab_off : nullptr;
             store_node<T, T>(B, side, level, I, inst, lo, hi, feasible, tab, ids, rec, hcap,
                              mixed && feasible ? NODE_CERT : 0, 0, true, nbase + t, mixed ? rows : -1,
-                             mixed ? cols : -1, room + t, 32);
+                             mixed ? cols : -1, res, mixed ? 32 : 1, true);
             if (level < I.k_max) {
-                lc.d += room[t] >= 0;
+                lc.d += lane == 0 && res && *res >= 0;
                 if (feasible && !B.exhaustive) stored |= 1u << t;
-                if (B.cover[side] && covers(I, inst, level)) {
-                    // the constraints nonbasic at this certified vertex
+                if constexpr (mixed) {
+                    // the constraints nonbasic at this certified vertex, in place of the offsets
                     unsigned nb[4] = {0, 0, 0, 0};
-                    if (feasible) nonbasic_mask(nid, nv, I.m, nb);
+                    if (feasible && B.cover[side] && covers(I, inst, level)) nonbasic_mask(nid, nv, I.m, nb);
                     if (lane == 0) {
-                        vms[2 * t] = nb[0] | (unsigned long long)nb[1] << 32;
-                        vms[2 * t + 1] = nb[2] | (unsigned long long)nb[3] << 32;
+                        room[t] = (long long)(nb[0] | (unsigned long long)nb[1] << 32);
+                        room[32 + t] = (long long)(nb[2] | (unsigned long long)nb[3] << 32);
                     }
                 }
             }
@@ -2055,7 +2061,8 @@ __device__ __forceinline__ void feasibility_body(const DevBuffers &B, const Tol 
         __syncwarp();
         if (((stored >> lane) & 1u) && nbase + lane < B.node_cap) {
             const Node nd = B.node[side][nbase + lane];
-            insert_node(B, side, level, B.inst[nd.inst], nd.inst, nd.lo, nd.hi, hcap, vms[2 * lane], vms[2 * lane + 1]);
+            insert_node(B, side, level, B.inst[nd.inst], nd.inst, nd.lo, nd.hi, hcap,
+                        mixed ? (unsigned long long)room[lane] : 0, mixed ? (unsigned long long)room[32 + lane] : 0);
         }
         __syncwarp();
     }

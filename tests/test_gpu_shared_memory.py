@@ -3,7 +3,10 @@
 The FP64 optimality kernel factors the KKT systems of four sets at a time when
 its slots have room for them, and one at a time otherwise (or when the room would
 leave an SM one block instead of two): problems on both sides of these limits (with |S| up to n, under a budget that ends the run at |S| =
-2) and of its limit |S| = 8, in both precisions, against the oracle."""
+2) and of its limit |S| = 8, in both precisions, against the oracle.
+
+The LP1 kernel runs four warps a block with a tableau each: problems whose FP64
+tableaus leave less than 4 KB of a block's shared memory."""
 import numpy as np
 import pytest
 
@@ -50,3 +53,9 @@ def test_group_and_single_factors_by_level(gpu_lib, make, n, m, p):
     ref = O.enumerate_sets(prob, k_max=n, nthreads=8)
     assert all(((ref.cand["level"] == k) & (ref.cand["optimal"] == 1)).any() for k in (8, 9))
     _compare(prob, ref, k_max=n)
+
+
+@pytest.mark.parametrize("n,m,p", [(35, 120, 13), (44, 128, 6), (59, 100, 5)])
+def test_largest_lp1_tableaus(gpu_lib, n, m, p):
+    prob = P.scale_problem(P.random_mpqp(n, m, p, seed=m + p))
+    _compare(prob, O.enumerate_sets(prob, k_max=2, nthreads=8), k_max=2, opt_cap=1 << 14)
