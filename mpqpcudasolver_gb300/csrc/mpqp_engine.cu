@@ -37,6 +37,8 @@ bool screen_dual_route(int mode, const InstDesc &I, const SlotDims &sd);
 bool screen_lanes_route(int mode, const InstDesc &I, const SlotDims &sd);
 size_t laws_smem_per_warp(const SlotDims &sd);
 const void *kernel_ptr(const char *name);
+size_t block_smem_limit();
+cudaError_t allow_smem(const void *fn, size_t smem);
 cudaError_t launch_enumerate(const DevBuffers &B, int level, int grid, cudaStream_t s);
 cudaError_t launch_order(const DevBuffers &B, cudaStream_t s);
 cudaError_t launch_scatter(const DevBuffers &B, int level, int grid, cudaStream_t s);
@@ -77,10 +79,12 @@ namespace mq {
 void set_error_text(const char *msg) { set_err(msg ? msg : ""); }
 }  // namespace mq
 
+// (a failed call's error is not left for the next launch to report)
 #define CK(call)                                                                                       \
     do {                                                                                               \
         cudaError_t _e = (call);                                                                       \
         if (_e != cudaSuccess) {                                                                       \
+            cudaGetLastError();                                                                        \
             set_err(std::string(#call) + ": " + cudaGetErrorString(_e));                               \
             return MPQP_ECUDA;                                                                         \
         }                                                                                              \
@@ -613,30 +617,20 @@ static void free_plan_mem(mpqp_plan *P)
 
 // Blocks of a persistent grid (SMs x resident blocks).  The answer depends on
 // the kernel, the block and the shared memory alone, so it is asked once per
-// device (a plan asks for a dozen).  A kernel's shared-memory limit only grows:
-// an earlier plan of larger instances may still run.
+// device (a plan asks for a dozen).
 static int grid_for(const void *fn, size_t smem, int *grid, int block = 128)
 {
-    struct Limit { int dev; const void *fn; size_t smem; };
     struct Known { int dev; const void *fn; size_t smem; int block, grid; };
     static std::mutex mu;
-    static std::vector<Limit> limits;   // one entry per device and kernel
     static std::vector<Known> known;    // bounded
     int dev = 0, sms = 0, nb = 0;
     CK(cudaGetDevice(&dev));
-    std::lock_guard<std::mutex> lk(mu);
-    if (smem > 48 * 1024) {
-        Limit *lim = nullptr;
-        for (Limit &l : limits) if (l.dev == dev && l.fn == fn) lim = &l;
-        if (!lim) { limits.push_back(Limit{dev, fn, smem}); lim = &limits.back(); }
-        lim->smem = std::max(lim->smem, smem);
-        const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lim->smem);
-        if (e != cudaSuccess) {
-            lim->smem = 0;
-            set_err(std::string("kernel shared memory limit: ") + cudaGetErrorString(e));
-            return MPQP_ECUDA;
-        }
+    const cudaError_t e = allow_smem(fn, smem);
+    if (e != cudaSuccess) {
+        set_err("kernel shared memory limit (" + std::to_string(smem) + " bytes): " + cudaGetErrorString(e));
+        return MPQP_ECUDA;
     }
+    std::lock_guard<std::mutex> lk(mu);
     for (const Known &k : known)
         if (k.dev == dev && k.fn == fn && k.smem == smem && k.block == block) { *grid = k.grid; return MPQP_OK; }
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -674,16 +668,6 @@ constexpr double kCoverMin = 100000.0;
 // 36.9 / 35.5 and 122.8 / 97.0 ms.  Past the share one instance is most of the
 // level anyway: |S| = 6 of the m = 62 batch (0.79)
 constexpr double kOrderMin = 40000.0, kOrderShare = 0.75;
-
-// The most dynamic shared memory a block of the kernels without static shared
-// memory can have (227 KB).
-static size_t block_smem_limit()
-{
-    int dev = 0, bytes = 0;
-    cudaGetDevice(&dev);
-    if (cudaDeviceGetAttribute(&bytes, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) { cudaGetLastError(); return 0; }
-    return (size_t)bytes;
-}
 
 // Whether k_optimality's slots get room for the KKT factors of a group of sets:
 // where the block then fits on an SM, and not where an SM would hold one block

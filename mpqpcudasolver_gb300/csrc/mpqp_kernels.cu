@@ -5497,6 +5497,32 @@ const void *kernel_ptr(const char *name)
     return nullptr;
 }
 
+// The most dynamic shared memory a block can have (227 KB: the kernels that use
+// it have no static shared memory); 0 when the device does not say.
+size_t block_smem_limit()
+{
+    int dev = 0, bytes = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&bytes, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return (size_t)bytes;
+}
+
+// Lets fn be launched with smem bytes of dynamic shared memory.  A kernel's
+// limit is the device's, whatever a caller needs: a plan of smaller instances,
+// or one that is refused, takes nothing away from a plan that still runs.
+cudaError_t allow_smem(const void *fn, size_t smem)
+{
+    if (smem <= 48 * 1024) return cudaSuccess;
+    const size_t most = block_smem_limit();
+    if (smem > most) return cudaErrorInvalidValue;
+    const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+    if (e != cudaSuccess) cudaGetLastError();   // (not left for the next launch to report)
+    return e;
+}
+
 cudaError_t launch_enumerate(const DevBuffers &B, int level, int grid, cudaStream_t s)
 {
     k_enumerate<<<grid, 128, 0, s>>>(B, level);
@@ -5592,11 +5618,8 @@ cudaError_t launch_redundancy(const double *M, const double *d, int nrows, int n
                               double tol, const Tol &lt, int max_piv, int *out, int grid, size_t smem, cudaStream_t s)
 {
     const bool block = redundancy_block(nrows, nv);
-    if (smem > 48 * 1024) {
-        const void *fn = block ? (const void *)k_redundancy_block : (const void *)k_redundancy;
-        cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-    }
+    const cudaError_t e = allow_smem(block ? (const void *)k_redundancy_block : (const void *)k_redundancy, smem);
+    if (e != cudaSuccess) return e;
     if (block) k_redundancy_block<<<grid, 128, smem, s>>>(M, d, nrows, nv, ld, check, n_check, tol, lt, max_piv, out);
     else k_redundancy<<<grid, 32, smem, s>>>(M, d, nrows, nv, ld, check, n_check, tol, lt, max_piv, out);
     return cudaGetLastError();

@@ -38,6 +38,8 @@
 namespace mq {
 size_t laws_smem_per_warp(const SlotDims &sd);
 const void *kernel_ptr(const char *name);
+size_t block_smem_limit();
+cudaError_t allow_smem(const void *fn, size_t smem);
 cudaError_t launch_region_laws(const DevBuffers &B, const Tol &tol, const SlotDims &sd, const uint64_t *masks,
                                long long n_sets, double *laws, int *sizes, long long stride, int grid,
                                size_t smem, cudaStream_t s);
@@ -250,12 +252,12 @@ int noalloc_impl(const mpqp_problem *prob, long long n_sets, const uint64_t *mas
     sd.maxN = d.lp ? n : 0;
     const size_t smem = 4 * laws_smem_per_warp(sd);
     const void *fn = kernel_ptr("laws");
-    int sms = 0, nb = 0, smem_max = 0;
-    if (cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
-        return fail(MPQP_ECUDA, "mpqp_region_laws_noalloc: device attribute query");
-    if (smem > (size_t)smem_max)
+    int sms = 0, nb = 0;
+    const size_t smem_max = block_smem_limit();
+    if (!smem_max) return fail(MPQP_ECUDA, "mpqp_region_laws_noalloc: device attribute query");
+    if (smem > smem_max)
         return fail(MPQP_EINVAL, "mpqp_region_laws_noalloc: kernel does not fit on an SM (shared memory)");
-    if (smem > 48 * 1024 && cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    if (allow_smem(fn, smem) != cudaSuccess)
         return fail(MPQP_ECUDA, "mpqp_region_laws_noalloc: shared-memory attribute");
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, 128, smem) != cudaSuccess)

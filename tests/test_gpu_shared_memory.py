@@ -6,7 +6,10 @@ leave an SM one block instead of two): problems on both sides of these limits (w
 2) and of its limit |S| = 8, in both precisions, against the oracle.
 
 The LP1 kernel runs four warps a block with a tableau each: problems whose FP64
-tableaus leave less than 4 KB of a block's shared memory."""
+tableaus leave less than 4 KB of a block's shared memory.
+
+A problem that does not fit is refused, and neither it nor a smaller one changes
+what an earlier plan may launch."""
 import numpy as np
 import pytest
 
@@ -59,3 +62,25 @@ def test_group_and_single_factors_by_level(gpu_lib, make, n, m, p):
 def test_largest_lp1_tableaus(gpu_lib, n, m, p):
     prob = P.scale_problem(P.random_mpqp(n, m, p, seed=m + p))
     _compare(prob, O.enumerate_sets(prob, k_max=2, nthreads=8), k_max=2, opt_cap=1 << 14)
+
+
+def test_refused_and_smaller_plans_leave_a_larger_one_alone(gpu_lib):
+    large = P.scale_problem(P.random_mpqp(16, 128, 14, seed=1))      # 157 KB a block of LP1
+    oversized = P.scale_problem(P.random_mpqp(16, 128, 26, seed=2))  # 250 KB
+    smaller = P.scale_problem(P.random_mpqp(12, 80, 6, seed=3))      # 57 KB
+    tiny = P.scale_problem(P.random_n4_m10_p2())
+    want = solver.solve([tiny], precision=solver.FP64)
+    plan = solver.Plan([large], precision=solver.FP64, k_max=1, use_graph=0)
+    plan.run()
+    first = plan.results()
+    with pytest.raises(solver.MpqpError) as e:
+        solver.solve([oversized], precision=solver.FP64, k_max=1)
+    assert e.value.code == solver.ECUDA
+    assert solver.solve([tiny], precision=solver.FP64).inst.tobytes() == want.inst.tobytes()
+    solver.solve([smaller], precision=solver.FP64, k_max=1)
+    plan.run()
+    again = plan.results()
+    plan.close()
+    assert again.candidates == 129
+    for f in ("feasible_digest", "optimal_digest", "region_digest"):
+        assert np.array_equal(first.inst[f], again.inst[f])
