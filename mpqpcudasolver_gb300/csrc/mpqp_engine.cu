@@ -40,6 +40,7 @@ const void *kernel_ptr(const char *name);
 size_t block_smem_limit();
 cudaError_t allow_smem(const void *fn, size_t smem);
 cudaError_t launch_enumerate(const DevBuffers &B, int level, int grid, cudaStream_t s);
+cudaError_t launch_room(const DevBuffers &B, int level, cudaStream_t s);
 cudaError_t launch_order(const DevBuffers &B, cudaStream_t s);
 cudaError_t launch_scatter(const DevBuffers &B, int level, int grid, cudaStream_t s);
 cudaError_t launch_cover(const DevBuffers &B, int level, int grid, cudaStream_t s);
@@ -826,6 +827,7 @@ static int enqueue(mpqp_plan *P, cudaStream_t s, EventMode events)
         } else {
             L("k_enumerate", launch_enumerate(B, k, grid(P->grid_enum, k - 1, 4), s));
         }
+        if (!B.arena_ample) L("k_room", launch_room(B, k, s));
         L(feas, launch_feasibility(B, P->tol, P->sd, k, P->prec, grid(P->grid_feas, k, P->feas_warps), P->smem_feas, s,
                                    P->feas_warps, P->feas_chunk));
         if (mixed) {
@@ -1060,6 +1062,7 @@ static int plan_create_locked(int n_inst, const mpqp_problem *probs, const mpqp_
     B.node_cap = node_cap;
     B.tab_cap = tab_cap;
     B.ids_cap = ids_cap;
+    B.arena_ample = arena_max <= (double)tab_cap * es;
     B.hash_cap = hash_cap;
     B.cand_cap = cand_cap;
     B.q_cap = cand_cap;
@@ -1180,7 +1183,7 @@ static int plan_create_locked(int n_inst, const mpqp_problem *probs, const mpqp_
     P->smem_optfb = 4 * opt_smem_per_warp(sd, false);
     P->smem_direct = smem_opt64;
     if ((rc = grid_for(kernel_ptr("enumerate"), 0, &P->grid_enum)) ||
-        (rc = grid_for(kernel_ptr(P->prec == PREC_MIXED ? "feas32" : "feas64"), P->smem_feas, &P->grid_feas,
+        (rc = grid_for(kernel_ptr(P->prec != PREC_MIXED ? "feas64" : B.arena_ample ? "feas32" : "feas32_room"), P->smem_feas, &P->grid_feas,
                        32 * P->feas_warps)) ||
         (rc = grid_for(kernel_ptr("cover"), 0, &P->grid_cover)) ||
         (rc = grid_for(kernel_ptr("scatter"), 0, &P->grid_scatter)) ||

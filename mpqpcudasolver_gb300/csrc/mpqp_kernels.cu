@@ -819,9 +819,8 @@ __host__ __device__ inline size_t lp1_slot_bytes(int maxM1, int maxLD1, int maxN
 // slot of k_feasibility: one buffer, in FP32 two words per candidate of the
 // chunk (the arena offsets reserved for it, then its vertex's constraints), and
 // the warp's mbarrier (16 bytes, last).  In FP64, where a buffer can fill a
-// quarter of the SM, the offsets are read from the candidates' node records
-// (LP1 of n = 10, m = 43 to |S| = 4 with the offsets in shared memory / in the
-// records 1,957 / 1,969 us, of 24 small problems 1,547 / 1,586 us).
+// quarter of the SM, the lanes keep the offsets (LP1 of 24 small problems
+// 1,547 us with them in shared memory, 1,545 so, 1,600 read from the node records).
 template <typename T>
 __host__ __device__ inline size_t feas_slot_bytes(int maxM1, int maxLD1, int maxNv)
 {
@@ -1262,6 +1261,43 @@ __global__ void __launch_bounds__(128) k_scatter(DevBuffers B, int level)
     }
 }
 
+// Whether LP1 reserves arena space for every candidate of a level that may store
+// a tableau, a chunk's at once, also for those that turn out infeasible (up to a
+// fifth of a level on MPC problems).  Only where that cannot cost a set its
+// tableau: where the arena holds all of them beside their parents', and beside
+// them all that the next level could store.  A candidate of the next level has
+// level + 1 subsets here and a set at most m - level supersets there, so those
+// number at most n (m - level) / (level + 1).  Otherwise space is reserved for
+// each set as it is stored.  Enumeration with space always reserved ahead / by
+// this rule, arenas of 1000, 400 and 100 MB: 8 MPC problems to |S| = 4 (mixed)
+// 4.04 / 4.01, 5.27 / 5.11 and 5.54 / 5.37 ms, FP64 64.2 / 62.9, 72.2 / 72.4 and
+// 77.7 / 77.2 ms; 32 mpLPs, whose LPs of under two pivots gain least from a
+// tableau, 18.3 / 19.0, 20.2 / 20.5 and 21.7 / 22.0 ms.  One warp; not launched
+// for a plan whose arena holds every combination (DevBuffers::arena_ample).
+__global__ void __launch_bounds__(32) k_room(DevBuffers B, int level)
+{
+    Ctl *ctl = B.ctl;
+    const int pside = (level & 1) ^ 1;
+    long long now = 0, next = 0;
+    for (int i = lane_id(); i < B.n_inst; i += 32) {
+        const InstDesc &I = B.inst[i];
+        const InstCtl &ic = B.ictl[i];
+        if (ic.stopped || level >= I.k_max || (I.budget > 0 && ic.cum_cand + ic.lvl_cand > I.budget)) continue;
+        now += ic.lvl_cand * I.tab_elems;
+        if (level + 1 < I.k_max) {
+            const long long most = ic.lvl_cand * (I.m - level) / (level + 1);
+            next += (I.budget > 0 && most > I.budget ? I.budget : most) * I.tab_elems;
+        }
+    }
+#pragma unroll
+    for (int off = 16; off; off >>= 1) {
+        now += __shfl_xor_sync(FULLMASK, now, off);
+        next += __shfl_xor_sync(FULLMASK, next, off);
+    }
+    // (the arena of the ids holds as many records as the other one tableaus)
+    if (lane_id() == 0) ctl->ahead = ctl->tab_used[pside] + now <= B.tab_cap && now + next <= B.tab_cap;
+}
+
 // Whether the sets of a level have cover slots: their children are the
 // instance's last level.
 __device__ __forceinline__ bool covers(const InstDesc &I, int inst, int level)
@@ -1395,58 +1431,76 @@ __device__ __forceinline__ void insert_node(const DevBuffers &B, int side, int l
     }
 }
 
+// In place of a tableau's offset: reserved when the candidate is stored.
+constexpr long long kReserveLater = -2;
+
+// Whether a reservation failed at this level.
+__device__ __forceinline__ bool arena_full(const Ctl *ctl, int side) { return *((const volatile int *)&ctl->tab_full[side]) != 0; }
+
+// Arena space for one tableau and its ids, by one lane that has seen the arena
+// not full (or whose own last reservation succeeded); -1: it is full now.  One
+// arena per kind, side 0 filled upward from 0, side 1 downward from the top; the
+// other side holds the parents and is fixed here.
+__device__ __noinline__ longlong2 reserve_space(const DevBuffers &B, int side, int tab_elems, int ids_bytes)
+{
+    Ctl *ctl = B.ctl;
+    const long long told = (long long)atomicAdd((unsigned long long *)&ctl->tab_used[side], (unsigned long long)tab_elems);
+    const long long iold = (long long)atomicAdd((unsigned long long *)&ctl->ids_used[side], (unsigned long long)ids_bytes);
+    if (told + tab_elems + ctl->tab_used[side ^ 1] > B.tab_cap || iold + ids_bytes + ctl->ids_used[side ^ 1] > B.ids_cap) {
+        // this node and the later ones of the level keep no tableau (a
+        // reservation past the end is abandoned, so the used counts only
+        // overstate); their children start from the root tableau
+        atomicExch(&ctl->tab_full[side], 1);
+        return longlong2{-1, -1};
+    }
+    return side == 0 ? longlong2{told, iold} : longlong2{B.tab_cap - told - tab_elems, B.ids_cap - iold - ids_bytes};
+}
+
+// ... for candidate t of a chunk, into its two words of a FP32 slot; after a
+// failure no later candidate of the chunk asks again.  By the whole warp.
+__device__ __noinline__ void reserve_to(const DevBuffers &B, int side, int tab_elems, int ids_bytes, long long *room, int t)
+{
+    const int lane = lane_id();
+    longlong2 sp{0, 0};
+    if (lane == t) {
+        sp = reserve_space(B, side, tab_elems, ids_bytes);
+        room[t] = sp.x;
+        room[32 + t] = sp.y;
+    }
+    if (__any_sync(FULLMASK, sp.x < 0) && lane > t) room[lane] = -1;
+    __syncwarp();
+}
+
 // Append a feasible (or, exhaustive, any) candidate as a node of `side`;
-// stores its tableau when it can have children.  Returns the node index or -1.
+// stores its tableau when it can have children.
 // src_ld: row stride of `tab` (0: the plan's stride, copied as is).
 // bulk: tab and ids are a shared-memory slot of the plan's layout (src_ld 0,
 // TT = TS); lane 0 copies them with bulk stores (bulk_wait_read before the
 // slot is written again, bulk_wait_all before the kernel ends).
-// reserved: the arena space reserved before (reserved[0] the tableau's and
-// reserved[stride] the ids' offset, -1: none; stride 1: the candidate's node
-// record, whose ids_off follows tab_off).  chunked: k_feasibility, which counts
-// its stores and inserts its sets into the hash itself.
+// toff, ioff (lane 0's count): the arena space reserved for it, -1: none.
+// chunked: k_feasibility, which counts its stores and inserts its sets into the
+// hash itself.  Returns whether a tableau was stored.
 template <typename TT, typename TS>
-__device__ long long store_node(const DevBuffers &B, int side, int level, const InstDesc &I, int inst,
+__device__ bool store_node(const DevBuffers &B, int side, int level, const InstDesc &I, int inst,
                                 uint64_t lo, uint64_t hi, bool feasible, const TS *tab, const uint8_t *ids,
                                 long long rec, long long hcap, int extra_flags, int src_ld = 0, bool bulk = false,
                                 long long pre_idx = -1, int rows_store = -1, int cols_store = -1,
-                                const long long *reserved = nullptr, int stride = 0, bool chunked = false)
+                                long long toff = -1, long long ioff = -1, bool chunked = false)
 {
-    static_assert(offsetof(Node, ids_off) == offsetof(Node, tab_off) + sizeof(long long), "reserved, stride 1");
     const int lane = lane_id();
     Ctl *ctl = B.ctl;
     const bool need_tab = level < I.k_max;
-    long long idx = 0, toff = -1, ioff = -1;
+    long long idx = 0;
     if (lane == 0) {
-        // one arena per kind, side 0 filled upward from 0, side 1 downward
-        // from the top; the other side holds the parents and is fixed here
         // pre_idx >= 0: the caller's slot (a candidate's node lives at the
         // candidate's index)
         idx = pre_idx >= 0 ? pre_idx : (long long)atomicAdd((unsigned long long *)&ctl->n_node[side], 1ull);
         if (idx >= B.node_cap) { atomicOr(&ctl->overflow, OV_NODE); idx = -1; }
-        if (reserved) {
-            toff = reserved[0];
-            ioff = reserved[stride];
-        } else if (need_tab && idx >= 0 && !*((volatile int *)&ctl->tab_full[side])) {
-            const long long told = (long long)atomicAdd((unsigned long long *)&ctl->tab_used[side], (unsigned long long)I.tab_elems);
-            const long long iold = (long long)atomicAdd((unsigned long long *)&ctl->ids_used[side], (unsigned long long)I.ids_bytes);
-            if (told + I.tab_elems + ctl->tab_used[side ^ 1] > B.tab_cap ||
-                iold + I.ids_bytes + ctl->ids_used[side ^ 1] > B.ids_cap) {
-                // the arena is full: this node and the later ones of the level
-                // keep no tableau (a reservation past the end is abandoned, so
-                // the used counts only overstate); their children start from
-                // the root tableau
-                atomicExch(&ctl->tab_full[side], 1);
-            } else {
-                toff = side == 0 ? told : B.tab_cap - told - I.tab_elems;
-                ioff = side == 0 ? iold : B.ids_cap - iold - I.ids_bytes;
-            }
-        }
     }
     idx = __shfl_sync(FULLMASK, idx, 0);
     toff = __shfl_sync(FULLMASK, toff, 0);
     ioff = __shfl_sync(FULLMASK, ioff, 0);
-    if (idx < 0) return -1;
+    if (idx < 0) return false;
     if (need_tab && toff < 0) {
         // a node without a tableau (still in the hash: the subset test needs it)
         if (lane == 0) {
@@ -1458,7 +1512,7 @@ __device__ long long store_node(const DevBuffers &B, int side, int level, const 
             B.node[side][idx] = nd;
             if (feasible && !B.exhaustive && !chunked) insert_node(B, side, level, I, inst, lo, hi, hcap, 0, 0);
         }
-        return idx;
+        return false;
     }
     if (need_tab) {
         if (lane == 0 && !chunked) atomicAdd((unsigned long long *)&B.ictl[inst].stored, 1ull);
@@ -1501,7 +1555,7 @@ __device__ long long store_node(const DevBuffers &B, int side, int level, const 
         if (feasible && !B.exhaustive && need_tab && !chunked)
             insert_node(B, side, level, I, inst, lo, hi, hcap, 0, 0);
     }
-    return idx;
+    return need_tab;
 }
 
 // Before an FP32 LP1 tableau is stored for the next level: each live column
@@ -1658,7 +1712,10 @@ __device__ __noinline__ void cold_stage_lp1_f32(const DevBuffers &B, const InstD
 // T = float : the FP32 pass of the mixed path; a verdict is final only when
 //             certified (see below), otherwise the candidate is queued for
 //             the FP64 re-solve.
-template <typename T>
+// Ample: the arena holds every combination (DevBuffers::arena_ample).  A kernel
+// of its own in FP32, because the mere presence of the other route slowed LP1 of
+// 32 mpLPs from 2,950 to 3,290 us.
+template <typename T, bool Ample>
 __device__ __forceinline__ void feasibility_body(const DevBuffers &B, const Tol &tol, const SlotDims &sd, int level,
                                                  int chunk)
 {
@@ -1686,6 +1743,7 @@ __device__ __forceinline__ void feasibility_body(const DevBuffers &B, const Tol 
     LocalInstCounters lc;
     lc.reset(-1);
     chunk = claim_size(wend, chunk);
+    const bool ahead = Ample || B.arena_ample || ctl->ahead;   // see k_room
     for (;;) {
         long long w0;
         if (lane == 0) w0 = (long long)atomicAdd(&ctl->ctr[0], (unsigned long long)chunk);
@@ -1703,44 +1761,38 @@ __device__ __forceinline__ void feasibility_body(const DevBuffers &B, const Tol 
         // lane t holds candidate t's parent tableau offset (for the prefetch)
         const long long my_toff = lane < cnt ? B.node[pside][mine.parent].tab_off : -1;
         const int my_inst = lane < cnt ? B.node[pside][mine.parent].inst : 0;
-        // Arena space for the tableaus of the whole chunk (also of the few
-        // candidates that will store none; one that goes to the FP64 re-solve
-        // finds its space in its node record): one pair of atomics instead of a
-        // pair per stored candidate, whose round trip the warp waited for.  With
-        // the hash inserts below: LP1 of 32 mpLPs (1.7M sets, 1.7 pivots each)
-        // 5,248 -> 3,297 us, of the m = 62 batch 177 -> 167 ms
+        // Where the arena has room to spare, space for the tableaus of the whole
+        // chunk (a candidate that goes to the FP64 re-solve finds its space in
+        // its node record): one pair of atomics instead of a pair per stored
+        // candidate, whose round trip the warp waited for.  With the hash inserts
+        // below: LP1 of 32 mpLPs (1.7M sets, 1.7 pivots each) 5,248 -> 3,297 us, of
+        // the m = 62 batch 177 -> 167 ms
+        long long toff = -1, ioff = -1;
         bool live = false;    // this lane's candidate is checked (its instance has not stopped)
-        bool keeps = false;   // ... and stores a tableau when feasible
         {
             const InstDesc &Il = B.inst[my_inst];
             const InstCtl &il = B.ictl[my_inst];
             live = lane < cnt && !il.stopped && !(Il.budget > 0 && il.cum_cand + il.lvl_cand > Il.budget);
-            keeps = live && level < Il.k_max;
-            const int te = keeps ? Il.tab_elems : 0, ib = keeps ? Il.ids_bytes : 0;
+            const bool keeps = live && level < Il.k_max;   // ... and stores a tableau when feasible
+            const int te = ahead && keeps ? Il.tab_elems : 0, ib = ahead && keeps ? Il.ids_bytes : 0;
             int ts = te, is = ib;   // inclusive sums
 #pragma unroll
             for (int off = 1; off < 32; off <<= 1) {
                 const int tv = __shfl_up_sync(FULLMASK, ts, off), iv = __shfl_up_sync(FULLMASK, is, off);
                 if (lane >= off) { ts += tv; is += iv; }
             }
-            long long tb = -1, ibase = 0;
-            if (lane == 31 && ts > 0 && !*((volatile int *)&ctl->tab_full[side])) {
+            long long tb = 0, ibase = 0;
+            if (lane == 31 && ts > 0) {
                 tb = (long long)atomicAdd((unsigned long long *)&ctl->tab_used[side], (unsigned long long)ts);
                 ibase = (long long)atomicAdd((unsigned long long *)&ctl->ids_used[side], (unsigned long long)is);
             }
             tb = __shfl_sync(FULLMASK, tb, 31);
             ibase = __shfl_sync(FULLMASK, ibase, 31);
-            long long toff = -1, ioff = -1;
-            if (keeps && tb >= 0) {
-                const long long told = tb + ts - te, iold = ibase + is - ib;
-                if (told + te + ctl->tab_used[side ^ 1] > B.tab_cap || iold + ib + ctl->ids_used[side ^ 1] > B.ids_cap) {
-                    // the arena is full: this node and the later ones of the level
-                    // keep no tableau (see store_node)
-                    atomicExch(&ctl->tab_full[side], 1);
-                } else {
-                    toff = side == 0 ? told : B.tab_cap - told - te;
-                    ioff = side == 0 ? iold : B.ids_cap - iold - ib;
-                }
+            if (!ahead && keeps && !arena_full(ctl, side)) toff = kReserveLater;
+            if (ahead && keeps) {
+                // side 0 from the arena's start, side 1 from its end (see store_node)
+                toff = side == 0 ? tb + ts - te : B.tab_cap - tb - ts;
+                ioff = side == 0 ? ibase + is - ib : B.ids_cap - ibase - is;
             }
             if constexpr (mixed) {
                 room[lane] = toff;
@@ -2027,13 +2079,20 @@ __device__ __forceinline__ void feasibility_body(const DevBuffers &B, const Tol 
                     cols = feasible && !B.exhaustive
                                ? retire_fixed_columns(tab, ld, rows, pcols, nid, nv, lo, hi) : pcols;
             }
-            const long long *res = mixed ? room + t
-                                         : nbase + t < B.node_cap ? &B.node[side][nbase + t].tab_off : nullptr;
-            store_node<T, T>(B, side, level, I, inst, lo, hi, feasible, tab, ids, rec, hcap,
-                             mixed && feasible ? NODE_CERT : 0, 0, true, nbase + t, mixed ? rows : -1,
-                             mixed ? cols : -1, res, mixed ? 32 : 1, true);
+            longlong2 sp{-1, -1};
+            if constexpr (mixed) {
+                if (!Ample && room[t] == kReserveLater) reserve_to(B, side, I.tab_elems, I.ids_bytes, room, t);
+                sp = longlong2{room[t], room[32 + t]};
+            } else {
+                sp = longlong2{__shfl_sync(FULLMASK, toff, t), __shfl_sync(FULLMASK, ioff, t)};
+                if (sp.x == kReserveLater && lane == 0)
+                    sp = arena_full(ctl, side) ? longlong2{-1, -1} : reserve_space(B, side, I.tab_elems, I.ids_bytes);
+            }
+            const bool kept = store_node<T, T>(B, side, level, I, inst, lo, hi, feasible, tab, ids, rec, hcap,
+                                               mixed && feasible ? NODE_CERT : 0, 0, true, nbase + t,
+                                               mixed ? rows : -1, mixed ? cols : -1, sp.x, sp.y, true);
+            lc.d += kept;
             if (level < I.k_max) {
-                lc.d += lane == 0 && res && *res >= 0;
                 if (feasible && !B.exhaustive) stored |= 1u << t;
                 if constexpr (mixed) {
                     // the constraints nonbasic at this certified vertex, in place of the offsets
@@ -2075,15 +2134,16 @@ __device__ __forceinline__ void feasibility_body(const DevBuffers &B, const Tol 
     }
 }
 
+template <bool Ample>
 __global__ void __launch_bounds__(128) k_feasibility_f32(DevBuffers B, Tol tol, SlotDims sd, int level, int chunk)
 {
-    feasibility_body<float>(B, tol, sd, level, chunk);
+    feasibility_body<float, Ample>(B, tol, sd, level, chunk);
 }
 
 __global__ void __launch_bounds__(128, kF64Blocks) k_feasibility_f64(DevBuffers B, Tol tol, SlotDims sd, int level,
                                                                      int chunk)
 {
-    feasibility_body<double>(B, tol, sd, level, chunk);
+    feasibility_body<double, false>(B, tol, sd, level, chunk);
 }
 
 // ---------------------------------------------------------------------
@@ -2152,9 +2212,16 @@ __global__ void __launch_bounds__(128, kF64Blocks) k_lp1_fp64(DevBuffers B, Tol 
                 R.lp1_status = st; R.lp1_pivots += piv; R.z = z; R.feasible = feasible; R.fp64 |= 1;
             }
         }
-        if (feasible || B.exhaustive)
+        if (feasible || B.exhaustive) {
+            // the space k_feasibility reserved is in the candidate's node record
+            longlong2 sp{-1, -1};
+            if (lane == 0 && level < I.k_max) {
+                if (w < B.node_cap) sp = longlong2{B.node[side][w].tab_off, B.node[side][w].ids_off};
+                if (sp.x < 0 && !arena_full(ctl, side)) sp = reserve_space(B, side, I.tab_elems, I.ids_bytes);
+            }
             store_node<float, double>(B, side, level, I, inst, lo, hi, feasible, tab, ids, rec, hcap, 0, I.ld1d, false,
-                                      w, rows, -1, w < B.node_cap ? &B.node[side][w].tab_off : nullptr, 1);
+                                      w, rows, -1, sp.x, sp.y);
+        }
     }
 }
 
@@ -5466,7 +5533,8 @@ const void *kernel_ptr(const char *name)
         {"cover", (const void *)k_cover},
         {"scatter", (const void *)k_scatter},
         {"feas64", (const void *)k_feasibility_f64},
-        {"feas32", (const void *)k_feasibility_f32},
+        {"feas32", (const void *)k_feasibility_f32<true>},
+        {"feas32_room", (const void *)k_feasibility_f32<false>},
         {"lp1_fp64", (const void *)k_lp1_fp64},
         {"lp1_cert", (const void *)k_lp1_cert},
         {"opt64", (const void *)k_optimality<double, false>},
@@ -5529,6 +5597,12 @@ cudaError_t launch_enumerate(const DevBuffers &B, int level, int grid, cudaStrea
     return cudaGetLastError();
 }
 
+cudaError_t launch_room(const DevBuffers &B, int level, cudaStream_t s)
+{
+    k_room<<<1, 32, 0, s>>>(B, level);
+    return cudaGetLastError();
+}
+
 // the level's candidates, from cand_raw to cand by instance
 cudaError_t launch_order(const DevBuffers &B, cudaStream_t s)
 {
@@ -5555,7 +5629,8 @@ cudaError_t launch_feasibility(const DevBuffers &B, const Tol &tol, const SlotDi
 {
     if (warps < 1 || warps > 4 || chunk < 1 || chunk > kFeasChunkMax) return cudaErrorInvalidValue;
     if (prec == PREC_FP64) k_feasibility_f64<<<grid, 32 * warps, smem, s>>>(B, tol, sd, level, chunk);
-    else k_feasibility_f32<<<grid, 32 * warps, smem, s>>>(B, tol, sd, level, chunk);
+    else if (B.arena_ample) k_feasibility_f32<true><<<grid, 32 * warps, smem, s>>>(B, tol, sd, level, chunk);
+    else k_feasibility_f32<false><<<grid, 32 * warps, smem, s>>>(B, tol, sd, level, chunk);
     return cudaGetLastError();
 }
 
