@@ -256,7 +256,9 @@ typedef struct {
     int tuned;                    /* 1: chosen by the autotuner             */
     int split_levels;             /* levels whose feasible sets did not all
                                      keep an LP1 tableau (arena full)       */
-    int pad_;
+    int plain_roots;              /* mixed: instances whose FP64 LP1 re-solves
+                                     start from the constraint rows, because
+                                     pre-pivoting them grew too far         */
 } mpqp_batch_result;
 
 void mpqp_default_options(mpqp_options *opt);

@@ -143,13 +143,20 @@ static inline int four_mod8_up(int x) { int y = (x + 3) & ~3; return (y & 4) ? y
 // (bid over M1, 255 past the live rows, then nid over nv); d.root_rows the
 // live rows.  Pivots in FP64: T_r /= T_rq (T_rq -> 1 / T_rq), then
 // T_i -= T_iq T_r (T_iq -> -T_iq / T_rq), the Tucker pivot of the kernels.
-// Returns the entry growth: the largest multiplier of a pivot or |T_ij| left.
+// Returns the growth: the largest |T_ij|, right-hand sides included, that any
+// pivot left in a row (also where later pivots cancel it: its rounding stays).
 static double prepivot_root_f(InstDesc &d, std::vector<double> &root_f)
 {
     const int ld = d.ld1, nv = d.nv, M1 = d.M1;
     std::vector<double> T(root_f.begin(), root_f.begin() + (size_t)(M1 + 1) * ld);
     std::vector<int> bid(M1), nid(nv);
-    double growth = 0.0;
+    std::vector<double> top(nv + 1, 0.0);   // per column, so that the scan vectorises
+    auto scan = [&](const double *Ti) {
+        for (int j = 0; j <= nv; j++) {
+            const double v = std::fabs(Ti[j]);
+            top[j] = top[j] < v ? v : top[j];
+        }
+    };
     for (int i = 0; i < M1; i++) bid[i] = nv + i;
     for (int j = 0; j < nv; j++) nid[j] = j;
     for (int q = 0; q < nv; q++) {
@@ -179,15 +186,15 @@ static double prepivot_root_f(InstDesc &d, std::vector<double> &root_f)
             if (i == r) continue;
             double *Ti = T.data() + (size_t)i * ld;
             const double f = Ti[q];
-            if (f == 0.0) continue;
-            for (int j = 0; j <= nv; j++) Ti[j] -= f * R[j];
-            Ti[q] = -f * inv;
+            if (f != 0.0) {
+                for (int j = 0; j <= nv; j++) Ti[j] -= f * R[j];
+                Ti[q] = -f * inv;
+            }
+            if (i < M1) scan(Ti);
         }
+        scan(R);
         std::swap(bid[r], nid[q]);
-        growth = std::max(growth, cmax * std::fabs(inv));
     }
-    for (int i = 0; i < M1; i++)
-        for (int j = 0; j < nv; j++) growth = std::max(growth, std::fabs(T[(size_t)i * ld + j]));
     std::vector<double> out((size_t)d.tab_elems + M1 + nv, 0.0);
     int rows = 0;
     for (int i = 0; i < M1; i++) {
@@ -201,6 +208,8 @@ static double prepivot_root_f(InstDesc &d, std::vector<double> &root_f)
     for (int j = 0; j < nv; j++) out[(size_t)d.tab_elems + M1 + j] = nid[j];
     root_f.swap(out);
     d.root_rows = rows;
+    double growth = 0.0;
+    for (double v : top) growth = std::max(growth, v);
     return growth;
 }
 
@@ -245,9 +254,10 @@ static void add_products(const double *V, int m, const double *U, int w, int n, 
     }
 }
 
-// largest entry growth of the host's pre-pivoting (FP64: errors of about 1e-16
-// times it, against the 1e-9 of tol_feas) with which the FP64 re-solves start
-// from the pre-pivoted root
+// largest growth of the host's pre-pivoting (FP64: errors of about 1e-16 times
+// it in the entries and, absolutely, in the right-hand sides, against the 1e-9 of
+// tol_feas) with which the FP64 re-solves start from the pre-pivoted root.  The
+// repository's problems, scaled, reach 70 (700 problems of every kind)
 constexpr double kPrepivotGrowth = 1e4;
 
 static int prepare_instance(const mpqp_problem &P, Prepared &out, int prec)
@@ -359,8 +369,8 @@ static int prepare_instance(const mpqp_problem &P, Prepared &out, int prec)
     };
     fill_root(out.root, d.ld1d);
     // the FP64 re-solves of the mixed path start from the same pre-pivoted
-    // tableau, unless its pivots grew the entries so far that starting from the
-    // constraint rows themselves is the safer FP64 arbiter
+    // tableau, unless its pivots grew the entries or the right-hand sides so far
+    // that starting from the constraint rows themselves is the safer FP64 arbiter
     double growth = 0.0;
     if (prec == PREC_MIXED) {
         fill_root(out.root_f, d.ld1);
@@ -1655,6 +1665,7 @@ static int plan_results_impl(mpqp_plan *P, mpqp_batch_result *&R, bool *complete
     }
     R->n_levels = nlev;
     R->split_levels = (int)ctl.split_levels;
+    for (const InstDesc &d : P->desc) R->plain_roots += P->prec == PREC_MIXED && d.o_rootp < 0;
     long long nopt = std::min(ctl.n_opt, P->B.opt_cap);
     std::vector<OptRec> ov(nopt);
     if (nopt) memcpy(ov.data(), head.data() + off_opt, sizeof(OptRec) * std::min(nopt, first));

@@ -71,7 +71,7 @@ class BatchResult(ctypes.Structure):
                 ("n_rec", ctypes.c_longlong), ("rec", ctypes.c_void_p), ("h2d_bytes", ctypes.c_longlong),
                 ("d2h_bytes", ctypes.c_longlong), ("tile_w", ctypes.c_int), ("feas_warps", ctypes.c_int),
                 ("feas_chunk", ctypes.c_int), ("tuned", ctypes.c_int), ("split_levels", ctypes.c_int),
-                ("pad_", ctypes.c_int)]
+                ("plain_roots", ctypes.c_int)]
 
 
 class GPUResults(ctypes.Structure):
@@ -232,6 +232,7 @@ class Result:
     d2h_bytes: int = 0
     settings: dict | None = None   # launch settings of the run (tile_w, feas_warps, feas_chunk, tuned)
     split_levels: int = 0          # levels whose feasible sets did not all keep an LP1 tableau
+    plain_roots: int = 0           # mixed: instances whose FP64 LP1 re-solves start from the constraint rows
 
     @property
     def candidates(self) -> int:
@@ -269,7 +270,7 @@ def _convert(rp) -> Result:
         rec = np.frombuffer(buf, dtype=REC_DTYPE).copy()
     settings = dict(tile_w=r.tile_w, feas_warps=r.feas_warps, feas_chunk=r.feas_chunk, tuned=r.tuned)
     return Result(r.status, r.device_ms, r.n_levels, r.overflow, inst, opt, rec, r.h2d_bytes, r.d2h_bytes, settings,
-                  r.split_levels)
+                  r.split_levels, r.plain_roots)
 
 
 def solve(probs, precision: int = FP64, k_min: int = 0, k_max=None, budget=0, **opts) -> Result:
