@@ -7,6 +7,7 @@ missing or when a CUDA call fails.
 from __future__ import annotations
 
 import ctypes
+import operator
 import os
 from dataclasses import dataclass
 
@@ -195,19 +196,23 @@ class _ProblemSet:
                        for nm, t in Problem._fields_], align=True)
 
     def __init__(self, probs, k_min=0, k_max=None, budget=0):
+        # integers as the C structure's fields take them: no floats
+        as_int = lambda t, x: t(operator.index(x)).value  # noqa: E731
         flat, rows, off = [], [], 0
+        k_min = as_int(ctypes.c_int, k_min)
         for i, pr in enumerate(probs):
             n, m = pr.n, pr.m
             kmax = n if k_max is None else (k_max[i] if isinstance(k_max, (list, tuple)) else k_max)
             bud = budget[i] if isinstance(budget, (list, tuple)) else budget
-            row = [n, m, pr.p, pr.CRA.shape[0], k_min, min(kmax, m), int(bud)]
+            row = [n, m, pr.p, pr.CRA.shape[0], k_min, as_int(ctypes.c_int, min(kmax, m)),
+                   as_int(ctypes.c_longlong, int(bud))]
             for a in (pr.Q, pr.c, pr.H, pr.A, pr.b, pr.F, pr.CRA, pr.CRb):
-                a = np.ravel(a)
+                a = np.asarray(a, dtype=np.float64).ravel()
                 flat.append(a)
                 row.append(off)
                 off += a.size
             rows.append(tuple(row))
-        self.keep = np.concatenate(flat, dtype=np.float64) if flat else np.zeros(0)
+        self.keep = np.concatenate(flat) if flat else np.zeros(0)
         self.rec = np.array(rows, dtype=self._DTYPE)
         base = self.keep.ctypes.data
         for nm in ("Q", "c", "H", "A", "b", "F", "At", "bt"):
