@@ -1134,11 +1134,10 @@ static int plan_create_locked(int n_inst, const mpqp_problem *probs, const mpqp_
     // what only saves time comes last: a plan with an arena size of the caller's
     // that leaves no room for it does without
     if (cover_cap) {
-        void *c0 = nullptr, *c1 = nullptr;
-        const size_t bytes = sizeof(CoverSlot) * cover_cap;
-        if (dev_alloc(P, &c0, bytes) == MPQP_OK && dev_alloc(P, &c1, bytes) == MPQP_OK) {
-            B.cover[0] = (CoverSlot *)c0;
-            B.cover[1] = (CoverSlot *)c1;
+        void *c = nullptr;   // both sides in one block: it is there or it is not
+        if (dev_alloc(P, &c, 2 * sizeof(CoverSlot) * cover_cap) == MPQP_OK) {
+            B.cover[0] = (CoverSlot *)c;
+            B.cover[1] = B.cover[0] + cover_cap;
             B.cover_cap = cover_cap;
         }
     }
