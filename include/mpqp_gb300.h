@@ -286,9 +286,11 @@ void mpqp_plan_destroy(mpqp_plan *plan);
 
 /* Plans take their device memory from a pool (one per device) that keeps
  * freed memory for the next plan, so destroying a plan is cheap; the pool's
- * idle memory counts as free when a plan sizes its buffers.  This returns the
- * idle memory of the current device's pool to the driver.  No counterpart in
- * the reference (its buffers live inside each mpqp() call). */
+ * idle memory counts as free when a plan sizes its buffers.  Region laws and row
+ * reductions use it too; a laws call of more than 64 MB gives back what it made
+ * the pool grow by.  This returns the idle memory of the current device's pool
+ * to the driver.  No counterpart in the reference (its buffers live inside each
+ * mpqp() call). */
 int mpqp_release_cached_memory(void);
 
 /* Region laws of optimal sets, computed in FP64 on the device:
