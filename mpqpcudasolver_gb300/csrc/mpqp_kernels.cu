@@ -1270,9 +1270,9 @@ __global__ void __launch_bounds__(128) k_scatter(DevBuffers B, int level)
 // number at most n (m - level) / (level + 1).  Otherwise space is reserved for
 // each set as it is stored.  Enumeration with space always reserved ahead / by
 // this rule, arenas of 1000, 400 and 100 MB: 8 MPC problems to |S| = 4 (mixed)
-// 4.04 / 4.01, 5.27 / 5.11 and 5.54 / 5.37 ms, FP64 64.2 / 62.9, 72.2 / 72.4 and
-// 77.7 / 77.2 ms; 32 mpLPs, whose LPs of under two pivots gain least from a
-// tableau, 18.3 / 19.0, 20.2 / 20.5 and 21.7 / 22.0 ms.  One warp; not launched
+// 4.04 / 3.98, 5.27 / 5.14 and 5.54 / 5.44 ms, FP64 64.2 / 62.8, 72.2 / 72.1 and
+// 77.7 / 77.3 ms; 32 mpLPs, whose LPs of under two pivots gain least from a
+// tableau, 18.3 / 19.3, 20.2 / 20.7 and 21.7 / 22.0 ms.  One warp; not launched
 // for a plan whose arena holds every combination (DevBuffers::arena_ample).
 __global__ void __launch_bounds__(32) k_room(DevBuffers B, int level)
 {
@@ -1471,36 +1471,29 @@ __device__ __noinline__ void reserve_to(const DevBuffers &B, int side, int tab_e
     __syncwarp();
 }
 
-// Append a feasible (or, exhaustive, any) candidate as a node of `side`;
-// stores its tableau when it can have children.
-// src_ld: row stride of `tab` (0: the plan's stride, copied as is).
-// bulk: tab and ids are a shared-memory slot of the plan's layout (src_ld 0,
-// TT = TS); lane 0 copies them with bulk stores (bulk_wait_read before the
-// slot is written again, bulk_wait_all before the kernel ends).
-// toff, ioff (lane 0's count): the arena space reserved for it, -1: none.
+// A feasible (or, exhaustive, any) candidate as node idx (the candidate's own
+// index) of `side`; stores its tableau when it can have children.
+// src_ld: 0 when tab and ids are a shared-memory slot of the plan's layout (TT =
+// TS), which lane 0 copies with bulk stores (bulk_wait_read before the slot is
+// written again, bulk_wait_all before the kernel ends); else the row stride of
+// `tab`, copied row by row.
+// rows_store, cols_store: the live rows and columns (-1: all).
+// toff, ioff: the arena space reserved for it, -1: none.
 // chunked: k_feasibility, which counts its stores and inserts its sets into the
 // hash itself.  Returns whether a tableau was stored.
 template <typename TT, typename TS>
 __device__ bool store_node(const DevBuffers &B, int side, int level, const InstDesc &I, int inst,
-                                uint64_t lo, uint64_t hi, bool feasible, const TS *tab, const uint8_t *ids,
-                                long long rec, long long hcap, int extra_flags, int src_ld = 0, bool bulk = false,
-                                long long pre_idx = -1, int rows_store = -1, int cols_store = -1,
-                                long long toff = -1, long long ioff = -1, bool chunked = false)
+                           uint64_t lo, uint64_t hi, bool feasible, const TS *tab, const uint8_t *ids,
+                           long long rec, long long hcap, int extra_flags, int src_ld, long long idx,
+                           int rows_store = -1, int cols_store = -1, long long toff = -1, long long ioff = -1,
+                           bool chunked = false)
 {
     const int lane = lane_id();
-    Ctl *ctl = B.ctl;
     const bool need_tab = level < I.k_max;
-    long long idx = 0;
-    if (lane == 0) {
-        // pre_idx >= 0: the caller's slot (a candidate's node lives at the
-        // candidate's index)
-        idx = pre_idx >= 0 ? pre_idx : (long long)atomicAdd((unsigned long long *)&ctl->n_node[side], 1ull);
-        if (idx >= B.node_cap) { atomicOr(&ctl->overflow, OV_NODE); idx = -1; }
+    if (idx >= B.node_cap) {
+        if (lane == 0) atomicOr(&B.ctl->overflow, OV_NODE);
+        return false;
     }
-    idx = __shfl_sync(FULLMASK, idx, 0);
-    toff = __shfl_sync(FULLMASK, toff, 0);
-    ioff = __shfl_sync(FULLMASK, ioff, 0);
-    if (idx < 0) return false;
     if (need_tab && toff < 0) {
         // a node without a tableau (still in the hash: the subset test needs it)
         if (lane == 0) {
@@ -1517,7 +1510,7 @@ __device__ bool store_node(const DevBuffers &B, int side, int level, const InstD
     if (need_tab) {
         if (lane == 0 && !chunked) atomicAdd((unsigned long long *)&B.ictl[inst].stored, 1ull);
         TT *dst = (TT *)B.tab[side] + toff;
-        if (bulk) {
+        if (src_ld == 0) {
             fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0) {
@@ -1527,8 +1520,6 @@ __device__ bool store_node(const DevBuffers &B, int side, int level, const InstD
                 bulk_store(B.ids[side] + ioff, ids, (unsigned)I.ids_bytes);
                 bulk_commit();
             }
-        } else if (src_ld == 0) {
-            warp_copy_v<TT>(dst, (const TT *)tab, I.tab_elems);
         } else {
             // re-stride (and convert) row by row; padding columns become 0
             // (rows_store >= 0: the live rows and the objective row after them)
@@ -1537,8 +1528,6 @@ __device__ bool store_node(const DevBuffers &B, int side, int level, const InstD
                 const int i = e / I.ld1, j = e - i * I.ld1;
                 dst[e] = j < ncol ? (TT)tab[(size_t)i * src_ld + j] : TT(0);
             }
-        }
-        if (!bulk) {
             uint8_t *di = B.ids[side] + ioff;
             for (int e = lane; e < I.M1 + I.nv; e += 32) di[e] = ids[e];
         }
@@ -1714,7 +1703,7 @@ __device__ __noinline__ void cold_stage_lp1_f32(const DevBuffers &B, const InstD
 //             the FP64 re-solve.
 // Ample: the arena holds every combination (DevBuffers::arena_ample).  A kernel
 // of its own in FP32, because the mere presence of the other route slowed LP1 of
-// 32 mpLPs from 2,950 to 3,290 us.
+// 32 mpLPs by a tenth (2,830 us without it).
 template <typename T, bool Ample>
 __device__ __forceinline__ void feasibility_body(const DevBuffers &B, const Tol &tol, const SlotDims &sd, int level,
                                                  int chunk)
@@ -1743,7 +1732,7 @@ __device__ __forceinline__ void feasibility_body(const DevBuffers &B, const Tol 
     LocalInstCounters lc;
     lc.reset(-1);
     chunk = claim_size(wend, chunk);
-    const bool ahead = Ample || B.arena_ample || ctl->ahead;   // see k_room
+    const bool ahead = Ample || (!mixed && B.arena_ample) || ctl->ahead;   // see k_room
     for (;;) {
         long long w0;
         if (lane == 0) w0 = (long long)atomicAdd(&ctl->ctr[0], (unsigned long long)chunk);
@@ -2085,11 +2074,13 @@ __device__ __forceinline__ void feasibility_body(const DevBuffers &B, const Tol 
                 sp = longlong2{room[t], room[32 + t]};
             } else {
                 sp = longlong2{__shfl_sync(FULLMASK, toff, t), __shfl_sync(FULLMASK, ioff, t)};
-                if (sp.x == kReserveLater && lane == 0)
-                    sp = arena_full(ctl, side) ? longlong2{-1, -1} : reserve_space(B, side, I.tab_elems, I.ids_bytes);
+                if (sp.x == kReserveLater) {
+                    if (lane == 0) sp = arena_full(ctl, side) ? longlong2{-1, -1} : reserve_space(B, side, I.tab_elems, I.ids_bytes);
+                    sp = longlong2{__shfl_sync(FULLMASK, sp.x, 0), __shfl_sync(FULLMASK, sp.y, 0)};
+                }
             }
             const bool kept = store_node<T, T>(B, side, level, I, inst, lo, hi, feasible, tab, ids, rec, hcap,
-                                               mixed && feasible ? NODE_CERT : 0, 0, true, nbase + t,
+                                               mixed && feasible ? NODE_CERT : 0, 0, nbase + t,
                                                mixed ? rows : -1, mixed ? cols : -1, sp.x, sp.y, true);
             lc.d += kept;
             if (level < I.k_max) {
@@ -2219,8 +2210,9 @@ __global__ void __launch_bounds__(128, kF64Blocks) k_lp1_fp64(DevBuffers B, Tol 
                 if (w < B.node_cap) sp = longlong2{B.node[side][w].tab_off, B.node[side][w].ids_off};
                 if (sp.x < 0 && !arena_full(ctl, side)) sp = reserve_space(B, side, I.tab_elems, I.ids_bytes);
             }
-            store_node<float, double>(B, side, level, I, inst, lo, hi, feasible, tab, ids, rec, hcap, 0, I.ld1d, false,
-                                      w, rows, -1, sp.x, sp.y);
+            sp = longlong2{__shfl_sync(FULLMASK, sp.x, 0), __shfl_sync(FULLMASK, sp.y, 0)};
+            store_node<float, double>(B, side, level, I, inst, lo, hi, feasible, tab, ids, rec, hcap, 0, I.ld1d, w, rows,
+                                      -1, sp.x, sp.y);
         }
     }
 }
@@ -2471,8 +2463,7 @@ __global__ void __launch_bounds__(128) k_lp1_cert(DevBuffers B, Tol tol, SlotDim
                     atomicAdd(&ic->feas_digest, mask_digest(lo, hi));
                     if (rec >= 0) { B.rec[rec].feasible = 1; B.rec[rec].fp64 |= 16; B.rec[rec].lp1_bound = bound; }
                 }
-                store_node<float, double>(B, level & 1, level, I, inst, lo, hi, true, nullptr, nullptr, rec, 0, 0, 0,
-                                          false, w);
+                store_node<float, double>(B, level & 1, level, I, inst, lo, hi, true, nullptr, nullptr, rec, 0, 0, 0, w);
             } else if (lane == 0) {
                 const long long qi = (long long)atomicAdd((unsigned long long *)&ctl->n_q_lp1, 1ull);
                 if (qi < B.q_cap) B.q_lp1[qi] = w; else atomicOr(&ctl->overflow, OV_QUEUE);
