@@ -1715,7 +1715,7 @@ static int plan_results_impl(mpqp_plan *P, mpqp_batch_result *&R, bool *complete
     }
     R->h2d_bytes = P->h2d_bytes;
     R->tile_w = P->tile_w; R->feas_warps = P->feas_warps; R->feas_chunk = P->feas_chunk; R->tuned = P->tuned;
-    R->d2h_bytes = (long long)(sizeof(Ctl) + sizeof(InstCtl) * P->n_inst + sizeof(OptRec) * nopt);
+    R->d2h_bytes = (long long)(head.size() + sizeof(OptRec) * std::max(nopt - first, 0LL));
     if (P->B.rec) {
         long long nrec = std::min(ctl.rec_base, P->B.rec_cap);
         R->d2h_bytes += (long long)sizeof(CandRec) * nrec;
