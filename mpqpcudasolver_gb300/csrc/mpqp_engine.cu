@@ -45,7 +45,7 @@ cudaError_t launch_order(const DevBuffers &B, cudaStream_t s);
 cudaError_t launch_scatter(const DevBuffers &B, int level, int grid, cudaStream_t s);
 cudaError_t launch_cover(const DevBuffers &B, int level, int grid, cudaStream_t s);
 cudaError_t launch_feasibility(const DevBuffers &B, const Tol &tol, const SlotDims &sd, int level, int prec,
-                               int grid, size_t smem, cudaStream_t s, int warps, int chunk);
+                               int grid, size_t smem, cudaStream_t s, int warps, int chunk, bool ask);
 cudaError_t launch_lp1_fp64(const DevBuffers &B, const Tol &tol, const SlotDims &sd, int level, int grid,
                             size_t smem, cudaStream_t s);
 cudaError_t launch_lp1_cert(const DevBuffers &B, const Tol &tol, const SlotDims &sd, int level, int grid,
@@ -441,6 +441,8 @@ struct mpqp_plan {
     int tile_w = 8, feas_warps = 4, feas_chunk = 32;
     int tuned = 0;              // 1: the settings came from the autotuner (or its cache)
     size_t smem_opt2 = 0;       // shared memory per block of the primal route
+    bool arena_ample = false;   // the arena holds the tableaus of every combination of two levels in a row
+    int grid_feas_room = 0;     // LP1 with arena space as k_room says
     int grid_enum = 0, grid_feas = 0, grid_lp1fb = 0, grid_opt = 0, grid_optfb = 0, grid_cert = 0;
     size_t smem_feas = 0, smem_lp1fb = 0, smem_opt = 0, smem_optfb = 0, smem_direct = 0, smem_cert = 0;
     int n_launches = 0;
@@ -697,6 +699,18 @@ constexpr double kDirectWaves = 3.0, kOnePassWaves = 4.0;
 // (95,284) 1,191 / 1,169, m = 48 to 4 (194,580) 1,314 / 1,264
 constexpr double kCoverMin = 100000.0;
 
+// sets of a level from which LP1 reserves arena space ahead whatever the arena's
+// size; below, in a plan whose arena is limited, as k_room says.  Reserving for each
+// set as it is stored costs round trips, reserving ahead the space of the
+// candidates that turn out infeasible, which are few on large levels.  Enumeration
+// with space always reserved ahead / as k_room says, sets without a tableau: 64 MPC
+// problems toward |S| = 12 (levels of 8 to 40M) in 200 GB 449 / 513 ms, 29.35M /
+// 29.21M; 32 mpLPs (up to 600K) in 1000, 400 and 100 MB 18.0 / 19.4, 19.9 / 21.0 and
+// 21.5 / 22.4 ms, 374K / 371K, 792K / 795K and 1,143K / 1,143K; 8 MPC problems to
+// |S| = 4 (170K) in 1000, 400 and 100 MB 3.96 / 3.95, 5.16 / 5.02 and 5.41 / 5.31 ms,
+// 5,734 / 0, 98,497 / 92,894 and 144,333 / 141,445
+constexpr double kAheadMin = 500000.0;
+
 // sets of a level from which its candidates are brought into their instances'
 // order (k_order, k_scatter: about 15 us), in a batch of different shapes, and the
 // largest share of one instance.  Enumeration without / with it, mixed and FP64:
@@ -864,9 +878,11 @@ static int enqueue(mpqp_plan *P, cudaStream_t s, EventMode events)
         } else {
             L("k_enumerate", launch_enumerate(B, k, grid(P->grid_enum, k - 1, 4), s));
         }
-        if (!B.arena_ample) L("k_room", launch_room(B, k, s));
-        L(feas, launch_feasibility(B, P->tol, P->sd, k, P->prec, grid(P->grid_feas, k, P->feas_warps), P->smem_feas, s,
-                                   P->feas_warps, P->feas_chunk));
+        const bool ask = !P->arena_ample && P->lvl_sets[k] < kAheadMin;
+        if (ask) L("k_room", launch_room(B, k, s));
+        L(feas, launch_feasibility(B, P->tol, P->sd, k, P->prec,
+                                   grid(ask ? P->grid_feas_room : P->grid_feas, k, P->feas_warps), P->smem_feas, s,
+                                   P->feas_warps, P->feas_chunk, ask));
         if (mixed) {
             L("k_lp1_cert", launch_lp1_cert(B, P->tol, P->sd, k, grid(P->grid_cert, k, 4), P->smem_cert, s));
             L("k_lp1_fp64", launch_lp1_fp64(B, P->tol, P->sd, k, grid(P->grid_lp1fb, k, 4), P->smem_lp1fb, s));
@@ -1018,20 +1034,23 @@ static int plan_create_locked(int n_inst, const mpqp_problem *probs, const mpqp_
     // combinatorial ceilings: at most C(m, k) candidates / nodes at level k
     double lvl_max = 0, arena_max = 0;
     {
-        std::vector<double> lvl(kMaxK + 2, 0.0), lvl_tab(kMaxK + 2, 0.0), lvl_top(kMaxK + 2, 0.0);
+        std::vector<double> lvl(kMaxK + 2, 0.0), pair_tab(kMaxK + 2, 0.0), lvl_top(kMaxK + 2, 0.0);
         bool mixed_shapes = false;
         for (int i = 0; i < n_inst; i++) {
             // an instance with a budget writes at most that many candidates
             // (and nodes) at any level: a level is enumerated only while it fits
             const double cap_i = P->desc[i].budget > 0 ? (double)P->desc[i].budget : 1e300;
-            double cmk = 1.0;
+            double cmk = 1.0, prev = 0.0;   // prev: tableaus the level before may store
             mixed_shapes |= P->desc[i].M1 != P->desc[0].M1 || P->desc[i].nv != P->desc[0].nv;
             for (int k = 0; k <= P->desc[i].k_max; k++) {
                 if (k > 0) cmk = cmk * (double)(P->desc[i].m - k + 1) / (double)k;
                 const double nk = std::min(cmk, cap_i);
                 lvl[k] += nk;
                 lvl_top[k] = std::max(lvl_top[k], nk);
-                if (k < P->desc[i].k_max) lvl_tab[k] += nk * (double)P->desc[i].tab_elems * (double)es;
+                // two levels in a row: their candidates are within the budget together
+                const double keep = k < P->desc[i].k_max ? nk : 0.0;
+                pair_tab[k] += std::min(prev + keep, cap_i) * (double)P->desc[i].tab_elems * (double)es;
+                prev = keep;
             }
         }
         P->lvl_sets = lvl;
@@ -1043,7 +1062,7 @@ static int plan_create_locked(int n_inst, const mpqp_problem *probs, const mpqp_
         for (const InstDesc &d : P->desc) if (d.k_max > 1) P->last_after[d.k_max - 1] = 1;
         for (int k = 0; k <= kMaxK; k++) {
             lvl_max = std::max(lvl_max, lvl[k]);
-            arena_max = std::max(arena_max, lvl_tab[k] + lvl_tab[k + 1]);
+            arena_max = std::max(arena_max, pair_tab[k]);
         }
     }
     long long cand_cap = o.cand_cap;
@@ -1099,7 +1118,7 @@ static int plan_create_locked(int n_inst, const mpqp_problem *probs, const mpqp_
     B.node_cap = node_cap;
     B.tab_cap = tab_cap;
     B.ids_cap = ids_cap;
-    B.arena_ample = arena_max <= (double)tab_cap * es;
+    P->arena_ample = arena_max <= (double)tab_cap * es;
     B.hash_cap = hash_cap;
     B.cand_cap = cand_cap;
     B.q_cap = cand_cap;
@@ -1219,7 +1238,9 @@ static int plan_create_locked(int n_inst, const mpqp_problem *probs, const mpqp_
     P->smem_optfb = 4 * opt_smem_per_warp(sd, false);
     P->smem_direct = smem_opt64;
     if ((rc = grid_for(kernel_ptr("enumerate"), 0, &P->grid_enum)) ||
-        (rc = grid_for(kernel_ptr(P->prec != PREC_MIXED ? "feas64" : B.arena_ample ? "feas32" : "feas32_room"), P->smem_feas, &P->grid_feas,
+        (rc = grid_for(kernel_ptr(P->prec == PREC_MIXED ? "feas32" : "feas64"), P->smem_feas, &P->grid_feas,
+                       32 * P->feas_warps)) ||
+        (rc = grid_for(kernel_ptr(P->prec == PREC_MIXED ? "feas32_room" : "feas64"), P->smem_feas, &P->grid_feas_room,
                        32 * P->feas_warps)) ||
         (rc = grid_for(kernel_ptr("cover"), 0, &P->grid_cover)) ||
         (rc = grid_for(kernel_ptr("scatter"), 0, &P->grid_scatter)) ||

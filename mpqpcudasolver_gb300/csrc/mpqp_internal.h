@@ -217,7 +217,7 @@ struct Ctl {
     // later nodes of that level keep no tableau, and their children start
     // LP1 from the root tableau (the arena's overflow is not an error)
     int tab_full[2];
-    int ahead;                  // LP1 reserves arena space for whole chunks (k_room)
+    int ahead;                  // k_room: LP1 reserves arena space for whole chunks
     long long split_levels;     // levels whose parents did not all keep a tableau
 };
 
@@ -245,7 +245,6 @@ struct DevBuffers {
     long long tab_cap;          // elements per arena
     uint8_t *ids[2];
     long long ids_cap;
-    int arena_ample;            // the arena holds the tableaus of every combination of two levels in a row
     HashSlot *hash[2];
     long long hash_cap;         // power of two
     CoverSlot *cover[2];        // parallel to the first cover_cap slots of hash (may be null)

@@ -1263,17 +1263,13 @@ __global__ void __launch_bounds__(128) k_scatter(DevBuffers B, int level)
 
 // Whether LP1 reserves arena space for every candidate of a level that may store
 // a tableau, a chunk's at once, also for those that turn out infeasible (up to a
-// fifth of a level on MPC problems).  Only where that cannot cost a set its
-// tableau: where the arena holds all of them beside their parents', and beside
-// them all that the next level could store.  A candidate of the next level has
-// level + 1 subsets here and a set at most m - level supersets there, so those
-// number at most n (m - level) / (level + 1).  Otherwise space is reserved for
-// each set as it is stored.  Enumeration with space always reserved ahead / by
-// this rule, arenas of 1000, 400 and 100 MB: 8 MPC problems to |S| = 4 (mixed)
-// 4.04 / 3.98, 5.27 / 5.14 and 5.54 / 5.44 ms, FP64 64.2 / 62.8, 72.2 / 72.1 and
-// 77.7 / 77.3 ms; 32 mpLPs, whose LPs of under two pivots gain least from a
-// tableau, 18.3 / 19.3, 20.2 / 20.7 and 21.7 / 22.0 ms.  One warp; not launched
-// for a plan whose arena holds every combination (DevBuffers::arena_ample).
+// fifth of a level on MPC problems): where that cannot cost a set its tableau, as
+// the arena holds all of them beside their parents', and beside them all that the
+// next level could store.  A candidate of the next level has level + 1 subsets
+// here and a set at most m - level supersets there, so those number at most
+// n (m - level) / (level + 1), and what is left of the budget.  Otherwise space is
+// reserved for each set as it is stored.  One warp; launched for the smaller levels
+// of plans with a limited arena (kAheadMin).
 __global__ void __launch_bounds__(32) k_room(DevBuffers B, int level)
 {
     Ctl *ctl = B.ctl;
@@ -1285,8 +1281,8 @@ __global__ void __launch_bounds__(32) k_room(DevBuffers B, int level)
         if (ic.stopped || level >= I.k_max || (I.budget > 0 && ic.cum_cand + ic.lvl_cand > I.budget)) continue;
         now += ic.lvl_cand * I.tab_elems;
         if (level + 1 < I.k_max) {
-            const long long most = ic.lvl_cand * (I.m - level) / (level + 1);
-            next += (I.budget > 0 && most > I.budget ? I.budget : most) * I.tab_elems;
+            const long long most = ic.lvl_cand * (I.m - level) / (level + 1), left = I.budget - ic.cum_cand - ic.lvl_cand;
+            next += (I.budget > 0 && most > left ? left : most) * I.tab_elems;
         }
     }
 #pragma unroll
@@ -1448,8 +1444,8 @@ __device__ __noinline__ longlong2 reserve_space(const DevBuffers &B, int side, i
     const long long iold = (long long)atomicAdd((unsigned long long *)&ctl->ids_used[side], (unsigned long long)ids_bytes);
     if (told + tab_elems + ctl->tab_used[side ^ 1] > B.tab_cap || iold + ids_bytes + ctl->ids_used[side ^ 1] > B.ids_cap) {
         // this node and the later ones of the level keep no tableau (a
-        // reservation past the end is abandoned, so the used counts only
-        // overstate); their children start from the root tableau
+        // reservation past the end is abandoned, so the used counts overstate
+        // until k_finalize); their children start from the root tableau
         atomicExch(&ctl->tab_full[side], 1);
         return longlong2{-1, -1};
     }
@@ -1701,12 +1697,12 @@ __device__ __noinline__ void cold_stage_lp1_f32(const DevBuffers &B, const InstD
 // T = float : the FP32 pass of the mixed path; a verdict is final only when
 //             certified (see below), otherwise the candidate is queued for
 //             the FP64 re-solve.
-// Ample: the arena holds every combination (DevBuffers::arena_ample).  A kernel
-// of its own in FP32, because the mere presence of the other route slowed LP1 of
-// 32 mpLPs by a tenth (2,830 us without it).
-template <typename T, bool Ample>
+// Ahead: arena space is always reserved ahead; else, with ask, as k_room says.  A
+// kernel of its own in FP32, because with both routes in one LP1 of 32 mpLPs took
+// 10 % longer and of 64 MPC problems 6 %.
+template <typename T, bool Ahead>
 __device__ __forceinline__ void feasibility_body(const DevBuffers &B, const Tol &tol, const SlotDims &sd, int level,
-                                                 int chunk)
+                                                 int chunk, bool ask)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     const int lane = lane_id(), wib = threadIdx.x >> 5;
@@ -1732,7 +1728,9 @@ __device__ __forceinline__ void feasibility_body(const DevBuffers &B, const Tol 
     LocalInstCounters lc;
     lc.reset(-1);
     chunk = claim_size(wend, chunk);
-    const bool ahead = Ample || (!mixed && B.arena_ample) || ctl->ahead;   // see k_room
+    const bool ahead = Ahead || !ask || ctl->ahead;
+    // the arena beside the parents' tableaus
+    const long long tab_end = B.tab_cap - ctl->tab_used[side ^ 1], ids_end = B.ids_cap - ctl->ids_used[side ^ 1];
     for (;;) {
         long long w0;
         if (lane == 0) w0 = (long long)atomicAdd(&ctl->ctr[0], (unsigned long long)chunk);
@@ -1770,18 +1768,22 @@ __device__ __forceinline__ void feasibility_body(const DevBuffers &B, const Tol 
                 const int tv = __shfl_up_sync(FULLMASK, ts, off), iv = __shfl_up_sync(FULLMASK, is, off);
                 if (lane >= off) { ts += tv; is += iv; }
             }
-            long long tb = 0, ibase = 0;
-            if (lane == 31 && ts > 0) {
+            long long tb = -1, ibase = 0;
+            if (lane == 31 && ts > 0 && !arena_full(ctl, side)) {
                 tb = (long long)atomicAdd((unsigned long long *)&ctl->tab_used[side], (unsigned long long)ts);
                 ibase = (long long)atomicAdd((unsigned long long *)&ctl->ids_used[side], (unsigned long long)is);
             }
             tb = __shfl_sync(FULLMASK, tb, 31);
             ibase = __shfl_sync(FULLMASK, ibase, 31);
             if (!ahead && keeps && !arena_full(ctl, side)) toff = kReserveLater;
-            if (ahead && keeps) {
-                // side 0 from the arena's start, side 1 from its end (see store_node)
-                toff = side == 0 ? tb + ts - te : B.tab_cap - tb - ts;
-                ioff = side == 0 ? ibase + is - ib : B.ids_cap - ibase - is;
+            if (ahead && keeps && tb >= 0) {
+                // side 0 from the arena's start, side 1 from its end (see reserve_space)
+                if (tb + ts > tab_end || ibase + is > ids_end) {
+                    atomicExch(&ctl->tab_full[side], 1);
+                } else {
+                    toff = side == 0 ? tb + ts - te : B.tab_cap - tb - ts;
+                    ioff = side == 0 ? ibase + is - ib : B.ids_cap - ibase - is;
+                }
             }
             if constexpr (mixed) {
                 room[lane] = toff;
@@ -2070,7 +2072,7 @@ __device__ __forceinline__ void feasibility_body(const DevBuffers &B, const Tol 
             }
             longlong2 sp{-1, -1};
             if constexpr (mixed) {
-                if (!Ample && room[t] == kReserveLater) reserve_to(B, side, I.tab_elems, I.ids_bytes, room, t);
+                if (!Ahead && room[t] == kReserveLater) reserve_to(B, side, I.tab_elems, I.ids_bytes, room, t);
                 sp = longlong2{room[t], room[32 + t]};
             } else {
                 sp = longlong2{__shfl_sync(FULLMASK, toff, t), __shfl_sync(FULLMASK, ioff, t)};
@@ -2125,16 +2127,16 @@ __device__ __forceinline__ void feasibility_body(const DevBuffers &B, const Tol 
     }
 }
 
-template <bool Ample>
+template <bool Ahead>
 __global__ void __launch_bounds__(128) k_feasibility_f32(DevBuffers B, Tol tol, SlotDims sd, int level, int chunk)
 {
-    feasibility_body<float, Ample>(B, tol, sd, level, chunk);
+    feasibility_body<float, Ahead>(B, tol, sd, level, chunk, !Ahead);
 }
 
 __global__ void __launch_bounds__(128, kF64Blocks) k_feasibility_f64(DevBuffers B, Tol tol, SlotDims sd, int level,
-                                                                     int chunk)
+                                                                     int chunk, bool ask)
 {
-    feasibility_body<double, false>(B, tol, sd, level, chunk);
+    feasibility_body<double, false>(B, tol, sd, level, chunk, ask);
 }
 
 // ---------------------------------------------------------------------
@@ -5350,6 +5352,10 @@ __global__ void k_finalize(DevBuffers B, int level)
         ctl->hcap[level & 1] = hash_cap_for(B, ctl->n_cand);   // what this level's inserts used
         ctl->n_cand = 0;
         if (ctl->tab_full[level & 1]) ctl->split_levels++;   // this level's children partly without a tableau
+        // reservations past the arena's end were abandoned
+        const int side = level & 1;
+        ctl->tab_used[side] = min(ctl->tab_used[side], B.tab_cap - ctl->tab_used[side ^ 1]);
+        ctl->ids_used[side] = min(ctl->ids_used[side], B.ids_cap - ctl->ids_used[side ^ 1]);
         if (level > 0) {
             ctl->n_node[pside] = 0;
             ctl->tab_used[pside] = 0;
@@ -5614,13 +5620,13 @@ cudaError_t launch_cover(const DevBuffers &B, int level, int grid, cudaStream_t 
 }
 
 // warps: warps per block (1..4, smem = warps x the slot); chunk: candidates
-// a warp claims at a time (1..32)
+// a warp claims at a time (1..32); ask: arena space as k_room says, else ahead
 cudaError_t launch_feasibility(const DevBuffers &B, const Tol &tol, const SlotDims &sd, int level, int prec,
-                               int grid, size_t smem, cudaStream_t s, int warps, int chunk)
+                               int grid, size_t smem, cudaStream_t s, int warps, int chunk, bool ask)
 {
     if (warps < 1 || warps > 4 || chunk < 1 || chunk > kFeasChunkMax) return cudaErrorInvalidValue;
-    if (prec == PREC_FP64) k_feasibility_f64<<<grid, 32 * warps, smem, s>>>(B, tol, sd, level, chunk);
-    else if (B.arena_ample) k_feasibility_f32<true><<<grid, 32 * warps, smem, s>>>(B, tol, sd, level, chunk);
+    if (prec == PREC_FP64) k_feasibility_f64<<<grid, 32 * warps, smem, s>>>(B, tol, sd, level, chunk, ask);
+    else if (!ask) k_feasibility_f32<true><<<grid, 32 * warps, smem, s>>>(B, tol, sd, level, chunk);
     else k_feasibility_f32<false><<<grid, 32 * warps, smem, s>>>(B, tol, sd, level, chunk);
     return cudaGetLastError();
 }
