@@ -332,7 +332,9 @@ __device__ __forceinline__ float trunc_float(unsigned long long bits, bool *ok)
 // 31 columns: its rules, operations and roundings (so the same pivots and
 // bit-identical values), with the bookkeeping in registers as in
 // simplex_fast32 (each lane the ids of its rows lane, lane + 32, ...; lanes
-// 0..ncols the objective row; lanes 0..ncols-1 the nonbasic ids).
+// 0..ncols the objective row; lanes 0..ncols-1 the nonbasic ids).  Under the
+// callers' bound of 128 registers ptxas spills 104-160, 244-436 and 296-384 bytes
+// of it at NS = 2, 3 and 4.
 //
 // Bound by the FP64 pipe (a warp instruction takes 16 cycles of an SM) and, on
 // small levels, by the pivot's latency.  Hence
