@@ -899,6 +899,9 @@ static int enqueue(mpqp_plan *P, cudaStream_t s, EventMode events)
     return MPQP_OK;
 }
 
+// candidates of a run up to which there is room for all of them as optimal sets (32 MB)
+constexpr long long kOptAll = 1 << 19;
+
 // share of the usable memory a plan's cover slots may take
 constexpr double kCoverShare = 0.05;
 
@@ -1032,7 +1035,7 @@ static int plan_create_locked(int n_inst, const mpqp_problem *probs, const mpqp_
         if (probs[i].budget > 0) total_budget += probs[i].budget; else all_budget = false;
     }
     // combinatorial ceilings: at most C(m, k) candidates / nodes at level k
-    double lvl_max = 0, arena_max = 0;
+    double lvl_max = 0, arena_max = 0, total_sets = 0;
     {
         std::vector<double> lvl(kMaxK + 2, 0.0), pair_tab(kMaxK + 2, 0.0), lvl_top(kMaxK + 2, 0.0);
         bool mixed_shapes = false;
@@ -1040,18 +1043,20 @@ static int plan_create_locked(int n_inst, const mpqp_problem *probs, const mpqp_
             // an instance with a budget writes at most that many candidates
             // (and nodes) at any level: a level is enumerated only while it fits
             const double cap_i = P->desc[i].budget > 0 ? (double)P->desc[i].budget : 1e300;
-            double cmk = 1.0, prev = 0.0;   // prev: tableaus the level before may store
+            double cmk = 1.0, prev = 0.0, sets = 0.0;   // prev: tableaus the level before may store
             mixed_shapes |= P->desc[i].M1 != P->desc[0].M1 || P->desc[i].nv != P->desc[0].nv;
             for (int k = 0; k <= P->desc[i].k_max; k++) {
                 if (k > 0) cmk = cmk * (double)(P->desc[i].m - k + 1) / (double)k;
                 const double nk = std::min(cmk, cap_i);
                 lvl[k] += nk;
+                sets += nk;
                 lvl_top[k] = std::max(lvl_top[k], nk);
                 // two levels in a row: their candidates are within the budget together
                 const double keep = k < P->desc[i].k_max ? nk : 0.0;
                 pair_tab[k] += std::min(prev + keep, cap_i) * (double)P->desc[i].tab_elems * (double)es;
                 prev = keep;
             }
+            total_sets += std::min(sets, cap_i);
         }
         P->lvl_sets = lvl;
         P->ordered.assign(lvl.size(), 0);
@@ -1110,7 +1115,11 @@ static int plan_create_locked(int n_inst, const mpqp_problem *probs, const mpqp_
     for (const InstDesc &d : P->desc) { min_tab = std::min(min_tab, (long long)d.tab_elems); max_ids = std::max(max_ids, (long long)d.ids_bytes); }
     long long ids_cap = std::max((tab_cap / min_tab + n_inst + 1) * max_ids, 2 * ids_tot0 + 1024);
     ids_cap = (ids_cap + 15) & ~15LL;
-    long long opt_cap = o.opt_cap > 0 ? o.opt_cap : std::max(node_cap / 8, (long long)4096);
+    // optimal sets: every candidate of a small run can be one (up to 7,837 of the
+    // 8,257 sets of an n = 16, m = 128, p = 15 problem to |S| = 2 are), of a large
+    // one a few in a hundred are
+    const long long opt_all = (long long)std::min(total_sets, (double)kOptAll);
+    long long opt_cap = o.opt_cap > 0 ? o.opt_cap : std::max({node_cap / 8, opt_all, (long long)4096});
     long long rec_cap = o.record ? (o.rec_cap > 0 ? o.rec_cap : cand_cap * 4) : 0;
     DevBuffers &B = P->B;
     memset(&B, 0, sizeof(B));
